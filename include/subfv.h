@@ -39,6 +39,10 @@ int subfv_probe_fp64_fma(int iters, double* tflops, double* ms);
  * n host doubles x, the quotients x/3 and x/6 that differ in any bit from CUDA's
  * division. */
 int subfv_probe_div_const(const double* x, int64_t n, int64_t* mismatches);
+/* Checks the kernels' quotient and square root (zero-safe forms of / and sqrt) against
+   the operators on n pairs: mismatches[0..3] counts FP64 quotients a / b, FP64 roots of
+   a, FP32 quotients and FP32 roots whose bits differ (two NaNs agree). */
+int subfv_probe_quotients(const double* a, const double* b, int64_t n, int64_t* mismatches);
 
 /* ---------------------------------------------------------------------------------
  * Topology: build_mesh (src/mesh/mesh_connectivity_module.F90:12-59) on the host,

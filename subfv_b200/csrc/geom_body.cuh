@@ -30,7 +30,7 @@ __device__ inline V3 vertex_mean(V3 s, int nvc) {
   if (nvc == 8) return {s.x * 0.125, s.y * 0.125, s.z * 0.125};
   if (nvc == 4) return {s.x * 0.25, s.y * 0.25, s.z * 0.25};
   if (nvc == 6) return {div6(s.x), div6(s.y), div6(s.z)};
-  return {s.x / nvc, s.y / nvc, s.z / nvc};
+  return {qdiv(s.x, nvc), qdiv(s.y, nvc), qdiv(s.z, nvc)};
 }
 
 // compute_face_centroid + compute_subface_norm + compute_face_norm (:177-271), one thread
@@ -65,7 +65,7 @@ __device__ inline void face_geom_body(const DevMesh& m, const int f) {
       c.z = c.z + div3(area * (pj.z + pp.z + cg.z));
       sum_area = sum_area + area;
     }
-  c = {c.x / sum_area, c.y / sum_area, c.z / sum_area};
+  c = {qdiv(c.x, sum_area), qdiv(c.y, sum_area), qdiv(c.z, sum_area)};
   m.fc[f] = make_double4(c.x, c.y, c.z, 0.0);
   const int4 fs = m.fsf[f];
   const int sfi[4] = {fs.x, fs.y, fs.z, fs.w};
@@ -83,7 +83,7 @@ __device__ inline void face_geom_body(const DevMesh& m, const int f) {
       const V3 nr = {0.5 * (a.x + b.x), 0.5 * (a.y + b.y), 0.5 * (a.z + b.z)};
       const double area = fnorm2_3(nr.x, nr.y, nr.z);
       if (FULL) {
-        const V3 un = {nr.x / area, nr.y / area, nr.z / area};
+        const V3 un = {qdiv(nr.x, area), qdiv(nr.y, area), qdiv(nr.z, area)};
         m.sfn[sf] = make_double4(un.x, un.y, un.z, area);
         S = {S.x + area * un.x, S.y + area * un.y, S.z + area * un.z};
       } else {
@@ -95,7 +95,7 @@ __device__ inline void face_geom_body(const DevMesh& m, const int f) {
       fnrm = {fnrm.x + nr.x, fnrm.y + nr.y, fnrm.z + nr.z};
     }
   const double fa = fnorm2_3(fnrm.x, fnrm.y, fnrm.z);
-  m.fn[f] = make_double4(fnrm.x / fa, fnrm.y / fa, fnrm.z / fa, fa);
+  m.fn[f] = make_double4(qdiv(fnrm.x, fa), qdiv(fnrm.y, fa), qdiv(fnrm.z, fa), fa);
   if (m.fS) m.fS[f] = make_double4(S.x, S.y, S.z, 0.0);
 }
 
@@ -313,7 +313,7 @@ __device__ inline void geom_step_body(const DevMesh& m, double* sol6, const doub
       cp = cpp;
     }
   }
-  cen = {cen.x / sum_vol, cen.y / sum_vol, cen.z / sum_vol};
+  cen = {qdiv(cen.x, sum_vol), qdiv(cen.y, sum_vol), qdiv(cen.z, sum_vol)};
   // compute_subelem_volume: subcell k is (cell, vertex k); its subfaces in sub_elem order
   bool ok = true;
   double vcell = 0.0;

@@ -62,8 +62,8 @@ __device__ inline double lam_side(double p_me, double p_ot, double tau_me, doubl
   T tm = (T)tau_me;
   T a = sqrt((T)kGamma * (T)p_me * tm) / tm;
   T mx = (T)p_ot - (T)p_me;
-  T b = sqrt((mx > (T)0 ? mx : (T)0) / tm);
-  T c = -(T)vdiff / tm;
+  T b = qsqrt(qdiv(mx > (T)0 ? mx : (T)0, tm));
+  T c = qdiv(-(T)vdiff, tm);
   T r = a;
   if (b > r) r = b;
   if (c > r) r = c;
@@ -99,7 +99,7 @@ __device__ inline void lag_face_body(const DevMesh& m, const double* __restrict_
     vr = dot3(ur.u, ur.v, ur.w, n0, n1, n2);
     l1 = lam_side<P>(pl, pr, ul.t, vr - vl);
     l2 = lam_side<P>(pr, pl, ur.t, vr - vl);
-    xb = (l1 * vl + l2 * vr - (pr - pl)) / (l2 + l1);
+    xb = qdiv(l1 * vl + l2 * vr - (pr - pl), l2 + l1);
     kind = 0.0;
   } else if (m.b2d && fabs(n2) > 1e-8) {
     l1 = lam_wall<P>(pl, ul.t);
@@ -214,7 +214,7 @@ __device__ inline void lag_node_body(const DevMesh& m, const int v) {
     double mb0 = 0.0 + I00 * B0 + I01 * B1 + I02 * B2;
     double mb1 = 0.0 + I10 * B0 + I11 * B1 + I12 * B2;
     double mb2 = 0.0 + I20 * B0 + I21 * B1 + I22 * B2;
-    double Pp = dot3(R0, R1, R2, mb0, mb1, mb2) / dot3(B0, B1, B2, mb0, mb1, mb2);
+    double Pp = qdiv(dot3(R0, R1, R2, mb0, mb1, mb2), dot3(B0, B1, B2, mb0, mb1, mb2));
     b0 = R0 - Pp * B0;
     b1 = R1 - Pp * B1;
     b2 = R2 - Pp * B2;
@@ -255,9 +255,9 @@ __device__ inline void lag_sidil_node_body(const DevMesh& m, const double* __res
   const double V = m.vol_v[v];
   rho_p = rho_p / V;
   a_p = a_p / V;
-  vx = vx / V;
-  vy = vy / V;
-  vz = vz / V;
+  vx = qdiv(vx, V);
+  vy = qdiv(vy, V);
+  vz = qdiv(vz, V);
   pp = pp / V;
   double g0 = 0.0, g1 = 0.0, g2 = 0.0, div_v = 0.0, b0 = 0.0, b1 = 0.0, b2 = 0.0;
   for (int q = m.vsf_off[v]; q < m.vsf_off[v + 1]; ++q) {
@@ -288,15 +288,15 @@ __device__ inline void lag_sidil_node_body(const DevMesh& m, const double* __res
     g2 = g2 + (rp - ul.p) * area * fn.z;
     div_v = div_v + dot3(r1 - ul.u, r2 - ul.v, r3 - ul.w, area * fn.x, area * fn.y, area * fn.z);
   }
-  g0 = g0 / V;
-  g1 = g1 / V;
-  g2 = g2 / V;
-  div_v = div_v / V;
+  g0 = qdiv(g0, V);
+  g1 = qdiv(g1, V);
+  g2 = qdiv(g2, V);
+  div_v = qdiv(div_v, V);
   if (m.is_bound[v]) {
     const double nb = fnorm2_3(b0, b1, b2);
-    b0 = b0 / nb;
-    b1 = b1 / nb;
-    b2 = b2 / nb;
+    b0 = qdiv(b0, nb);
+    b1 = qdiv(b1, nb);
+    b2 = qdiv(b2, nb);
     const double gb = dot3(g0, g1, g2, b0, b1, b2);
     g0 = g0 - gb * b0;
     g1 = g1 - gb * b1;

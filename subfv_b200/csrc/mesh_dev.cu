@@ -414,7 +414,7 @@ __global__ void k_cell_geometry(DevMesh m) {
     V3 p = ld3(m.x, m.ev[vb + k]);
     ce = {ce.x + p.x, ce.y + p.y, ce.z + p.z};
   }
-  ce = {ce.x / nvc, ce.y / nvc, ce.z / nvc};
+  ce = {qdiv(ce.x, nvc), qdiv(ce.y, nvc), qdiv(ce.z, nvc)};
   int faces[8];
   int nfc = 0;
   for (int k = 0; k < 8; ++k) {
@@ -435,14 +435,14 @@ __global__ void k_cell_geometry(DevMesh m) {
     for (int k = 0; k < n; ++k) {
       V3 cp = ld3(m.x, vid[k]), cpp = ld3(m.x, vid[(k + 1) % n]);
       V3 x = left ? cross(sub(cp, cf), sub(cpp, cf)) : cross(sub(cpp, cf), sub(cp, cf));
-      double vol = dot(x, fe) / 6.0;
+      double vol = div6(dot(x, fe));
       cen.x = cen.x + vol * (cp.x + cpp.x + cf.x + ce.x) / 4.0;
       cen.y = cen.y + vol * (cp.y + cpp.y + cf.y + ce.y) / 4.0;
       cen.z = cen.z + vol * (cp.z + cpp.z + cf.z + ce.z) / 4.0;
       sum_vol = sum_vol + vol;
     }
   }
-  cen = {cen.x / sum_vol, cen.y / sum_vol, cen.z / sum_vol};
+  cen = {qdiv(cen.x, sum_vol), qdiv(cen.y, sum_vol), qdiv(cen.z, sum_vol)};
   m.cc[c] = make_double4(cen.x, cen.y, cen.z, 0.0);
   bool ok = true;
   double vcell = 0.0;
@@ -472,7 +472,7 @@ __global__ void k_cell_geometry(DevMesh m) {
         x1 = cross(cc3, b);
         x2 = cross(b, a);
       }
-      vol = vol + dot(x1, fe) / 6.0 + dot(x2, fe) / 6.0;
+      vol = vol + div6(dot(x1, fe)) + div6(dot(x2, fe));
     }
     m.vol_se[s] = vol;
     ok = ok && (vol > 0.0);
@@ -491,7 +491,7 @@ __global__ void k_cell_geometry(DevMesh m) {
     vdiv = vdiv + dot(ld3(m.fc, f), an);
     nt = {nt.x + an.x, nt.y + an.y, nt.z + an.z};
   }
-  vdiv = vdiv / 3.0;
+  vdiv = div3(vdiv);
   for (int j = 0; j < nfc; ++j) {
     int f = faces[j];
     double sg = m.flr[f].x == c ? 1.0 : -1.0;

@@ -80,7 +80,7 @@ __device__ inline void p2c(const T* w, T* u) {
 template <class T>
 __device__ inline void c2p(const T* u, T* w) {
   w[0] = u[0];
-  for (int k = 1; k < 4; ++k) w[k] = u[k] / u[0];
+  for (int k = 1; k < 4; ++k) w[k] = qdiv(u[k], u[0]);
   w[4] = (T)(G - 1) * (u[4] - (T)0.5 * w[0] * (w[1] * w[1] + w[2] * w[2] + w[3] * w[3]));
 }
 template <class T>
@@ -260,7 +260,7 @@ __device__ void lu_solve3(double A[3][3], double* x, const double* b) {
       for (int i = k + 1; i < 3; ++i) y[i] = y[i] - y[k] * A[i][k];
   for (int k = 2; k >= 0; --k)
     if (y[k] != 0.0) {
-      y[k] = y[k] / A[k][k];
+      y[k] = qdiv(y[k], A[k][k]);
       for (int i = 0; i < k; ++i) y[i] = y[i] - y[k] * A[i][k];
     }
   for (int k = 0; k < 3; ++k) x[k] = y[k];
@@ -291,7 +291,7 @@ __device__ inline T oi3(T a0, T a1, T a2) {
         res += q * q;
       }
     }
-  return scale * sqrt(res);
+  return scale * qsqrt(res);
 }
 
 // sol_potential_flow_2d / _3d (ns_euler_exact_sol_module.F90:105-170) at x, primitive.
@@ -344,8 +344,8 @@ __device__ __noinline__ void right_state_ext(int kind, const BcVals bv, const do
   if (kind == 2) {
     for (int k = 0; k < 5; ++k) sol_r[k] = sol_l[k];
     for (int k = 1; k < 4; ++k) sol_r[k] = (T)2.0 * sol_l[0] * (T)bv.v[k] - sol_l[k];
-    const T nl = oi3<T>(sol_l[1] / sol_l[0], sol_l[2] / sol_l[0], sol_l[3] / sol_l[0]);
-    const T nr = oi3<T>(sol_r[1] / sol_r[0], sol_r[2] / sol_r[0], sol_r[3] / sol_r[0]);
+    const T nl = oi3<T>(qdiv(sol_l[1], sol_l[0]), qdiv(sol_l[2], sol_l[0]), qdiv(sol_l[3], sol_l[0]));
+    const T nr = oi3<T>(qdiv(sol_r[1], sol_r[0]), qdiv(sol_r[2], sol_r[0]), qdiv(sol_r[3], sol_r[0]));
     sol_r[4] = sol_l[4] - (T)0.5 * sol_l[0] * (nl * nl) + (T)0.5 * sol_l[0] * (nr * nr);
     return;
   }
@@ -468,12 +468,12 @@ __device__ void two_wave(const double* wl64, const double* wr64, const double* n
   fr[0] = vnr * ur[0];
   for (int k = 1; k < 4; ++k) fr[k] = vnr * ur[k] + pr * n[k - 1];
   fr[4] = (ur[4] + pr) * vnr;
-  T lam_l = tmax2(tmax2(al * rhol, sqrt(rhol * tmax2((T)0, pr - pl))), -rhol * (vnr - vnl));
-  T lam_r = tmax2(tmax2(ar * rhor, sqrt(rhor * tmax2((T)0, pl - pr))), -rhor * (vnr - vnl));
+  T lam_l = tmax2(tmax2(al * rhol, qsqrt(rhol * tmax2((T)0, pr - pl))), -rhol * (vnr - vnl));
+  T lam_r = tmax2(tmax2(ar * rhor, qsqrt(rhor * tmax2((T)0, pl - pr))), -rhor * (vnr - vnl));
   T sl = vnl - lam_l / rhol;
   T sr = vnr + lam_r / rhor;
   for (int k = 0; k < 5; ++k) {
-    T et = (sr * ur[k] - sl * ul[k] - (fr[k] - fl[k])) / (sr - sl);
+    T et = qdiv(sr * ur[k] - sl * ul[k] - (fr[k] - fl[k]), sr - sl);
     T f = (T)0.5 * (fl[k] + fr[k]) - (T)0.5 * (fabs(sl) * (et - ul[k]) + fabs(sr) * (ur[k] - et));
     lr[0][k] = (double)f;
     lr[1][k] = (double)(-f);
@@ -510,9 +510,9 @@ __device__ __noinline__ void three_wave(const double* wl64, const double* wr64, 
   fr[0] = vnr * ur[0];
   for (int k = 1; k < 4; ++k) fr[k] = vnr * ur[k] + pr * n[k - 1];
   fr[4] = (ur[4] + pr) * vnr;
-  T lam_l = tmax2(tmax2(al * rhol, sqrt(rhol * tmax2(c0, pr - pl))), -rhol * (vnr - vnl));
-  T lam_r = tmax2(tmax2(ar * rhor, sqrt(rhor * tmax2(c0, pl - pr))), -rhor * (vnr - vnl));
-  T v_et = (lam_l * vnl + lam_r * vnr - (pr - pl)) / (lam_r + lam_l);
+  T lam_l = tmax2(tmax2(al * rhol, qsqrt(rhol * tmax2(c0, pr - pl))), -rhol * (vnr - vnl));
+  T lam_r = tmax2(tmax2(ar * rhor, qsqrt(rhor * tmax2(c0, pl - pr))), -rhor * (vnr - vnl));
+  T v_et = qdiv(lam_l * vnl + lam_r * vnr - (pr - pl), lam_r + lam_l);
   T vt_et[3] = {c0, c0, c0}, tang_energy = c0;
   if (modified) {
     T vt_l[3], vt_r[3], dvt[3];
@@ -520,28 +520,28 @@ __device__ __noinline__ void three_wave(const double* wl64, const double* wr64, 
       vt_l[d] = wl[1 + d] - vnl * n[d];
       vt_r[d] = wr[1 + d] - vnr * n[d];
     }
-    for (int d = 0; d < 3; ++d) vt_et[d] = (lam_l * vt_l[d] + lam_r * vt_r[d]) / (lam_l + lam_r);
+    for (int d = 0; d < 3; ++d) vt_et[d] = qdiv(lam_l * vt_l[d] + lam_r * vt_r[d], lam_l + lam_r);
     for (int d = 0; d < 3; ++d) dvt[d] = vt_r[d] - vt_l[d];
     const T tang_coeff = -(lam_l * lam_r / (lam_l + lam_r));
     tang_energy = tang_coeff * dotT(dvt, vt_et);
   }
-  T rhol_et = c1 / (c1 / rhol + (v_et - vnl) / lam_l);
+  T rhol_et = c1 / (c1 / rhol + qdiv(v_et - vnl, lam_l));
   T pl_bar = pl - lam_l * (v_et - vnl);
-  T rhor_et = c1 / (c1 / rhor + (vnr - v_et) / lam_r);
+  T rhor_et = c1 / (c1 / rhor + qdiv(vnr - v_et, lam_r));
   T pr_bar = pr + lam_r * (v_et - vnr);
   T sle[5], sre[5];
   sle[0] = rhol_et;
   sre[0] = rhor_et;
   if (modified) {
     for (int k = 1; k < 4; ++k) sle[k] = rhol_et * (v_et * n[k - 1] + vt_et[k - 1]);
-    sle[4] = rhol_et * (el + (pl * vnl - pl_bar * v_et - tang_energy) / lam_l);
+    sle[4] = rhol_et * (el + qdiv(pl * vnl - pl_bar * v_et - tang_energy, lam_l));
     for (int k = 1; k < 4; ++k) sre[k] = rhor_et * (v_et * n[k - 1] + vt_et[k - 1]);
-    sre[4] = rhor_et * (er + (pr_bar * v_et - pr * vnr + tang_energy) / lam_r);
+    sre[4] = rhor_et * (er + qdiv(pr_bar * v_et - pr * vnr + tang_energy, lam_r));
   } else {
     for (int k = 1; k < 4; ++k) sle[k] = rhol_et * (wl[k] + (v_et - vnl) * n[k - 1]);
-    sle[4] = rhol_et * (el + (pl * vnl - pl_bar * v_et) / lam_l);
+    sle[4] = rhol_et * (el + qdiv(pl * vnl - pl_bar * v_et, lam_l));
     for (int k = 1; k < 4; ++k) sre[k] = rhor_et * (wr[k] + (v_et - vnr) * n[k - 1]);
-    sre[4] = rhor_et * (er + (pr_bar * v_et - pr * vnr) / lam_r);
+    sre[4] = rhor_et * (er + qdiv(pr_bar * v_et - pr * vnr, lam_r));
   }
   const T sl = vnl - lam_l / rhol, sr = vnr + lam_r / rhor;
   for (int k = 0; k < 5; ++k) {
@@ -582,18 +582,18 @@ __device__ __noinline__ void multi_point_pressure(const double* wl64, const doub
   fr[0] = vnr * ur[0];
   for (int k = 1; k < 4; ++k) fr[k] = vnr * ur[k] + pr * n[k - 1];
   fr[4] = (ur[4] + pr) * vnr;
-  T vn_bar = (lam_l * vnl + lam_r * vnr - (pr - pl)) / (lam_r + lam_l);
-  T vn_l_et = vnl - (p_nodal - pl) / lam_l;
-  T rhol_et = c1 / (c1 / rhol + (vn_bar - vnl) / lam_l);
+  T vn_bar = qdiv(lam_l * vnl + lam_r * vnr - (pr - pl), lam_r + lam_l);
+  T vn_l_et = vnl - qdiv(p_nodal - pl, lam_l);
+  T rhol_et = c1 / (c1 / rhol + qdiv(vn_bar - vnl, lam_l));
   T sle[5], sre[5];
   sle[0] = rhol_et;
   for (int k = 1; k < 4; ++k) sle[k] = rhol_et * (vt_l[k - 1] + vn_l_et * n[k - 1]);
-  sle[4] = rhol_et * (el + (pl * vnl - p_nodal * (ph ? vn_l_et : vn_bar)) / lam_l);
-  T vn_r_et = vnr + (p_nodal - pr) / lam_r;
-  T rhor_et = c1 / (c1 / rhor + (vnr - vn_bar) / lam_r);
+  sle[4] = rhol_et * (el + qdiv(pl * vnl - p_nodal * (ph ? vn_l_et : vn_bar), lam_l));
+  T vn_r_et = vnr + qdiv(p_nodal - pr, lam_r);
+  T rhor_et = c1 / (c1 / rhor + qdiv(vnr - vn_bar, lam_r));
   sre[0] = rhor_et;
   for (int k = 1; k < 4; ++k) sre[k] = rhor_et * (vt_r[k - 1] + vn_r_et * n[k - 1]);
-  sre[4] = rhor_et * (er + (p_nodal * (ph ? vn_r_et : vn_bar) - pr * vnr) / lam_r);
+  sre[4] = rhor_et * (er + qdiv(p_nodal * (ph ? vn_r_et : vn_bar) - pr * vnr, lam_r));
   const T sl = vnl - lam_l / rhol, sr = vnr + lam_r / rhor;
   for (int k = 0; k < 5; ++k) {
     const T f = ch * (fl[k] + fr[k]) -
@@ -616,15 +616,15 @@ __device__ inline void nodal_pressure_terms(int iter, bool wall1, const double* 
   const double rhor = wr[0], vnr = dotT(wr + 1, n), pr = wr[4], ar = sqrt(G * wr[4] / wr[0]);
   auto pbar_of = [&](double ll, double lr) { return (lr * pl + ll * pr - lr * ll * (vnr - vnl)) / (lr + ll); };
   if (iter == 1) {
-    lam_l = fmax2(fmax2(fmax2(lam_l, al * rhol), sqrt(rhol * fmax2(0.0, pr - pl))), -rhol * (vnr - vnl));
-    lam_r = fmax2(fmax2(fmax2(lam_r, ar * rhor), sqrt(rhor * fmax2(0.0, pl - pr))), -rhor * (vnr - vnl));
+    lam_l = fmax2(fmax2(fmax2(lam_l, al * rhol), qsqrt(rhol * fmax2(0.0, pr - pl))), -rhol * (vnr - vnl));
+    lam_r = fmax2(fmax2(fmax2(lam_r, ar * rhor), qsqrt(rhor * fmax2(0.0, pl - pr))), -rhor * (vnr - vnl));
     const double pb = pbar_of(lam_l, lam_r);
-    lam_l = fmax2(lam_l, al * rhol + 1.5 * sqrt(fmax2(0.0, (pb - pl) * rhol)));
-    lam_r = fmax2(lam_r, ar * rhor + 1.5 * sqrt(fmax2(0.0, (pb - pr) * rhor)));
+    lam_l = fmax2(lam_l, al * rhol + 1.5 * qsqrt(fmax2(0.0, (pb - pl) * rhol)));
+    lam_r = fmax2(lam_r, ar * rhor + 1.5 * qsqrt(fmax2(0.0, (pb - pr) * rhor)));
   } else {
     const double pq = wall1 ? pbar_of(lam_l, lam_r) : p_node;
-    lam_l = fmax2(lam_l, al * rhol + 1.5 * sqrt(fmax2(0.0, (pq - pl) * rhol)));
-    lam_r = fmax2(lam_r, ar * rhor + 1.5 * sqrt(fmax2(0.0, (pq - pr) * rhor)));
+    lam_l = fmax2(lam_l, al * rhol + 1.5 * qsqrt(fmax2(0.0, (pq - pl) * rhol)));
+    lam_r = fmax2(lam_r, ar * rhor + 1.5 * qsqrt(fmax2(0.0, (pq - pr) * rhor)));
   }
   const double pb = pbar_of(lam_l, lam_r);
   if (wall1) {
@@ -720,17 +720,17 @@ __device__ bool multi_point(const double* wl64, const double* wr64, const double
   for (int k = 1; k < 4; ++k) fr[k] = vnr * ur[k] + pr * n[k - 1];
   fr[4] = (ur[4] + pr) * vnr;
   T v_et = (T)vn_nodal;
-  T rhol_et = (T)1.0 / ((T)1.0 / rhol + (v_et - vnl) / lam_l);
+  T rhol_et = (T)1.0 / ((T)1.0 / rhol + qdiv(v_et - vnl, lam_l));
   T pl_bar = pl - lam_l * (v_et - vnl);
   T sle[5], sre[5];
   sle[0] = rhol_et;
   for (int k = 1; k < 4; ++k) sle[k] = rhol_et * (wl[k] + (v_et - vnl) * n[k - 1]);
-  sle[4] = rhol_et * (el + (pl * vnl - pl_bar * v_et) / lam_l);
-  T rhor_et = (T)1.0 / ((T)1.0 / rhor + (vnr - v_et) / lam_r);
+  sle[4] = rhol_et * (el + qdiv(pl * vnl - pl_bar * v_et, lam_l));
+  T rhor_et = (T)1.0 / ((T)1.0 / rhor + qdiv(vnr - v_et, lam_r));
   T pr_bar = pr + lam_r * (v_et - vnr);
   sre[0] = rhor_et;
   for (int k = 1; k < 4; ++k) sre[k] = rhor_et * (wr[k] + (v_et - vnr) * n[k - 1]);
-  sre[4] = rhor_et * (er + (pr_bar * v_et - pr * vnr) / lam_r);
+  sre[4] = rhor_et * (er + qdiv(pr_bar * v_et - pr * vnr, lam_r));
   bool ok = !(rhol_et < (T)0 || rhor_et < (T)0);
   T sl = vnl - lam_l / rhol;
   T sr = vnr + lam_r / rhor;
@@ -775,14 +775,14 @@ __device__ void nodal_solve(const NsParams& P, double mat[3][3], const double* R
         mr[d] = s;
         mb[d] = t;
       }
-      double p_bound = dotT(mr, Bp) / dotT(mb, Bp);
+      double p_bound = qdiv(dotT(mr, Bp), dotT(mb, Bp));
       for (int d = 0; d < 3; ++d) r2[d] = Rp[d] - p_bound * Bp[d];
       for (int d = 0; d < 3; ++d) {
         double s = 0.0;
         for (int e = 0; e < 3; ++e) s = s + mat[d][e] * r2[e];
         vnode[d] = s;
       }
-      double f = dotT(vnode, Bp) / dotT(Bp, Bp);
+      double f = qdiv(dotT(vnode, Bp), dotT(Bp, Bp));
       for (int d = 0; d < 3; ++d) vnode[d] = vnode[d] - f * Bp[d];
     } else {
       lu_solve3(mat, vnode, Rp);
@@ -814,7 +814,7 @@ constexpr int kNodeThreads = 256;  // the largest block of the node kernel
 // sum A (lambda_l + lambda_r)(v* - vbar) n, which the FP64 solve of M v* = R closes,
 // then holds to FP64 rounding (with an FP64 flux), so the totals stay conserved.
 __device__ inline double vbar_of(double lam_l, double lam_r, double vnl, double vnr, double pl, double pr) {
-  return (lam_l * vnl + lam_r * vnr - (pr - pl)) / (lam_r + lam_l);
+  return qdiv(lam_l * vnl + lam_r * vnr - (pr - pl), lam_r + lam_l);
 }
 
 // compute_lambdas_and_solve_nodal_pressure for one vertex (thread-per-vertex layout):
@@ -918,20 +918,20 @@ __device__ void ns_node_vertex(const DevMesh& m, const NsParams& P, const double
           const bool wall = (wallm >> j) & 1u;
           const L c1 = (L)1, c15 = (L)1.5, c0 = (L)0;
           if (iter == 1) {
-            lam_l = tmax2(tmax2(tmax2(lam_l, al * rhol), sqrt(rhol * tmax2(c0, pr - pl))), -rhol * (vnr - vnl));
-            lam_r = tmax2(tmax2(tmax2(lam_r, ar * rhor), sqrt(rhor * tmax2(c0, pl - pr))), -rhor * (vnr - vnl));
+            lam_l = tmax2(tmax2(tmax2(lam_l, al * rhol), qsqrt(rhol * tmax2(c0, pr - pl))), -rhol * (vnr - vnl));
+            lam_r = tmax2(tmax2(tmax2(lam_r, ar * rhor), qsqrt(rhor * tmax2(c0, pl - pr))), -rhor * (vnr - vnl));
             vbar = vbar_of((double)lam_l, (double)lam_r, vnl_f, vnr_f, pl_f, pr_f);
-            lam_l = tmax2(lam_l, al * rhol * (c1 + c15 * tmax2(c0, -((L)vbar - vnl) / al)));
-            lam_r = tmax2(lam_r, ar * rhor * (c1 + c15 * tmax2(c0, ((L)vbar - vnr) / ar)));
+            lam_l = tmax2(lam_l, al * rhol * (c1 + c15 * tmax2(c0, qdiv(-((L)vbar - vnl), al))));
+            lam_r = tmax2(lam_r, ar * rhor * (c1 + c15 * tmax2(c0, qdiv((L)vbar - vnr, ar))));
           } else if (wall && P.bc_style == 1) {
             // the previous iteration's vbar, from the bounds it ended with
             vbar = vbar_of((double)lam_l, (double)lam_r, vnl_f, vnr_f, pl_f, pr_f);
-            lam_l = tmax2(lam_l, al * rhol * (c1 + c15 * tmax2(c0, -((L)vbar - vnl) / al)));
-            lam_r = tmax2(lam_r, ar * rhor * (c1 + c15 * tmax2(c0, ((L)vbar - vnr) / ar)));
+            lam_l = tmax2(lam_l, al * rhol * (c1 + c15 * tmax2(c0, qdiv(-((L)vbar - vnl), al))));
+            lam_r = tmax2(lam_r, ar * rhor * (c1 + c15 * tmax2(c0, qdiv((L)vbar - vnr, ar))));
           } else {
             const L v_et = (L)dotT(vn3, n);
-            lam_l = tmax2(lam_l, al * rhol * (c1 + c15 * tmax2(c0, -(v_et - vnl) / al)));
-            lam_r = tmax2(lam_r, ar * rhor * (c1 + c15 * tmax2(c0, (v_et - vnr) / ar)));
+            lam_l = tmax2(lam_l, al * rhol * (c1 + c15 * tmax2(c0, qdiv(-(v_et - vnl), al))));
+            lam_r = tmax2(lam_r, ar * rhor * (c1 + c15 * tmax2(c0, qdiv(v_et - vnr, ar))));
           }
           vbar = vbar_of((double)lam_l, (double)lam_r, vnl_f, vnr_f, pl_f, pr_f);
           lam[j][0] = lam_l;
@@ -1124,18 +1124,18 @@ __device__ void ns_node_group(const DevMesh& m, const NsParams& P, const double*
         const L rhor = wr[0], vnr = dotT(wr + 1, nt), pr = wr[4];
         const L c1 = (L)1, c15 = (L)1.5, c0 = (L)0;
         if (iter == 1) {
-          lam_l = tmax2(tmax2(tmax2(lam_l, al * rhol), sqrt(rhol * tmax2(c0, pr - pl))), -rhol * (vnr - vnl));
-          lam_r = tmax2(tmax2(tmax2(lam_r, ar * rhor), sqrt(rhor * tmax2(c0, pl - pr))), -rhor * (vnr - vnl));
+          lam_l = tmax2(tmax2(tmax2(lam_l, al * rhol), qsqrt(rhol * tmax2(c0, pr - pl))), -rhol * (vnr - vnl));
+          lam_r = tmax2(tmax2(tmax2(lam_r, ar * rhor), qsqrt(rhor * tmax2(c0, pl - pr))), -rhor * (vnr - vnl));
           vbar = vbar_of((double)lam_l, (double)lam_r, vnl_f, vnr_f, pl_f, pr_f);
-          lam_l = tmax2(lam_l, al * rhol * (c1 + c15 * tmax2(c0, -((L)vbar - vnl) / al)));
-          lam_r = tmax2(lam_r, ar * rhor * (c1 + c15 * tmax2(c0, ((L)vbar - vnr) / ar)));
+          lam_l = tmax2(lam_l, al * rhol * (c1 + c15 * tmax2(c0, qdiv(-((L)vbar - vnl), al))));
+          lam_r = tmax2(lam_r, ar * rhor * (c1 + c15 * tmax2(c0, qdiv((L)vbar - vnr, ar))));
         } else if (wall && P.bc_style == 1) {
-          lam_l = tmax2(lam_l, al * rhol * (c1 + c15 * tmax2(c0, -((L)vbar - vnl) / al)));
-          lam_r = tmax2(lam_r, ar * rhor * (c1 + c15 * tmax2(c0, ((L)vbar - vnr) / ar)));
+          lam_l = tmax2(lam_l, al * rhol * (c1 + c15 * tmax2(c0, qdiv(-((L)vbar - vnl), al))));
+          lam_r = tmax2(lam_r, ar * rhor * (c1 + c15 * tmax2(c0, qdiv((L)vbar - vnr, ar))));
         } else {
           const L v_et = (L)dotT(vn3, n);
-          lam_l = tmax2(lam_l, al * rhol * (c1 + c15 * tmax2(c0, -(v_et - vnl) / al)));
-          lam_r = tmax2(lam_r, ar * rhor * (c1 + c15 * tmax2(c0, (v_et - vnr) / ar)));
+          lam_l = tmax2(lam_l, al * rhol * (c1 + c15 * tmax2(c0, qdiv(-(v_et - vnl), al))));
+          lam_r = tmax2(lam_r, ar * rhor * (c1 + c15 * tmax2(c0, qdiv(v_et - vnr, ar))));
         }
         vbar = vbar_of((double)lam_l, (double)lam_r, vnl_f, vnr_f, pl_f, pr_f);
         const double lsum = (double)lam_r + (double)lam_l;
@@ -1544,7 +1544,7 @@ __device__ void ns_cell_grad_body(const DevMesh& m, const NsParams& P, const dou
       for (int i = 0; i < 15; ++i) g[i] = g[i] + vol * (T)ng[i];
       dvs = dvs + vol;
     }
-    for (int i = 0; i < 15; ++i) g[i] = g[i] / dvs;
+    for (int i = 0; i < 15; ++i) g[i] = qdiv(g[i], dvs);
   } else if (P.method == 3) {  // the vertex gradient of smallest norm, per variable
     const double* ng1 = ngrad + 15 * (size_t)m.ev[vb];
     for (int i = 0; i < 15; ++i) g[i] = (T)ng1[i];
@@ -1573,14 +1573,14 @@ __device__ void ns_cell_grad_body(const DevMesh& m, const NsParams& P, const dou
       }
     }
     if (P.method == 6) {  // OI of the (3, 5) central gradient: the norm of its first column
-      for (int i = 0; i < 15; ++i) cg[i] = cg[i] / cws;
+      for (int i = 0; i < 15; ++i) cg[i] = qdiv(cg[i], cws);
       const T q = eps + oi3<T>(cg[0], cg[5], cg[10]);
       const T wc = cws / (q * q);
       for (int i = 0; i < 15; ++i) g[i] = g[i] + wc * cg[i];
       for (int k = 0; k < 5; ++k) ws[k] = ws[k] + wc;
     }
     for (int k = 0; k < 5; ++k)
-      for (int d = 0; d < 3; ++d) g[5 * d + k] = g[5 * d + k] / ws[k];
+      for (int d = 0; d < 3; ++d) g[5 * d + k] = qdiv(g[5 * d + k], ws[k]);
   }
   double u0[5];
   ld5(U, c, u0);
@@ -1627,13 +1627,13 @@ __device__ void ns_cell_grad_body(const DevMesh& m, const NsParams& P, const dou
     for (int d = 0; d < 3; ++d) dw0 = dw0 + g[5 * d] * dx[d];
     for (int d = 0; d < 3; ++d) dw4 = dw4 + g[5 * d + 4] * dx[d];
     if (dw0 < (T)0)
-      omega = tmin2(omega, tmax2((T)0, (w0[0] - rmin) / (tol - dw0)));
+      omega = tmin2(omega, tmax2((T)0, qdiv(w0[0] - rmin, tol - dw0)));
     else
-      omega = tmin2(omega, tmax2((T)0, -(w0[0] - rmax) / (tol + dw0)));
+      omega = tmin2(omega, tmax2((T)0, qdiv(-(w0[0] - rmax), tol + dw0)));
     if (dw4 < (T)0)
-      omega = tmin2(omega, tmax2((T)0, (w0[4] - pmin) / (tol - dw4)));
+      omega = tmin2(omega, tmax2((T)0, qdiv(w0[4] - pmin, tol - dw4)));
     else
-      omega = tmin2(omega, tmax2((T)0, -(w0[4] - pmax) / (tol + dw4)));
+      omega = tmin2(omega, tmax2((T)0, qdiv(-(w0[4] - pmax), tol + dw4)));
   }
   for (int i = 0; i < 15; ++i) go[i] = (double)(omega * g[i]);
 }
@@ -1737,7 +1737,7 @@ __device__ void ns_cell_grad_group(const DevMesh& m, const NsParams& P, const do
       const T x = __shfl_sync(kAll, vol, j, kCellLanes);
       if (in) dvs = dvs + x;
     }
-    for (int i = 0; i < 15; ++i) g[i] = g[i] / dvs;
+    for (int i = 0; i < 15; ++i) g[i] = qdiv(g[i], dvs);
   } else if (P.method == 3) {  // the vertex gradient of smallest norm, per variable
     for (int k = 0; k < 5; ++k) {
       const T o = oi3<T>(ng[k], ng[5 + k], ng[10 + k]);
@@ -1785,14 +1785,14 @@ __device__ void ns_cell_grad_group(const DevMesh& m, const NsParams& P, const do
         const T x = __shfl_sync(kAll, vol, j, kCellLanes);
         if (in) cws = cws + x;
       }
-      for (int i = 0; i < 15; ++i) cg[i] = cg[i] / cws;
+      for (int i = 0; i < 15; ++i) cg[i] = qdiv(cg[i], cws);
       const T q = eps + oi3<T>(cg[0], cg[5], cg[10]);
       const T wc = cws / (q * q);
       for (int i = 0; i < 15; ++i) g[i] = g[i] + wc * cg[i];
       for (int k = 0; k < 5; ++k) ws[k] = ws[k] + wc;
     }
     for (int k = 0; k < 5; ++k)
-      for (int d = 0; d < 3; ++d) g[5 * d + k] = g[5 * d + k] / ws[k];
+      for (int d = 0; d < 3; ++d) g[5 * d + k] = qdiv(g[5 * d + k], ws[k]);
   }
   T om = 1;  // physical_slope_limiter: this lane's vertex
   {
@@ -1830,13 +1830,13 @@ __device__ void ns_cell_grad_group(const DevMesh& m, const NsParams& P, const do
     for (int d = 0; d < 3; ++d) dw0 = dw0 + g[5 * d] * dx[d];
     for (int d = 0; d < 3; ++d) dw4 = dw4 + g[5 * d + 4] * dx[d];
     if (dw0 < (T)0)
-      om = tmin2(om, tmax2((T)0, (w0[0] - rmin) / (tol - dw0)));
+      om = tmin2(om, tmax2((T)0, qdiv(w0[0] - rmin, tol - dw0)));
     else
-      om = tmin2(om, tmax2((T)0, -(w0[0] - rmax) / (tol + dw0)));
+      om = tmin2(om, tmax2((T)0, qdiv(-(w0[0] - rmax), tol + dw0)));
     if (dw4 < (T)0)
-      om = tmin2(om, tmax2((T)0, (w0[4] - pmin) / (tol - dw4)));
+      om = tmin2(om, tmax2((T)0, qdiv(w0[4] - pmin, tol - dw4)));
     else
-      om = tmin2(om, tmax2((T)0, -(w0[4] - pmax) / (tol + dw4)));
+      om = tmin2(om, tmax2((T)0, qdiv(-(w0[4] - pmax), tol + dw4)));
   }
   omega = 1;
   for (int j = 0; j < nmax; ++j) {
@@ -1911,8 +1911,8 @@ __device__ void ns_timedisc_body(const DevMesh& m, const NsParams& P, const doub
       double us[5], Ub[5], dU[5];
       ld5(U_rhs, c, us);
       for (int k = 0; k < 5; ++k) {
-        Ub[k] = us[k] + r[k] / den;
-        dU[k] = (r2[k] - r[k]) / den;
+        Ub[k] = us[k] + qdiv(r[k], den);
+        dU[k] = qdiv(r2[k] - r[k], den);
       }
       const double w = fmin2(1.0, max_omega_for_positivity(Ub, dU));
       for (int k = 0; k < 5; ++k) r[k] = r[k] + w * (r2[k] - r[k]);
@@ -1928,7 +1928,7 @@ __device__ void ns_timedisc_body(const DevMesh& m, const NsParams& P, const doub
       for (int k = 0; k < 5; ++k) rv[k] = r[k] * r[k];
       for (int k = 0; k < 5; ++k) {
         const double rr = r[k] + s * u[k];
-        d5[k] = rr / s - u[k];
+        d5[k] = qdiv(rr, s) - u[k];
         ad[k] = a2 * d5[k];
       }
     }
@@ -1947,7 +1947,7 @@ __device__ void ns_timedisc_body(const DevMesh& m, const NsParams& P, const doub
             res += q * q;
           }
         }
-      rn = scale * sqrt(res);
+      rn = scale * qsqrt(res);
     }
     double* dl = delta + 5 * (size_t)c;
     for (int k = 0; k < 5; ++k) dl[k] = d5[k];
@@ -2193,7 +2193,7 @@ __global__ void __launch_bounds__(128) kb_ns_apply(const NsItem* __restrict__ it
 // dF.n/dU for the Euler flux, conservative variables
 __device__ void euler_jac(const double* U, const double* n, double A[5][5]) {
   const double rho = U[0];
-  const double u[3] = {U[1] / rho, U[2] / rho, U[3] / rho};
+  const double u[3] = {qdiv(U[1], rho), qdiv(U[2], rho), qdiv(U[3], rho)};
   const double q2 = u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
   const double p = (G - 1) * (U[4] - 0.5 * rho * q2);
   const double vn = dotT(u, n);
@@ -2222,8 +2222,8 @@ __device__ void two_wave_jac(const double* wl, const double* wr, const double* n
   double ul[5], ur[5];
   p2c(wl, ul);
   p2c(wr, ur);
-  const double lam_l = fmax2(fmax2(al * rhol, sqrt(rhol * fmax2(0.0, pr - pl))), -rhol * (vnr - vnl));
-  const double lam_r = fmax2(fmax2(ar * rhor, sqrt(rhor * fmax2(0.0, pl - pr))), -rhor * (vnr - vnl));
+  const double lam_l = fmax2(fmax2(al * rhol, qsqrt(rhol * fmax2(0.0, pr - pl))), -rhol * (vnr - vnl));
+  const double lam_r = fmax2(fmax2(ar * rhor, qsqrt(rhor * fmax2(0.0, pl - pr))), -rhor * (vnr - vnl));
   const double sl = vnl - lam_l / rhol, sr = vnr + lam_r / rhor;
   double AL[5][5], AR[5][5];
   euler_jac(ul, n, AL);
@@ -2248,9 +2248,9 @@ struct EulerJacScalars {
 };
 __device__ inline void euler_jac_scalars(const double* U, const double* n, EulerJacScalars& e) {
   const double rho = U[0];
-  e.u[0] = U[1] / rho;
-  e.u[1] = U[2] / rho;
-  e.u[2] = U[3] / rho;
+  e.u[0] = qdiv(U[1], rho);
+  e.u[1] = qdiv(U[2], rho);
+  e.u[2] = qdiv(U[3], rho);
   const double q2 = e.u[0] * e.u[0] + e.u[1] * e.u[1] + e.u[2] * e.u[2];
   const double p = (G - 1) * (U[4] - 0.5 * rho * q2);
   e.vn = dotT(e.u, n);
@@ -2404,8 +2404,8 @@ __global__ void __launch_bounds__(64) k_be_assemble(DevMesh m, NsParams P, const
     double ul[5], ur[5];
     p2c(wl, ul);
     p2c(wr, ur);
-    const double lam_l = fmax2(fmax2(al * rhol, sqrt(rhol * fmax2(0.0, pr - pl))), -rhol * (vnr - vnl));
-    const double lam_r = fmax2(fmax2(ar * rhor, sqrt(rhor * fmax2(0.0, pl - pr))), -rhor * (vnr - vnl));
+    const double lam_l = fmax2(fmax2(al * rhol, qsqrt(rhol * fmax2(0.0, pr - pl))), -rhol * (vnr - vnl));
+    const double lam_r = fmax2(fmax2(ar * rhor, qsqrt(rhor * fmax2(0.0, pl - pr))), -rhor * (vnr - vnl));
     const double sl = vnl - lam_l / rhol, sr = vnr + lam_r / rhor;
     EulerJacScalars eL, eR;
     euler_jac_scalars(ul, n, eL);
@@ -2474,8 +2474,8 @@ __global__ void k_ns_flux_limiting(DevMesh m, NsParams P, const double* __restri
   double us[5], Ub[5], dU[5];
   ld5(U, c, us);
   for (int k = 0; k < 5; ++k) {
-    Ub[k] = us[k] + r1[k] / den;
-    dU[k] = (r2[k] - r1[k]) / den;
+    Ub[k] = us[k] + qdiv(r1[k], den);
+    dU[k] = qdiv(r2[k] - r1[k], den);
   }
   const double w = fmin2(1.0, max_omega_for_positivity(Ub, dU));
   for (int k = 0; k < 5; ++k) r1[k] = r1[k] + w * (r2[k] - r1[k]);
@@ -2766,8 +2766,8 @@ __global__ void __launch_bounds__(128) k_proc_flux_limiting(DevMesh m, const dou
   const double den = m.vol[c] / dt + sl[c];
   double Ub[5], dU[5];
   for (int k = 0; k < 5; ++k) {
-    Ub[k] = u[k] + r[k] / den;
-    dU[k] = (r2[k] - r[k]) / den;
+    Ub[k] = u[k] + qdiv(r[k], den);
+    dU[k] = qdiv(r2[k] - r[k], den);
   }
   const double w = fmin2(1.0, max_omega_for_positivity(Ub, dU));
   for (int k = 0; k < 5; ++k) r[k] = r[k] + w * (r2[k] - r[k]);
@@ -2804,7 +2804,7 @@ __global__ void __launch_bounds__(128) k_proc_timedisc(DevMesh m, const double* 
       lu_solve5(D, x);
       for (int k = 0; k < 25; ++k) dg[k] = D[k];
     } else {
-      for (int k = 0; k < 5; ++k) x[k] = x[k] / s;
+      for (int k = 0; k < 5; ++k) x[k] = qdiv(x[k], s);
     }
     for (int k = 0; k < 5; ++k) {
       d5[k] = x[k] - u[k];
@@ -2825,7 +2825,7 @@ __global__ void __launch_bounds__(128) k_proc_timedisc(DevMesh m, const double* 
           res += q * q;
         }
       }
-    rn[c] = scale * sqrt(res);
+    rn[c] = scale * qsqrt(res);
   }
   __shared__ double wm[4];
   om = warp_min(om);

@@ -124,7 +124,7 @@ __device__ inline void lu_solve5(double* A, double* b) {
       for (int i = k + 1; i < 5; ++i) b[i] = b[i] - b[k] * A[i + 5 * k];
   for (int k = 4; k >= 0; --k)
     if (b[k] != 0.0) {
-      b[k] = b[k] / A[k + 5 * k];
+      b[k] = qdiv(b[k], A[k + 5 * k]);
       for (int i = 0; i < k; ++i) b[i] = b[i] - b[k] * A[i + 5 * k];
     }
 }

@@ -126,3 +126,54 @@ extern "C" int subfv_probe_div_const(const double* x, int64_t n, int64_t* mismat
   if (bad) cudaFree(bad);
   return rc;
 }
+
+// Checks qdiv / qsqrt (common.cuh) against CUDA's operators on n pairs (a, b): counts per
+// operation (FP64 quotient, FP64 root of a, FP32 quotient, FP32 root) the pairs whose
+// results differ in any bit, two NaNs counting as equal. No counterpart in the reference.
+namespace {
+__device__ inline bool same(double p, double q) {
+  return __double_as_longlong(p) == __double_as_longlong(q) || (p != p && q != q);
+}
+__device__ inline bool same(float p, float q) { return __float_as_int(p) == __float_as_int(q) || (p != p && q != q); }
+__global__ void k_quotients(const double* __restrict__ a, const double* __restrict__ b, long n,
+                            unsigned long long* __restrict__ bad) {
+  unsigned long long nb[4] = {0, 0, 0, 0};
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+    const double x = a[i], y = b[i];
+    const float xf = (float)x, yf = (float)y;
+    nb[0] += !same(qdiv(x, y), x / y);
+    nb[1] += !same(qsqrt(x), sqrt(x));
+    nb[2] += !same(qdiv(xf, yf), xf / yf);
+    nb[3] += !same(qsqrt(xf), sqrtf(xf));
+  }
+  for (int k = 0; k < 4; ++k)
+    if (nb[k]) atomicAdd(bad + k, nb[k]);
+}
+}  // namespace
+
+extern "C" int subfv_probe_quotients(const double* a, const double* b, int64_t n, int64_t* mismatches) {
+  if (!a || !b || n < 0 || !mismatches) {
+    set_error("subfv_probe_quotients: bad argument");
+    return -2;
+  }
+  double* d = nullptr;
+  unsigned long long* bad = nullptr;
+  unsigned long long h[4] = {0, 0, 0, 0};
+  const size_t bytes = (size_t)n * sizeof(double);
+  int rc = 0;
+  if (cudaMalloc(&d, 2 * bytes + 1) != cudaSuccess || cudaMalloc(&bad, sizeof(h)) != cudaSuccess ||
+      cudaMemset(bad, 0, sizeof(h)) != cudaSuccess ||
+      cudaMemcpy(d, a, bytes, cudaMemcpyHostToDevice) != cudaSuccess ||
+      cudaMemcpy(d + n, b, bytes, cudaMemcpyHostToDevice) != cudaSuccess)
+    rc = -1;
+  if (rc == 0) {
+    k_quotients<<<592, 256>>>(d, d + n, (long)n, bad);
+    if (cudaGetLastError() != cudaSuccess || cudaMemcpy(h, bad, sizeof(h), cudaMemcpyDeviceToHost) != cudaSuccess)
+      rc = -1;
+  }
+  if (rc) set_error("subfv_probe_quotients: CUDA error");
+  for (int k = 0; rc == 0 && k < 4; ++k) mismatches[k] = (int64_t)h[k];
+  if (d) cudaFree(d);
+  if (bad) cudaFree(bad);
+  return rc;
+}
