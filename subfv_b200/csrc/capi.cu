@@ -239,6 +239,7 @@ int subfv_mesh_create_from_topology(const subfv_topology* tp, int b2d, subfv_mes
 
 int subfv_mesh_destroy(subfv_mesh* m) {
   if (!m) return 0;
+  *m->alive = false;
   // scratch of the stateless calls (allocated on first use only); a mesh that never
   // needed it is released without any device-wide synchronisation
   void* scratch[] = {m->stage, m->sol6, m->rhs6, m->mass, m->sc};

@@ -1,5 +1,8 @@
 // Opaque handle types of the C-ABI, shared by the translation units that implement it.
 #pragma once
+#include <atomic>
+#include <memory>
+
 #include "../../include/subfv.h"
 #include "common.cuh"
 #include "mesh_dev.cuh"
@@ -15,6 +18,8 @@ struct subfv_mesh {
   // the backward-Euler Jacobian's host pattern, built on first use and kept with the mesh
   void* imp_pattern = nullptr;
   void (*imp_pattern_free)(void*) = nullptr;
+  // false once the mesh is destroyed: a state that outlives it has no stream to free on
+  std::shared_ptr<std::atomic<bool>> alive = std::make_shared<std::atomic<bool>>(true);
 };
 
 namespace subfv {

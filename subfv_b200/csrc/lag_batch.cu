@@ -19,6 +19,7 @@
 
 #include "handles.cuh"
 #include "lagrange.cuh"
+#include "pool.cuh"
 
 using namespace subfv;
 
@@ -78,13 +79,6 @@ struct subfv_lag_batch {
 };
 
 namespace {
-
-template <class T>
-int dalloc_async(T** p, size_t n, cudaStream_t s) {
-  SUBFV_CUDA(cudaMallocAsync((void**)p, std::max<size_t>(n, 1) * sizeof(T), s));
-  SUBFV_CUDA(cudaMemsetAsync(*p, 0, std::max<size_t>(n, 1) * sizeof(T), s));
-  return 0;
-}
 
 void slot_free_state(Slot& q, cudaStream_t s) {
   if (q.sol6) cudaFreeAsync(q.sol6, s);
@@ -295,10 +289,10 @@ int subfv_lag_batch_add(subfv_lag_batch* b, subfv_mesh* m, int take_mesh, const 
   cudaStream_t s = d.stream;
   const size_t ne = d.ne;
   double *stage = nullptr, *mstage = nullptr;
-  if (cudaMallocAsync((void**)&q.sol6, kRec * ne * sizeof(double), s) != cudaSuccess ||
-      cudaMallocAsync((void**)&q.rhs6, kRhs * ne * sizeof(double), s) != cudaSuccess ||
-      cudaMallocAsync((void**)&stage, 5 * ne * sizeof(double), s) != cudaSuccess ||
-      cudaMallocAsync((void**)&mstage, ne * sizeof(double), s) != cudaSuccess) {
+  if (pool_alloc((void**)&q.sol6, kRec * ne * sizeof(double), s) ||
+      pool_alloc((void**)&q.rhs6, kRhs * ne * sizeof(double), s) ||
+      pool_alloc((void**)&stage, 5 * ne * sizeof(double), s) ||
+      pool_alloc((void**)&mstage, ne * sizeof(double), s)) {
     slot_free_state(q, s);
     set_error("subfv_lag_batch_add: device allocation failed");
     return -1;

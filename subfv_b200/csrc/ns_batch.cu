@@ -17,6 +17,7 @@
 
 #include "handles.cuh"
 #include "ns.cuh"
+#include "pool.cuh"
 
 using namespace subfv;
 
@@ -86,7 +87,7 @@ namespace {
 
 template <class T>
 int dalloc_async(T** p, size_t n, cudaStream_t s) {
-  SUBFV_CUDA(cudaMallocAsync((void**)p, std::max<size_t>(n, 1) * sizeof(T), s));
+  if (pool_alloc((void**)p, std::max<size_t>(n, 1) * sizeof(T), s)) return -1;
   SUBFV_CUDA(cudaMemsetAsync(*p, 0, std::max<size_t>(n, 1) * sizeof(T), s));
   return 0;
 }
@@ -336,7 +337,7 @@ int subfv_ns_batch_add(subfv_ns_batch* b, subfv_mesh* m, int take_mesh, const do
       dalloc_async(&q.partial, 6 * (size_t)ns_partial_blocks(d), s) ||
       (o2 && (dalloc_async(&q.U1, kRec * ne, s) || dalloc_async(&q.rhs2, kRhs * ne, s) ||
               dalloc_async(&q.ngrad, 15 * nv, s) || dalloc_async(&q.grad, 15 * ne, s))) ||
-      cudaMallocAsync((void**)&stage, 5 * ne * sizeof(double), s) != cudaSuccess) {
+      pool_alloc((void**)&stage, 5 * ne * sizeof(double), s)) {
     slot_free_state(q, s);
     return -1;
   }

@@ -9,6 +9,7 @@
 #include "handles.cuh"
 #include "ns.cuh"
 #include "ns_diffusion.cuh"
+#include "pool.cuh"
 
 using namespace subfv;
 
@@ -26,6 +27,8 @@ struct ImplicitCtx {
 
 struct subfv_ns_state {
   subfv_mesh* m = nullptr;
+  std::shared_ptr<std::atomic<bool>> mesh_alive;
+  char* arena = nullptr;  // one allocation that holds every buffer below
   NsParams P{};
   double *U0 = nullptr, *U1 = nullptr, *fs = nullptr, *rhs1 = nullptr, *rhs2 = nullptr;
   double *ngrad = nullptr, *grad = nullptr, *delta = nullptr, *partial = nullptr, *stage = nullptr;
@@ -70,14 +73,28 @@ int check_cfg(const subfv_ns_cfg* c) {
   return 0;
 }
 
-// zeroed on the stream that later fills the buffer (the mesh's non-blocking stream does
-// not order against the legacy default stream)
-template <class T>
-int dalloc(T** p, size_t n, cudaStream_t s) {
-  SUBFV_CUDA(cudaMalloc((void**)p, std::max<size_t>(n, 1) * sizeof(T)));
-  SUBFV_CUDA(cudaMemsetAsync(*p, 0, std::max<size_t>(n, 1) * sizeof(T), s));
-  return 0;
-}
+// The buffers of a state, carved from one pool allocation: add() each, then one
+// allocation, zeroed on the stream that later fills the buffers (the mesh's non-blocking
+// stream does not order against the legacy default stream), then the pointers are set.
+struct Arena {
+  struct Part {
+    void** p;
+    size_t at;
+  };
+  std::vector<Part> parts;
+  size_t bytes = 0;
+  template <class T>
+  void add(T** p, size_t n) {
+    parts.push_back({(void**)p, bytes});
+    bytes += (std::max<size_t>(n, 1) * sizeof(T) + 255) & ~(size_t)255;
+  }
+  int make(char** base, cudaStream_t s) {
+    if (pool_alloc((void**)base, bytes, s)) return -1;
+    SUBFV_CUDA(cudaMemsetAsync(*base, 0, bytes, s));
+    for (const Part& q : parts) *q.p = *base + q.at;
+    return 0;
+  }
+};
 
 // One iteration of ns_main.F90:83-107 (graph-capturable).
 void enqueue_ns_step(subfv_ns_state* s) {
@@ -210,16 +227,20 @@ int subfv_ns_state_create(subfv_mesh* m, const subfv_ns_cfg* cfg, const double* 
   // per vertex (one per subface) shortens each vertex's serial chain (Gresho 64x64: 0.39
   // against 0.48 ms per iteration); subfv_ns_state_set_node_kernel overrides it
   if (d.nv < kSmallMeshVertices) s->P.node_group = 1;
+  s->mesh_alive = m->alive;
   const size_t ne = d.ne, nv = d.nv, nse = d.nse;
-  cudaStream_t q = d.stream;
-  if (dalloc(&s->U0, kRec * ne, q) || dalloc(&s->U1, kRec * ne, q) || dalloc(&s->fs, kNsFs * nse, q) ||
-      dalloc(&s->rhs1, kRhs * ne, q) || dalloc(&s->rhs2, kRhs * ne, q) || dalloc(&s->ngrad, 15 * nv, q) ||
-      dalloc(&s->grad, 15 * ne, q) || dalloc(&s->delta, 5 * ne, q) ||
-      dalloc(&s->partial, 6 * (size_t)ns_partial_blocks(d), q) || dalloc(&s->stage, 5 * ne, q) ||
-      dalloc(&s->sc, 1, q)) {
-    subfv_ns_state_destroy(s);
-    return -1;
-  }
+  Arena mem;
+  mem.add(&s->U0, kRec * ne);
+  mem.add(&s->U1, kRec * ne);
+  mem.add(&s->fs, kNsFs * nse);
+  mem.add(&s->rhs1, kRhs * ne);
+  mem.add(&s->rhs2, kRhs * ne);
+  mem.add(&s->ngrad, 15 * nv);
+  mem.add(&s->grad, 15 * ne);
+  mem.add(&s->delta, 5 * ne);
+  mem.add(&s->partial, 6 * (size_t)ns_partial_blocks(d));
+  mem.add(&s->stage, 5 * ne);
+  mem.add(&s->sc, 1);
   if (s->P.diff) {
     // periodic nodes use the union stencil of their images (mesh_dev.cuh)
     if (ensure_diffusion_stencil(&d)) {
@@ -235,10 +256,16 @@ int subfv_ns_state_create(subfv_mesh* m, const subfv_ns_cfg* cfg, const double* 
     }
     s->D = diff_params_from(*cfg, d);
     s->P.diff_kd = s->D.kd;
-    if (diffusion_prepare(smem) || dalloc(&s->dterm, (size_t)s->D.kd * nse, q) || dalloc(&s->mu0c, 1, q)) {
+    mem.add(&s->dterm, (size_t)s->D.kd * nse);
+    mem.add(&s->mu0c, 1);
+    if (diffusion_prepare(smem)) {
       subfv_ns_state_destroy(s);
       return -1;
     }
+  }
+  if (mem.make(&s->arena, d.stream)) {
+    subfv_ns_state_destroy(s);
+    return -1;
   }
   NsScalars h{};
   h.dtred = 1e10;
@@ -291,11 +318,12 @@ int subfv_ns_state_destroy(subfv_ns_state* s) {
     delete c;
   }
   if (s->graph) cudaGraphExecDestroy(s->graph);
-  double* bufs[] = {s->U0, s->U1, s->fs, s->rhs1, s->rhs2, s->ngrad, s->grad, s->delta, s->partial, s->stage};
-  for (double* b : bufs) cudaFree(b);
-  cudaFree(s->sc);
-  cudaFree(s->dterm);
-  cudaFree(s->mu0c);
+  if (s->arena) {
+    // after the work queued on the mesh's stream; cudaFree waits for it when the mesh, and
+    // its stream, went first
+    if (*s->mesh_alive) cudaFreeAsync(s->arena, s->m->d.stream);
+    else cudaFree(s->arena);
+  }
   delete s;
   return 0;
 }
