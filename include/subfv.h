@@ -40,8 +40,9 @@ int subfv_probe_fp64_fma(int iters, double* tflops, double* ms);
  * division. */
 int subfv_probe_div_const(const double* x, int64_t n, int64_t* mismatches);
 /* Checks the kernels' quotient and square root (zero-safe forms of / and sqrt) against
-   the operators on n pairs: mismatches[0..3] counts FP64 quotients a / b, FP64 roots of
-   a, FP32 quotients and FP32 roots whose bits differ (two NaNs agree). */
+   the operators on n pairs: mismatches[0..4] counts FP64 quotients a / b, FP64 roots of
+   a, FP32 quotients, FP32 roots and FP64 quotients from 1 / b whose bits differ (two
+   NaNs agree). */
 int subfv_probe_quotients(const double* a, const double* b, int64_t n, int64_t* mismatches);
 
 /* ---------------------------------------------------------------------------------

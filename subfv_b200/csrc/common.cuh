@@ -86,6 +86,33 @@ __device__ inline float qsqrt(float x) {
   return x == 0.0f ? x : s;
 }
 
+// a / b, bit-identical to the IEEE quotient, from the correctly rounded reciprocal
+// y = 1.0 / b, for denominators that several numerators share: a first quotient, one
+// correction that makes it faithful, and Markstein's final correction, exact for a
+// correctly rounded reciprocal and a faithful quotient (P. Markstein, IBM J. Res. Dev.
+// 34(1), 1990). a and b between 2^-400 and 2^400 in magnitude, so that no step under- or
+// overflows; a zero numerator's quotient is a * y; anything else takes the division, which
+// the empty volatile asm keeps from being computed ahead of the branch (a call out of line
+// would make the kernels spill around it). 80-95 cycles a warp against qdiv's 129, and a
+// third of its instructions.
+__device__ inline bool exponent_in_reach(double x) {
+  return ((unsigned)__double2hiint(x) & 0x7fffffffu) - ((1023u - 400u) << 20) < (800u << 20);
+}
+__device__ inline double div_by(double a, double b, double y) {
+  const double q0 = a * y;
+  const double q1 = fma(fma(-b, q0, a), y, q0);
+  const double q = fma(fma(-b, q1, a), y, q1);
+  const bool z = a == 0.0;
+  if (!((z || exponent_in_reach(a)) && exponent_in_reach(y))) {
+    double n = a;
+    asm volatile("" : "+d"(n));
+    return n / b;
+  }
+  return z ? q0 : q;
+}
+// FP32: the division itself is short
+__device__ inline float div_by(float a, float b, float) { return qdiv(a, b); }
+
 // gfortran's inline NORM2 of a 3-vector: scaled sum of squares, scale starting at 1.
 __device__ inline double fnorm2_3(double a0, double a1, double a2) {
   // With every |a_i| <= 1 the scale stays 1, each a_i / scale is a_i exactly and a zero

@@ -262,6 +262,7 @@ int devmesh_create(const subfv_mesh_desc* d, DevMesh* m) {
   int max_vse = 0;
   for (int v = 0; v < nv; ++v) max_vse = std::max(max_vse, vse_off[v + 1] - vse_off[v]);
   m->max_vse = max_vse;
+  m->nvse = (int)vse.size();
   m->nvsf = nvsf;
   m->vsf_identity = ident ? 1 : 0;
   m->max_vsf = max_vsf;
@@ -314,6 +315,15 @@ int devmesh_create(const subfv_mesh_desc* d, DevMesh* m) {
     }
     for (int v = 0; v < nv; ++v) vorder[v] = v;
     std::stable_sort(vorder.begin(), vorder.end(), [&](int a, int b) { return vkey[a] < vkey[b]; });
+    // the tile node kernel's classes (positions of vorder, ascending subface counts)
+    bool fits = true;
+    for (int i = 0; i < nv; ++i) {
+      const int v = vorder[i], ns = vsf_off[v + 1] - vsf_off[v], nc = vse_off[v + 1] - vse_off[v];
+      const int cls = ns <= 8 ? 0 : ns <= 16 ? 1 : 2;
+      fits = fits && ns <= 32 && nc <= (4 << cls);
+      for (int c = cls; c < 3; ++c) m->tile_end[c] = i + 1;
+    }
+    if (!fits) m->tile_end[0] = m->tile_end[1] = m->tile_end[2] = 0;
   }
   if (upload(&m->forder, forder, B, s) || upload(&m->vorder, vorder, B, s)) return -1;
   if (upload(&m->x, x, B, s) || alloc(&m->vp, nv, B, s) || alloc(&m->vol_v, nv, B, s) || upload(&m->is_bound, isb, B, s) ||
@@ -382,7 +392,7 @@ void devmesh_free(DevMesh* m) {
                   m->vsf, m->p_node, m->vse_off, m->vse, m->csf_off, m->csf, m->status,
                   m->vel_off, m->vel, m->cse_sorted, m->frec, m->centry, m->fS, m->fpos, m->gface, m->gsub, m->forder, m->vorder,
                   m->dsf_off, m->dsf, m->dsf_se, m->dsf_seloc, m->dse_off, m->dse, m->dse_sfloc,
-                  m->dcache, m->dcache_off, m->npinv};
+                  m->dcache, m->dcache_off, m->npinv, m->vslot, m->vcorner};
   diffusion_cache_forget(m);
   // stream-ordered frees: they wait for the mesh stream's work but not for other
   // streams (a caller that used the mesh elsewhere orders that work first)

@@ -64,8 +64,25 @@ struct NsTable {
   int* hdr = nullptr;
   int cap = 0;
   int block_v = 128, group = 8, grid_v = 1, grid_c = 1;
+  // the tile node kernel's work: prefix of the problems' tiles (grid_v blocks share them
+  // out), and whether every problem's mesh has its codes
+  int* wt = nullptr;
+  int tiles = 0;
 };
 constexpr int kNsCellBlock = 128;
+// The node kernel in tiles of vertices (ns_node_tile.cu): multi_point without excluded
+// boundary vertices and two_wave, on meshes whose vertices have at most 32 subfaces.
+// ensure_node_codes builds its per-mesh codes on first use, on the mesh's stream.
+// Their bytes are charged with a state on the mesh (node_codes_bytes), not with the mesh,
+// which holds none of them until then.
+int ensure_node_codes(DevMesh* m);
+int64_t node_codes_bytes(const DevMesh& m);
+int node_tiles(const DevMesh& m);  // blocks of the tile node kernel
+bool node_tile_serves(const DevMesh& m, const NsParams& P);
+bool node_tile_serves(const NsTable& t, const NsParams& P);
+void launch_node_tile(const DevMesh& m, const NsParams& P, const double* U, const double* grad, double* fs, int so,
+                      const NsScalars* sc);
+void launch_kb_node_tile(const NsTable& t, const NsParams& P, cudaStream_t s, int which, int so);
 // One step of the time loop for every problem of the table, in shared launches.
 void launch_ns_batch_step(const NsTable& t, const NsParams& P, cudaStream_t s);
 

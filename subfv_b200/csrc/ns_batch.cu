@@ -49,7 +49,7 @@ int64_t state_bytes(const DevMesh& d, int second_order) {
   const int64_t ne = d.ne, nv = d.nv, nse = d.nse;
   const int64_t o1 = kRec * ne + kNsFs * nse + kRhs * ne + 5 * ne + 6 * (int64_t)ns_partial_blocks(d);
   const int64_t o2 = kRec * ne + kRhs * ne + 15 * nv + 15 * ne;
-  return 8 * (o1 + (second_order ? o2 : 0));
+  return 8 * (o1 + (second_order ? o2 : 0)) + node_codes_bytes(d);
 }
 
 }  // namespace
@@ -66,7 +66,7 @@ struct subfv_ns_batch {
   // device table and its pinned host staging (double-buffered staging)
   NsTable tab{};
   NsItem* h_items[2] = {nullptr, nullptr};
-  int* h_w[2] = {nullptr, nullptr};  // [wv (cap+1) | wc (cap+1) | hdr (4)]
+  int* h_w[2] = {nullptr, nullptr};  // [wv (cap+1) | wc (cap+1) | wt (cap+1) | hdr (4)]
   cudaEvent_t stage_ev[2] = {nullptr, nullptr};
   int stage_cur = 0;
   bool dirty = true;
@@ -127,20 +127,27 @@ int table_upload(subfv_ns_batch* b) {
   NsItem* it = b->h_items[k];
   int* wv = b->h_w[k];
   int* wc = wv + (b->cap + 1);
-  int* hdr = wc + (b->cap + 1);
+  int* wt = wc + (b->cap + 1);
+  int* hdr = wt + (b->cap + 1);
   const int n = (int)b->order.size();
-  int group = 8;
-  for (int i = 0; i < n; ++i) group = std::max(group, ns_node_lanes(b->slots[b->order[i]].mesh->d));
-  if (group != b->tab.group) {  // the captured step loop launches the node kernel for one group size
+  int group = 8, tiles = 1;
+  for (int i = 0; i < n; ++i) {
+    const DevMesh& d = b->slots[b->order[i]].mesh->d;
+    group = std::max(group, ns_node_lanes(d));
+    tiles = tiles && d.node_codes > 0;
+  }
+  // the captured step loop launches one node kernel, for one group size
+  if (n && (group != b->tab.group || tiles != b->tab.tiles)) {
     if (b->graph) {
       SUBFV_CUDA(cudaStreamSynchronize(b->stream));
       cudaGraphExecDestroy(b->graph);
       b->graph = nullptr;
     }
     b->tab.group = group;
+    b->tab.tiles = tiles;
   }
   const int nbv = b->tab.block_v;  // vertices per work block
-  wv[0] = wc[0] = 0;
+  wv[0] = wc[0] = wt[0] = 0;
   for (int i = 0; i < n; ++i) {
     Slot& q = b->slots[b->order[i]];
     NsItem& I = it[i];
@@ -158,11 +165,13 @@ int table_upload(subfv_ns_batch* b) {
     I.sc = b->sc + b->order[i];
     wv[i + 1] = wv[i] + (I.m.nv + nbv - 1) / nbv;
     wc[i + 1] = wc[i] + (I.m.ne + kNsCellBlock - 1) / kNsCellBlock;
+    wt[i + 1] = wt[i] + node_tiles(I.m);
   }
   hdr[0] = n;
   if (n) SUBFV_CUDA(cudaMemcpyAsync(b->tab.items, it, n * sizeof(NsItem), cudaMemcpyHostToDevice, b->stream));
   SUBFV_CUDA(cudaMemcpyAsync(b->tab.wv, wv, (n + 1) * sizeof(int), cudaMemcpyHostToDevice, b->stream));
   SUBFV_CUDA(cudaMemcpyAsync(b->tab.wc, wc, (n + 1) * sizeof(int), cudaMemcpyHostToDevice, b->stream));
+  SUBFV_CUDA(cudaMemcpyAsync(b->tab.wt, wt, (n + 1) * sizeof(int), cudaMemcpyHostToDevice, b->stream));
   SUBFV_CUDA(cudaMemcpyAsync(b->tab.hdr, hdr, sizeof(int), cudaMemcpyHostToDevice, b->stream));
   SUBFV_CUDA(cudaEventRecord(b->stage_ev[k], b->stream));
   b->stage_cur ^= 1;
@@ -237,7 +246,7 @@ int subfv_ns_batch_create(const subfv_ns_cfg* cfg, int capacity, int64_t budget_
     return -1;
   };
   if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) return fail();
-  const size_t nw = 2 * (size_t)(capacity + 1) + 4;
+  const size_t nw = 3 * (size_t)(capacity + 1) + 4;
   if (cudaMalloc(&b->sc, capacity * sizeof(NsScalars)) != cudaSuccess ||
       cudaMalloc(&b->status, capacity * sizeof(unsigned)) != cudaSuccess ||
       cudaMalloc(&b->tab.items, capacity * sizeof(NsItem)) != cudaSuccess ||
@@ -247,7 +256,8 @@ int subfv_ns_batch_create(const subfv_ns_cfg* cfg, int capacity, int64_t budget_
   cudaMemsetAsync(b->status, 0, capacity * sizeof(unsigned), b->stream);
   cudaMemsetAsync(b->tab.wv, 0, nw * sizeof(int), b->stream);
   b->tab.wc = b->tab.wv + (capacity + 1);
-  b->tab.hdr = b->tab.wc + (capacity + 1);
+  b->tab.wt = b->tab.wc + (capacity + 1);
+  b->tab.hdr = b->tab.wt + (capacity + 1);
   b->tab.cap = capacity;
   b->tab.block_v = 128;
   b->tab.group = 8;
@@ -311,7 +321,7 @@ int subfv_ns_batch_add(subfv_ns_batch* b, subfv_mesh* m, int take_mesh, const do
     set_error("subfv_ns_batch_add: null argument");
     return -2;
   }
-  if (handle_ensure_full_geometry(m->d)) return -1;
+  if (handle_ensure_full_geometry(m->d) || ensure_node_codes(&m->d)) return -1;
   const DevMesh& d = m->d;
   if (ns_node_lanes(d) == 0) {
     set_error("subfv_ns_batch_add: a vertex has more than 32 subfaces or subcells");

@@ -127,8 +127,9 @@ extern "C" int subfv_probe_div_const(const double* x, int64_t n, int64_t* mismat
   return rc;
 }
 
-// Checks qdiv / qsqrt (common.cuh) against CUDA's operators on n pairs (a, b): counts per
-// operation (FP64 quotient, FP64 root of a, FP32 quotient, FP32 root) the pairs whose
+// Checks qdiv / qsqrt / div_by (common.cuh) against CUDA's operators on n pairs (a, b): counts per
+// operation (FP64 quotient, FP64 root of a, FP32 quotient, FP32 root, FP64 quotient from
+// the denominator's reciprocal) the pairs whose
 // results differ in any bit, two NaNs counting as equal. No counterpart in the reference.
 namespace {
 __device__ inline bool same(double p, double q) {
@@ -137,7 +138,7 @@ __device__ inline bool same(double p, double q) {
 __device__ inline bool same(float p, float q) { return __float_as_int(p) == __float_as_int(q) || (p != p && q != q); }
 __global__ void k_quotients(const double* __restrict__ a, const double* __restrict__ b, long n,
                             unsigned long long* __restrict__ bad) {
-  unsigned long long nb[4] = {0, 0, 0, 0};
+  unsigned long long nb[5] = {0, 0, 0, 0, 0};
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
     const double x = a[i], y = b[i];
     const float xf = (float)x, yf = (float)y;
@@ -145,8 +146,9 @@ __global__ void k_quotients(const double* __restrict__ a, const double* __restri
     nb[1] += !same(qsqrt(x), sqrt(x));
     nb[2] += !same(qdiv(xf, yf), xf / yf);
     nb[3] += !same(qsqrt(xf), sqrtf(xf));
+    nb[4] += !same(div_by(x, y, 1.0 / y), x / y);
   }
-  for (int k = 0; k < 4; ++k)
+  for (int k = 0; k < 5; ++k)
     if (nb[k]) atomicAdd(bad + k, nb[k]);
 }
 }  // namespace
@@ -158,7 +160,7 @@ extern "C" int subfv_probe_quotients(const double* a, const double* b, int64_t n
   }
   double* d = nullptr;
   unsigned long long* bad = nullptr;
-  unsigned long long h[4] = {0, 0, 0, 0};
+  unsigned long long h[5] = {0, 0, 0, 0, 0};
   const size_t bytes = (size_t)n * sizeof(double);
   int rc = 0;
   if (cudaMalloc(&d, 2 * bytes + 1) != cudaSuccess || cudaMalloc(&bad, sizeof(h)) != cudaSuccess ||
@@ -172,7 +174,7 @@ extern "C" int subfv_probe_quotients(const double* a, const double* b, int64_t n
       rc = -1;
   }
   if (rc) set_error("subfv_probe_quotients: CUDA error");
-  for (int k = 0; rc == 0 && k < 4; ++k) mismatches[k] = (int64_t)h[k];
+  for (int k = 0; rc == 0 && k < 5; ++k) mismatches[k] = (int64_t)h[k];
   if (d) cudaFree(d);
   if (bad) cudaFree(bad);
   return rc;

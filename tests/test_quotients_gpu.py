@@ -31,8 +31,8 @@ def _pairs(kind):
 @pytest.mark.parametrize("kind", ["special", "bits", "states"])
 def test_quotients_have_the_operators_bits(native, cuda_ok, kind):
     a, b = (np.ascontiguousarray(x) for x in _pairs(kind))
-    bad = (C.c_int64 * 4)(-1, -1, -1, -1)
+    bad = (C.c_int64 * 5)(-1, -1, -1, -1, -1)
     pd = lambda x: x.ctypes.data_as(C.POINTER(C.c_double))
     with np.errstate(invalid="ignore"):
         assert native.subfv_probe_quotients(pd(a), pd(b), a.size, bad) == 0
-    assert list(bad) == [0, 0, 0, 0]
+    assert list(bad) == [0, 0, 0, 0, 0]
