@@ -14,8 +14,9 @@
 //   consumer of the block partials (every block of the next kernel, or one finishing
 //   block) sums them with the same fixed tree. Deterministic run to run; not the
 //   reference's left-to-right order.
-// * Gram-Schmidt (modified, as the reference's): the axpy of step i is fused with the dot
-//   product of step i+1, so one Arnoldi column of step j costs j passes over the vectors.
+// * Gram-Schmidt (modified, as the reference's): one launch per Arnoldi column keeps the
+//   new vector in registers and shared memory over all its projections (k_mgs_column);
+//   beyond its capacity, the axpy of step i is fused with the dot product of step i+1.
 // * One restart cycle's Arnoldi process (m columns) has no host decision in it: it is
 //   captured once per matrix and workspace as a CUDA graph and replayed.
 // * Givens rotations and the back substitution run on the host in the reference's order.
@@ -380,6 +381,163 @@ __global__ void __launch_bounds__(kRedThreads) k_normalize(const double* src, do
   for (long k = (long)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += T) y[k] = src[k] / h;
 }
 
+// One Arnoldi column's modified Gram-Schmidt and normalisation in one launch: the new
+// vector w = V_jj stays in the threads' registers (E elements each, further nes in shared
+// memory) while every projection h_i = (w, V_i), w -= h_i V_i runs, with one exchange
+// between the blocks per projection. What bounds it is that exchange: each block stores
+// its partial sum, block 0 sums them by a fixed tree and stores the total, which the
+// others wait for. (Every block reading all partials saves a hop but takes 11,000 cycles
+// with 148 blocks polling the same lines, against 3,000.) The slots of a cycle start as
+// kNoPartial and each is written once, so a reader waits for the value itself: no counters
+// to reset, and nothing else passes between the blocks, which therefore need no fence. The
+// launch is cooperative (all blocks resident); a wait that runs out sets *fail and ends the
+// block, and with it the others.
+// KEEP: V_i stays in registers from its dot product to its axpy, and V_{i+1} is loaded
+// during the exchange, so each basis vector is read once; without it (E = 16) twice, the
+// second time from L2. One launch per projection read w and V_i again and wrote w each
+// time: 6.5 us a projection at 296,000 unknowns, here 1.7.
+constexpr unsigned long long kNoPartial = ~0ull;
+constexpr int kMgsThreads = 1024;
+constexpr int kMgsSharedMax = 27;       // 216 KB of the SM's shared memory
+constexpr int kMgsSpin = 2000000;       // polls of an L2 word: about a second
+constexpr int kMgsLaneSlots = 5;        // block 0's lanes read the partials of up to 160 blocks
+constexpr int kMgsStride = 32 * kMgsLaneSlots + 16;  // a sum's words: the partials, then the total on a line of its own
+
+__device__ inline unsigned long long mgs_word(double v) {  // never the mark: another NaN in its place
+  const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
+  return bits == kNoPartial ? 0x7ff8000000000000ull : bits;
+}
+
+__device__ inline double mgs_sum(double s, unsigned long long* slots, unsigned* fail, bool* ok) {
+  __shared__ double part[32];
+  __shared__ unsigned long long total;
+  volatile unsigned long long* all = slots;
+  volatile unsigned long long* sum = slots + 32 * kMgsLaneSlots;
+  s = warp_tree(s);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const double v = warp_tree(part[threadIdx.x]);
+    if (blockIdx.x == 0) {
+      // all of a lane's slots in flight at once, until each holds a value
+      unsigned long long bits[kMgsLaneSlots];
+      const unsigned long long own = __shfl_sync(0xffffffffu, mgs_word(v), 0);
+      bool late = true;
+      for (int spin = 0; spin < kMgsSpin && late; ++spin) {
+#pragma unroll
+        for (int u = 0; u < kMgsLaneSlots; ++u) {
+          const int q = threadIdx.x + 32 * u;
+          bits[u] = q == 0 ? own : q < (int)gridDim.x ? all[q] : 0ull;
+        }
+        late = false;
+#pragma unroll
+        for (int u = 0; u < kMgsLaneSlots; ++u) late = late || bits[u] == kNoPartial;
+      }
+      double t = 0.0;
+#pragma unroll
+      for (int u = 0; u < kMgsLaneSlots; ++u) t = t + __longlong_as_double((long long)bits[u]);
+      late = __any_sync(0xffffffffu, late);
+      t = warp_tree(t);
+      if (threadIdx.x == 0) {
+        total = late ? kNoPartial : mgs_word(t);
+        if (!late) *sum = total;
+      }
+    } else if (threadIdx.x == 0) {
+      all[blockIdx.x] = mgs_word(v);
+      unsigned long long t = kNoPartial;
+      for (int spin = 0; spin < kMgsSpin && t == kNoPartial; ++spin) t = *sum;
+      total = t;
+    }
+    if (threadIdx.x == 0 && total == kNoPartial) *fail = 1u;
+  }
+  __syncthreads();
+  const unsigned long long t = total;
+  __syncthreads();  // the shared words are written again by the next sum
+  *ok = t != kNoPartial;
+  return __longlong_as_double((long long)t);
+}
+
+template <int E, bool KEEP>
+__global__ void __launch_bounds__(kMgsThreads, 1) k_mgs_column(double* V, long n, int jj, double* __restrict__ hcol,
+                                                               unsigned long long* slots, int nes, unsigned* fail) {
+  extern __shared__ double ws[];  // [nes][kMgsThreads]
+  const long T = (long)gridDim.x * kMgsThreads, k0 = (long)blockIdx.x * kMgsThreads + threadIdx.x;
+  double* wv = V + (size_t)(jj - 1) * n;
+  double w[E], cur[KEEP ? E : 1], nxt[KEEP ? E : 1];
+  bool ok = true;
+  double s = 0.0;
+#pragma unroll
+  for (int e = 0; e < E; ++e) w[e] = k0 + e * T < n ? wv[k0 + e * T] : 0.0;
+  if constexpr (KEEP) {
+#pragma unroll
+    for (int e = 0; e < E; ++e) cur[e] = k0 + e * T < n ? V[k0 + e * T] : 0.0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) nxt[e] = jj > 2 && k0 + e * T < n ? V[(size_t)n + k0 + e * T] : 0.0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) s = s + w[e] * cur[e];
+  } else {
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+      if (k0 + e * T < n) s = s + w[e] * V[k0 + e * T];
+    for (int e = 0; e < nes; ++e) {
+      const long k = k0 + (E + e) * T;
+      const double x = k < n ? wv[k] : 0.0;
+      ws[e * kMgsThreads + threadIdx.x] = x;
+      if (k < n) s = s + x * V[k];
+    }
+  }
+  double h = mgs_sum(s, slots, fail, &ok);
+  for (int i = 1; i <= jj - 1; ++i) {
+    if (!ok) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) hcol[i - 1] = h;
+    const bool more = i < jj - 1;
+    s = 0.0;
+    if constexpr (KEEP) {
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        w[e] = w[e] - h * cur[e];
+        s = s + w[e] * (more ? nxt[e] : w[e]);
+      }
+      const double* v2 = V + (size_t)(i + 1) * n;  // V_{i+2}
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        cur[e] = nxt[e];
+        if (i + 2 <= jj - 1 && k0 + e * T < n) nxt[e] = v2[k0 + e * T];
+      }
+    } else {
+      const double *v0 = V + (size_t)(i - 1) * n, *v1 = V + (size_t)i * n;
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const long k = k0 + e * T;
+        if (k < n) {
+          w[e] = w[e] - h * v0[k];
+          s = s + w[e] * (more ? v1[k] : w[e]);
+        }
+      }
+#pragma unroll 4
+      for (int e = 0; e < nes; ++e) {
+        const long k = k0 + (E + e) * T;
+        if (k < n) {
+          const double x = ws[e * kMgsThreads + threadIdx.x] - h * v0[k];
+          ws[e * kMgsThreads + threadIdx.x] = x;
+          s = s + x * (more ? v1[k] : x);
+        }
+      }
+    }
+    h = mgs_sum(s, slots + (size_t)i * kMgsStride, fail, &ok);
+  }
+  if (!ok) return;
+  const double nrm = sqrt(h);
+  if (blockIdx.x == 0 && threadIdx.x == 0) hcol[jj - 1] = nrm;
+#pragma unroll
+  for (int e = 0; e < E; ++e)
+    if (k0 + e * T < n) wv[k0 + e * T] = w[e] / nrm;
+  for (int e = 0; e < nes; ++e) {
+    const long k = k0 + (E + e) * T;
+    if (k < n) wv[k] = ws[e * kMgsThreads + threadIdx.x] / nrm;
+  }
+}
+
 __global__ void k_sub(const double* __restrict__ b, const double* __restrict__ w, double* __restrict__ r, long n) {
   const long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (k < n) r[k] = b[k] - w[k];
@@ -472,6 +630,11 @@ void bcsr_free(DevBcsr* A) {
   *A = DevBcsr();
 }
 
+namespace {
+// projections and norms of a cycle: jj sums in column jj = 2 .. krylov + 1
+size_t mgs_slots(int krylov) { return (size_t)krylov * (krylov + 3) / 2; }
+}  // namespace
+
 int gmres_work_alloc(GmresWork* W, long n, int krylov) {
   W->n = n;
   W->krylov = krylov;
@@ -484,7 +647,14 @@ int gmres_work_alloc(GmresWork* W, long n, int krylov) {
   SUBFV_CUDA(cudaMalloc(&W->ty, n * sizeof(double)));
   SUBFV_CUDA(cudaMalloc(&W->z, (krylov + 2) * sizeof(double)));
   SUBFV_CUDA(cudaMalloc(&W->partial, 2 * kRedBlocks * sizeof(double)));
-  SUBFV_CUDA(cudaMalloc(&W->H, (size_t)(krylov + 1) * krylov * sizeof(double)));
+  SUBFV_CUDA(cudaMalloc(&W->H, ((size_t)(krylov + 1) * krylov + 1) * sizeof(double)));  // and the fail word
+  int dev = 0, sms = 0;
+  SUBFV_CUDA(cudaGetDevice(&dev));
+  SUBFV_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  W->mgs_blocks = (int)std::min<long>(std::min(sms, 32 * kMgsLaneSlots), (n + kMgsThreads - 1) / kMgsThreads);
+  const long per = (n + (long)W->mgs_blocks * kMgsThreads - 1) / ((long)W->mgs_blocks * kMgsThreads);
+  W->mgs_per = per <= 16 + kMgsSharedMax ? (int)per : 0;
+  if (W->mgs_per) SUBFV_CUDA(cudaMalloc(&W->slots, mgs_slots(krylov) * kMgsStride * sizeof(unsigned long long)));
   SUBFV_CUDA(cudaMalloc(&W->scal, 8 * sizeof(double)));
   W->bytes = (size_t)n * (krylov + 7) * 8;
   return 0;
@@ -492,7 +662,7 @@ int gmres_work_alloc(GmresWork* W, long n, int krylov) {
 
 void gmres_work_free(GmresWork* W) {
   if (W->cycle) cudaGraphExecDestroy(W->cycle);
-  void* p[] = {W->V, W->r, W->w, W->zp, W->z, W->partial, W->H, W->scal, W->d, W->rr, W->ty};
+  void* p[] = {W->V, W->r, W->w, W->zp, W->z, W->partial, W->H, W->scal, W->d, W->rr, W->ty, W->slots};
   for (void* q : p)
     if (q) cudaFree(q);
   *W = GmresWork();
@@ -625,10 +795,37 @@ int bcsr_set_colors(DevBcsr* A, int ncs, const int* color) {
 }
 
 namespace {
+template <int E, bool KEEP>
+cudaError_t launch_mgs_e(GmresWork& W, int jj, double* hcol, unsigned long long* slots, unsigned* fail, cudaStream_t s) {
+  const int nes = W.mgs_per > E ? W.mgs_per - E : 0;
+  const size_t smem = (size_t)nes * kMgsThreads * sizeof(double);
+  if (smem) cudaFuncSetAttribute(k_mgs_column<E, KEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 kMgsSharedMax * kMgsThreads * (int)sizeof(double));
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(W.mgs_blocks);
+  cfg.blockDim = dim3(kMgsThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute a{};
+  a.id = cudaLaunchAttributeCooperative;
+  a.val.cooperative = 1;
+  cfg.attrs = &a;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_mgs_column<E, KEEP>, W.V, W.n, jj, hcol, slots, nes, fail);
+}
+// the fewest registers that hold a thread's elements (and its basis vector elements up to 8)
+cudaError_t launch_mgs(GmresWork& W, int jj, double* hcol, unsigned long long* slots, unsigned* fail, cudaStream_t s) {
+  if (W.mgs_per <= 1) return launch_mgs_e<1, true>(W, jj, hcol, slots, fail, s);
+  if (W.mgs_per <= 2) return launch_mgs_e<2, true>(W, jj, hcol, slots, fail, s);
+  if (W.mgs_per <= 4) return launch_mgs_e<4, true>(W, jj, hcol, slots, fail, s);
+  if (W.mgs_per <= 8) return launch_mgs_e<8, true>(W, jj, hcol, slots, fail, s);
+  return launch_mgs_e<16, false>(W, jj, hcol, slots, fail, s);
+}
+
 // One restart cycle's Arnoldi process: V_1 = r/|r| (|r|^2 from the partials that the
 // preceding device_norm2 left in W.partial), then columns 2..m+1 with modified
 // Gram-Schmidt, H on the device. Launch-only (no host decision), so it can be captured.
-void arnoldi_cycle(const DevBcsr& A, GmresWork& W, int precond, bool fp32) {
+cudaError_t arnoldi_cycle(const DevBcsr& A, GmresWork& W, int precond, bool fp32) {
   const int m = W.krylov;
   const long n = W.n;
   cudaStream_t s = A.stream;
@@ -636,7 +833,10 @@ void arnoldi_cycle(const DevBcsr& A, GmresWork& W, int precond, bool fp32) {
   double* pb = W.partial + kRedBlocks;
   auto Vc = [&](int j) { return W.V + (size_t)(j - 1) * n; };  // 1-based
   auto Hd = [&](int i, int j) { return W.H + (i - 1) + (size_t)(m + 1) * (j - 1); };
-  cudaMemsetAsync(W.H, 0, (size_t)(m + 1) * m * sizeof(double), s);
+  cudaMemsetAsync(W.H, 0, ((size_t)(m + 1) * m + 1) * sizeof(double), s);
+  unsigned* fail = reinterpret_cast<unsigned*>(W.H + (size_t)(m + 1) * m);
+  unsigned long long* slots = W.slots;
+  if (W.mgs_per) cudaMemsetAsync(slots, 0xff, mgs_slots(m) * kMgsStride * sizeof(unsigned long long), s);
   k_normalize<<<kRedBlocks, kRedThreads, 0, s>>>(W.r, Vc(1), pa, kRedBlocks, W.scal, n);
   for (int jj = 2; jj <= m + 1; ++jj) {
     if (precond) {
@@ -646,6 +846,12 @@ void arnoldi_cycle(const DevBcsr& A, GmresWork& W, int precond, bool fp32) {
     } else {
       launch_bcsr_spmv(A, Vc(jj - 1), Vc(jj), fp32);
     }
+    if (W.mgs_per) {
+      const cudaError_t e = launch_mgs(W, jj, Hd(1, jj - 1), slots, fail, s);
+      if (e != cudaSuccess) return e;
+      slots += (size_t)jj * kMgsStride;
+      continue;
+    }
     k_dot<<<kRedBlocks, kRedThreads, 0, s>>>(Vc(1), Vc(jj), n, pa);
     for (int i = 1; i <= jj - 1; ++i) {
       const double* nx = i < jj - 1 ? Vc(i + 1) : nullptr;  // the last one is |V_jj|^2
@@ -654,6 +860,7 @@ void arnoldi_cycle(const DevBcsr& A, GmresWork& W, int precond, bool fp32) {
     }
     k_normalize<<<kRedBlocks, kRedThreads, 0, s>>>(Vc(jj), Vc(jj), pa, kRedBlocks, Hd(jj, jj - 1), n);
   }
+  return cudaGetLastError();
 }
 
 // Replays the cycle from a graph captured for this matrix, workspace and mode.
@@ -669,8 +876,7 @@ int run_arnoldi_cycle(const DevBcsr& A, GmresWork& W, int precond, bool fp32) {
   if (!W.cycle) {
     cudaGraph_t g = nullptr;
     SUBFV_CUDA(cudaStreamBeginCapture(A.stream, cudaStreamCaptureModeThreadLocal));
-    arnoldi_cycle(A, W, precond, fp32);
-    const cudaError_t le = cudaGetLastError();
+    const cudaError_t le = arnoldi_cycle(A, W, precond, fp32);
     const cudaError_t ce = cudaStreamEndCapture(A.stream, &g);
     SUBFV_CUDA(le);
     SUBFV_CUDA(ce);
@@ -689,7 +895,7 @@ int gmres_device(const DevBcsr& A, GmresWork& W, double* x, const double* b, dou
   const int m = W.krylov;
   const long n = W.n;
   cudaStream_t s = A.stream;
-  std::vector<double> H((size_t)(m + 1) * m), y(m + 1), c(m + 1), sn(m + 1), z(m + 1);
+  std::vector<double> H((size_t)(m + 1) * m + 1), y(m + 1), c(m + 1), sn(m + 1), z(m + 1);
   auto h = [&](int i, int j) -> double& { return H[(i - 1) + (size_t)(m + 1) * (j - 1)]; };
   st->conv = 0;
   SUBFV_CUDA(cudaMemsetAsync(x, 0, n * sizeof(double), s));
@@ -714,7 +920,11 @@ int gmres_device(const DevBcsr& A, GmresWork& W, double* x, const double* b, dou
     SUBFV_CUDA(cudaMemcpyAsync(H.data(), W.H, H.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
     SUBFV_CUDA(cudaStreamSynchronize(s));
     SUBFV_CUDA(cudaGetLastError());
-    if (j == 1 && H_first_host) std::memcpy(H_first_host, H.data(), H.size() * sizeof(double));
+    if (H.back() != 0.0) {
+      set_error("gmres: a block of the Gram-Schmidt kernel waited too long for the others");
+      return -1;
+    }
+    if (j == 1 && H_first_host) std::memcpy(H_first_host, H.data(), (size_t)(m + 1) * m * sizeof(double));
     int nr = m, i;
     for (i = 1; i <= m; ++i) {  // Givens rotations (:1634-1658)
       for (int k = 2; k <= i; ++k) {

@@ -47,6 +47,10 @@ struct GmresWork {
   double *partial = nullptr, *H = nullptr, *scal = nullptr;
   double *d = nullptr, *rr = nullptr;  // refinement correction and residual
   double* ty = nullptr;                 // the LU-SGS forward sweep
+  // k_mgs_column: its blocks, the elements a thread holds (0: the vector does not fit), and
+  // the blocks' partial sums of a cycle
+  int mgs_blocks = 0, mgs_per = 0;
+  unsigned long long* slots = nullptr;
   size_t bytes = 0;
   cudaGraphExec_t cycle = nullptr;  // the captured Arnoldi cycle and what it was captured for
   uintptr_t cycle_key[10] = {};
