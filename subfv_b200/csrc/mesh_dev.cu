@@ -262,7 +262,6 @@ int devmesh_create(const subfv_mesh_desc* d, DevMesh* m) {
   int max_vse = 0;
   for (int v = 0; v < nv; ++v) max_vse = std::max(max_vse, vse_off[v + 1] - vse_off[v]);
   m->max_vse = max_vse;
-  m->nvse = (int)vse.size();
   m->nvsf = nvsf;
   m->vsf_identity = ident ? 1 : 0;
   m->max_vsf = max_vsf;
@@ -318,9 +317,8 @@ int devmesh_create(const subfv_mesh_desc* d, DevMesh* m) {
     // the tile node kernel's classes (positions of vorder, ascending subface counts)
     bool fits = true;
     for (int i = 0; i < nv; ++i) {
-      const int v = vorder[i], ns = vsf_off[v + 1] - vsf_off[v], nc = vse_off[v + 1] - vse_off[v];
-      const int cls = ns <= 8 ? 0 : ns <= 16 ? 1 : 2;
-      fits = fits && ns <= 32 && nc <= (4 << cls);
+      const int ns = vsf_off[vorder[i] + 1] - vsf_off[vorder[i]], cls = ns <= 8 ? 0 : ns <= 16 ? 1 : 2;
+      fits = fits && ns <= 32;
       for (int c = cls; c < 3; ++c) m->tile_end[c] = i + 1;
     }
     if (!fits) m->tile_end[0] = m->tile_end[1] = m->tile_end[2] = 0;

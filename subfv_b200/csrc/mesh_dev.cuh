@@ -29,7 +29,6 @@ struct DevMesh {
   int b2d = 1;
   int vsf_identity = 0;  // vsf[p] == p for every p (no periodic extension)
   int max_vsf = 0, max_vse = 0;  // the most subfaces / subcells around one vertex
-  int nvse = 0;                  // entries of vse
   int max_evc = 0;               // the most vertices of one cell
   // vertices
   double4* x = nullptr;
@@ -110,8 +109,8 @@ struct DevMesh {
   // The tile node kernel's codes of every (vertex, subface) and (vertex, subcell) pair
   // (ns_node_tile.cu, k_build_node_codes), built by the first explicit Euler state on the
   // mesh; node_codes: 1 built, -1 the mesh's vertices do not fit them, 0 not tried.
-  // tile_end: how many vertices of vorder have at most 8, 16 and 32 subfaces, with at
-  // most 4, 8 and 16 corners (0 in all when some vertex has more).
+  // tile_end: how many vertices of vorder have at most 8, 16 and 32 subfaces (0 in all when
+  // some vertex has more).
   int2* vslot = nullptr;
   int4* vcorner = nullptr;
   int node_codes = 0;

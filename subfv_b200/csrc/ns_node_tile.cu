@@ -44,6 +44,7 @@ constexpr int kTileThreads = 256, kTileBlock = kTileThreads + 32;
 // iterations: 14.9 against 16.3 ms; 64 tubes: 133 against 145 ms); shared memory, 59 KB a
 // block, allows three as well.
 constexpr int kTileBlocksPerSm = 3;
+constexpr int kTileCorners = kTileThreads / 2;  // a vertex has at most half as many corners as positions
 // log2 of a tile's vertices by class: the vertices with up to 8, 16 and 32 subfaces
 __host__ __device__ constexpr int tile_log2(int cls) { return 5 - cls; }
 
@@ -58,6 +59,7 @@ struct TileSmem {
   double term[12][kTileThreads];  // component c of the thread's subface
   double sum[12][32];
   double vn[3][32];
+  int nsf[32];
   T rec[kRecFields * kRecs];
 };
 
@@ -113,8 +115,8 @@ __device__ inline void tile_solver(const DevMesh& m, const int bc_style, const i
 // block calls.
 template <class T, class L, int SCH>
 __device__ void ns_node_tile(const DevMesh& m, const NsParams& P, const double* __restrict__ U,
-                             const double* __restrict__ grad, double* __restrict__ fs, const int so, const int t0,
-                             const int nvt, const int log2, const NsScalars* sc, TileSmem<T>& sm) {
+                             const double* __restrict__ grad, double* __restrict__ fs, const int so, const int tile,
+                             const int t0, const int nvt, const int log2, const NsScalars* sc, TileSmem<T>& sm) {
   using AL = typename std::conditional<SCH == 4, T, L>::type;
   if (threadIdx.x >= kTileThreads) {
     __syncthreads();  // corner records
@@ -125,31 +127,27 @@ __device__ void ns_node_tile(const DevMesh& m, const NsParams& P, const double* 
   const int tv = 1 << log2;                                          // vertices, and threads between positions
   const int x = threadIdx.x & (tv - 1), w = threadIdx.x >> log2;     // this thread's vertex and position
   const int S = kTileThreads >> log2;                                // positions
-  const bool live = x < nvt;
-  const int v = live ? m.vorder[t0 + x] : 0;
-  const int p0 = m.vsf_off[v], nsfn = live ? m.vsf_off[v + 1] - p0 : 0;
-  const int q0 = m.vse_off[v], nsen = live ? m.vse_off[v + 1] - q0 : 0;
-  const bool mine = w < nsfn;
   // this thread's subface, loaded beside the corners' states
-  int2 vs = make_int2(0, 0);
+  const int2 vs = m.vslot[(size_t)kTileThreads * tile + threadIdx.x];
+  const bool mine = vs.x >= 0;
+  const int nsfn = mine ? (vs.y >> 26) + 1 : 0;
   double n[4] = {0.0, 0.0, 0.0, 0.0};
   if (mine) {
-    vs = m.vslot[p0 + w];
     const double4 sn = m.sfn[vs.x];
     n[0] = sn.x;
     n[1] = sn.y;
     n[2] = sn.z;
     n[3] = sn.w;
   }
-  if (w < nsen) {
-    const int c = m.vcorner[q0 + w].y;
+  const int c = threadIdx.x < kTileCorners ? m.vcorner[(size_t)kTileCorners * tile + threadIdx.x].y : -1;
+  if (c >= 0) {
     double u64[5];
     ld5(U, c, u64);
     T u[5], ws[5];
     for (int i = 0; i < 5; ++i) u[i] = (T)u64[i];
     T ir = c2p_ir(u, ws);
     if (so) {
-      const double4 cc = m.cc[c], xv = m.x[v];
+      const double4 cc = m.cc[c], xv = m.x[m.vorder[t0 + x]];
       const T dx[3] = {(T)(xv.x - cc.x), (T)(xv.y - cc.y), (T)(xv.z - cc.z)};
       const double* g = grad + 15 * (size_t)c;
       for (int i = 0; i < 5; ++i) {
@@ -161,12 +159,13 @@ __device__ void ns_node_tile(const DevMesh& m, const NsParams& P, const double* 
     }
     put_record<T, AL>(sm.rec + (w << log2) + x, ws, ir);
   }
+  if (w == 0) sm.nsf[x] = nsfn;
   __syncthreads();
-  const int kl = vs.y & 31;
-  int kr = (vs.y >> 5) & 31;
+  const int kl = mine ? vs.y & 31 : 0;
+  int kr = mine ? (vs.y >> 5) & 31 : 0;
   bool wall = false;
   if (mine && kr == 31) {  // a boundary subface: its ghost state in a record of its own
-    const int y = -1 - (vs.y >> 10);
+    const int y = -1 - ((vs.y >> 10) & 0xffff);
     wall = is_wall(P, y);
     const T* r = sm.rec + (kl << log2) + x;
     const T nt[3] = {(T)n[0], (T)n[1], (T)n[2]};
@@ -234,6 +233,7 @@ __device__ void ns_node_tile(const DevMesh& m, const NsParams& P, const double* 
       for (int d = 0; d < 3; ++d) term[tc * (9 + d)] = b ? n[3] * n[d] : 0.0;
       for (int d = 0; d < 9; ++d) term[tc * d] = 0.0;  // a sum is never -0: adding +0 leaves it
     }
+    const int nsfx = sm.nsf[x];  // subfaces of this thread's vertex
     for (int iter = 1; iter <= 4; ++iter) {
       bool changed = iter == 1;
       if (mine && iter > 1) {
@@ -277,7 +277,7 @@ __device__ void ns_node_tile(const DevMesh& m, const NsParams& P, const double* 
         const int c = i >> log2;  // (i - threadIdx.x is a multiple of the tile's vertices: i is vertex x)
         const double* tr = &sm.term[c][x];
         double s = 0.0;
-        for (int j = 0; j < nsfn; ++j) s = s + tr[j << log2];
+        for (int j = 0; j < nsfx; ++j) s = s + tr[j << log2];
         sm.sum[c][x] = s;
       }
       __syncthreads();
@@ -354,20 +354,20 @@ __device__ void ns_node_tile(const DevMesh& m, const NsParams& P, const double* 
   }
   __syncthreads();
   // corner sums: a task per corner and half of the six components, in subface order
-  for (int k = w; k < 2 * nsen; k += S) {
-    const int corner = k >> 1, c0 = 3 * (k & 1);
-    const int4 vc = m.vcorner[q0 + corner];
-    if (vc.x < 0) continue;  // a periodic image's subcell: its sums are zero here
+  {
+    const int half = threadIdx.x / kTileCorners, c0 = 3 * half;
+    const int4 cs = m.vcorner[(size_t)kTileCorners * tile + threadIdx.x - half * kTileCorners];
+    if (cs.x < 0) return;  // no corner, or another vertex's subcell
     double s[3] = {0.0, 0.0, 0.0};
-    for (unsigned b = (unsigned)vc.z | (unsigned)vc.w; b; b &= b - 1) {
+    for (unsigned b = (unsigned)cs.z | (unsigned)cs.w; b; b &= b - 1) {
       const int j = __ffs(b) - 1;
       const double* tr = &sm.term[c0][(j << log2) + x];
-      if ((vc.z >> j) & 1)
+      if ((cs.z >> j) & 1)
         for (int i = 0; i < 3; ++i) s[i] = s[i] + tr[tc * i];
-      if ((vc.w >> j) & 1)
+      if ((cs.w >> j) & 1)
         for (int i = 0; i < 3; ++i) s[i] = s[i] + tr[tc * (6 + i)];
     }
-    double* out = fs + kNsFs * (size_t)vc.x + c0;
+    double* out = fs + kNsFs * (size_t)cs.x + c0;
     for (int i = 0; i < 3; ++i) out[i] = s[i];
   }
 }
@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(kTileBlock, kTileBlocksPerSm) k_ns_node_tile(D
   if (sc && sc->done) return;
   int log2, t0, nvt;
   tile_at(m, blockIdx.x, &log2, &t0, &nvt);
-  ns_node_tile<T, L, SCH>(m, P, U, grad, fs, so, t0, nvt, log2, sc, *reinterpret_cast<TileSmem<T>*>(g_tile_smem));
+  ns_node_tile<T, L, SCH>(m, P, U, grad, fs, so, blockIdx.x, t0, nvt, log2, sc, *reinterpret_cast<TileSmem<T>*>(g_tile_smem));
 }
 
 // the batched form: the tiles of every problem of the table (wt: their prefix) are shared
@@ -420,53 +420,79 @@ __global__ void __launch_bounds__(kTileBlock, kTileBlocksPerSm) kb_ns_node_tile(
     if (I.sc->done) continue;
     int log2, t0, nvt;
     tile_at(I.m, u - wt[lo], &log2, &t0, &nvt);
-    ns_node_tile<T, L, SCH>(I.m, P, which ? I.U1 : I.U0, I.grad, I.fs, so, t0, nvt, log2, I.sc,
+    ns_node_tile<T, L, SCH>(I.m, P, which ? I.U1 : I.U0, I.grad, I.fs, so, u - wt[lo], t0, nvt, log2, I.sc,
                             *reinterpret_cast<TileSmem<T>*>(g_tile_smem));
     __syncthreads();  // the corner sums' reads before the next tile's terms
   }
 }
 
-// vslot: per (vertex, list position p) its subface, and bits 0-4 the left cell's corner,
-// 5-9 the right cell's (31: boundary, with its tag from bit 10). vcorner: per (vertex,
-// corner q) the subcell its sums go to (-1: a periodic image's), its cell, and the
-// positions whose left / right flux enters its sums. fail: a cell of a subface is no
-// corner of the vertex.
+// The codes of a tile, laid out as its threads read them. vslot[256 tile + thread]: the
+// subface (-1: none), then from bit 0 its left cell's corner (5 bits), its right cell's (5
+// bits, 31: boundary), the boundary's tag (16 bits) and the vertex's subface count less one
+// (5 bits). vcorner[128 tile + thread]: the subcell that a corner's sums go to (-1: none),
+// its cell (-1: no corner) and the positions whose left / right flux enters its sums. A
+// vertex's corners are its own subcells, then the other cells of its subfaces (a periodic
+// vertex's list holds its images' subfaces). Both arrays start as -1. fail: a vertex has
+// more corners than the tile's class, or a tag beyond its bits.
 __global__ void k_build_node_codes(DevMesh m, int2* __restrict__ vslot, int4* __restrict__ vcorner, int* fail) {
-  const int v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= m.nv) return;
-  const int p0 = m.vsf_off[v], ns = m.vsf_off[v + 1] - p0;
-  const int q0 = m.vse_off[v], nc = m.vse_off[v + 1] - q0;
-  if (ns > 32 || nc > 30) {
-    *fail = 1;
-    return;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= m.nv) return;
+  const int cls = i < m.tile_end[0] ? 0 : i < m.tile_end[1] ? 1 : 2, log2 = tile_log2(cls);
+  int tile = 0, begin = 0;
+  for (int c = 0; c < cls; begin = m.tile_end[c++])
+    tile += (m.tile_end[c] - begin + (1 << tile_log2(c)) - 1) >> tile_log2(c);
+  tile += (i - begin) >> log2;
+  const int x = (i - begin) & ((1 << log2) - 1);
+  int2* slot = vslot + (size_t)kTileThreads * tile + x;
+  int4* corner = vcorner + (size_t)kTileCorners * tile + x;
+  const int v = m.vorder[i], p0 = m.vsf_off[v], ns = m.vsf_off[v + 1] - p0;
+  const int q0 = m.vse_off[v], nq = m.vse_off[v + 1] - q0, cap = 4 << cls;
+  int sub[16], cell[16], nc = 0;
+  unsigned lm[16], rm[16];
+  bool ok = true;
+  for (int q = 0; q < nq; ++q) {
+    const int s = m.vse[q0 + q];
+    if (m.se_vert[s] != v) continue;
+    if (nc == cap) {
+      ok = false;
+      break;
+    }
+    sub[nc] = s;
+    cell[nc] = m.se_elem[s];
+    lm[nc] = rm[nc] = 0u;
+    ++nc;
   }
-  unsigned lm[30], rm[30];
-  for (int k = 0; k < nc; ++k) lm[k] = rm[k] = 0u;
-  for (int j = 0; j < ns; ++j) {
+  auto corner_of = [&](int c) {
+    for (int k = 0; k < nc; ++k)
+      if (cell[k] == c) return k;
+    if (nc == cap) {
+      ok = false;
+      return 0;
+    }
+    sub[nc] = -1;
+    cell[nc] = c;
+    lm[nc] = rm[nc] = 0u;
+    return nc++;
+  };
+  for (int j = 0; ok && j < ns; ++j) {
     const int sf = m.vsf[p0 + j];
     const int2 lr = m.flr[m.sf_face[sf]];
-    int kl = -1, kr = lr.y < 0 ? 31 : -1;
-    for (int k = 0; k < nc; ++k) {
-      const int c = m.se_elem[m.vse[q0 + k]];
-      if (c == lr.x && kl < 0) kl = k;
-      if (lr.y >= 0 && c == lr.y && kr < 0) kr = k;
-    }
+    const int kl = corner_of(lr.x), kr = lr.y < 0 ? 31 : corner_of(lr.y);
     const unsigned tag = lr.y < 0 ? (unsigned)(-1 - lr.y) : 0u;
-    if (kl < 0 || kr < 0 || tag >= (1u << 21)) {
-      *fail = 1;
-      return;
-    }
-    vslot[p0 + j] = make_int2(sf, (int)((unsigned)kl | ((unsigned)kr << 5) | (tag << 10)));
+    if (tag > 0xffffu) ok = false;
+    slot[j << log2] = make_int2(sf, (int)((unsigned)kl | ((unsigned)kr << 5) | (tag << 10) | ((unsigned)(ns - 1) << 26)));
+    // the flux enters the sums of this vertex's subcells, by their positions in its list
     const int2 se = m.sf_se[sf];
-    if (m.se_vert[se.x] == v && m.se_loc[se.x] < nc) {
-      lm[m.se_loc[se.x]] |= 1u << j;
-      if (se.y >= 0 && m.se_vert[se.y] == v && m.se_loc[se.y] < nc) rm[m.se_loc[se.y]] |= 1u << j;
+    if (m.se_vert[se.x] == v && m.se_loc[se.x] < nq) {
+      for (int k = 0; k < nc; ++k)
+        if (sub[k] >= 0 && sub[k] == m.vse[q0 + m.se_loc[se.x]]) lm[k] |= 1u << j;
+      if (se.y >= 0 && m.se_vert[se.y] == v && m.se_loc[se.y] < nq)
+        for (int k = 0; k < nc; ++k)
+          if (sub[k] >= 0 && sub[k] == m.vse[q0 + m.se_loc[se.y]]) rm[k] |= 1u << j;
     }
   }
-  for (int k = 0; k < nc; ++k) {
-    const int s = m.vse[q0 + k];
-    vcorner[q0 + k] = make_int4(m.se_vert[s] == v ? s : -1, m.se_elem[s], (int)lm[k], (int)rm[k]);
-  }
+  for (int k = 0; k < nc; ++k) corner[k << log2] = make_int4(sub[k], cell[k], (int)lm[k], (int)rm[k]);
+  if (!ok) *fail = 1;
 }
 
 template <class T, class L, int SCH>
@@ -498,7 +524,7 @@ bool node_tile_serves(const DevMesh& m, const NsParams& P) { return m.node_codes
 bool node_tile_serves(const NsTable& t, const NsParams& P) { return t.tiles && tile_scheme(P); }
 
 int64_t node_codes_bytes(const DevMesh& m) {
-  return (int64_t)m.nvsf * (int64_t)sizeof(int2) + (int64_t)m.nvse * (int64_t)sizeof(int4);
+  return (int64_t)node_tiles(m) * (int64_t)(kTileThreads * sizeof(int2) + kTileCorners * sizeof(int4));
 }
 
 int ensure_node_codes(DevMesh* m) {
@@ -507,11 +533,13 @@ int ensure_node_codes(DevMesh* m) {
     m->node_codes = -1;
     return 0;
   }
-  const size_t nc = (size_t)m->nvse;
+  const size_t nt = node_tiles(*m), sb = nt * kTileThreads * sizeof(int2), cb = nt * kTileCorners * sizeof(int4);
   int* fail = nullptr;
-  SUBFV_CUDA(cudaMallocAsync((void**)&m->vslot, std::max<size_t>(m->nvsf, 1) * sizeof(int2), m->stream));
-  SUBFV_CUDA(cudaMallocAsync((void**)&m->vcorner, std::max<size_t>(nc, 1) * sizeof(int4), m->stream));
+  SUBFV_CUDA(cudaMallocAsync((void**)&m->vslot, sb, m->stream));
+  SUBFV_CUDA(cudaMallocAsync((void**)&m->vcorner, cb, m->stream));
   SUBFV_CUDA(cudaMallocAsync((void**)&fail, sizeof(int), m->stream));
+  SUBFV_CUDA(cudaMemsetAsync(m->vslot, 0xff, sb, m->stream));
+  SUBFV_CUDA(cudaMemsetAsync(m->vcorner, 0xff, cb, m->stream));
   SUBFV_CUDA(cudaMemsetAsync(fail, 0, sizeof(int), m->stream));
   k_build_node_codes<<<grid_for(m->nv, 128), 128, 0, m->stream>>>(*m, m->vslot, m->vcorner, fail);
   SUBFV_CUDA(cudaGetLastError());
