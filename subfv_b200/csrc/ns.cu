@@ -1235,33 +1235,38 @@ __device__ void ns_timedisc_body(const DevMesh& m, const NsParams& P, const doub
 }
 
 
-// scalar tail of add_timedisc_and_solve (:582-608); last_stage also advances t
+// scalar tail of add_timedisc_and_solve (:582-608); last_stage also advances t. Called by
+// every thread of a kTdBlock-thread block: the residual sums of the problem's blocks by a
+// fixed tree (a thread per block of partial sums, warps by shuffles, the warps in order),
+// then one thread's scalars. One thread adding the partials in block order waited on L2
+// for each eight of them: 23 of the kernel's 32 us at 305 blocks.
 __device__ void ns_finalize_body(NsScalars* sc, const NsParams& P, const double* __restrict__ partial, int nblocks,
                                  unsigned* status, int last_stage) {
   if (sc->done) {
-    sc->skip = 1;
+    if (threadIdx.x == 0) sc->skip = 1;
     return;
+  }
+  __shared__ double wsum[6][kTdBlock / 32];
+  double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  for (int b = threadIdx.x; b < nblocks; b += kTdBlock)
+#pragma unroll
+    for (int k = 0; k < 6; ++k) v[k] = v[k] + __ldcg(partial + 6 * (size_t)b + k);
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    const double x = warp_sum_tree(v[k]);
+    if ((threadIdx.x & 31) == 0) wsum[k][threadIdx.x >> 5] = x;
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  double res = 0.0, rv[5];
+  for (int k = 0; k < 6; ++k) {
+    double x = wsum[k][0];
+    for (int w = 1; w < kTdBlock / 32; ++w) x = x + wsum[k][w];
+    if (k == 0) res = x;
+    else rv[k - 1] = x;
   }
   double dt = P.cfl * sc->dtred;
   if (!P.lts) dt = fmin2(sc->tmax - sc->t + 1e-12, dt);
-  // the partial sums in block order, the loads of eight blocks issued before their adds
-  double res = 0.0, rv[5] = {0, 0, 0, 0, 0};
-  constexpr int kAhead = 8;
-  for (int b0 = 0; b0 < nblocks; b0 += kAhead) {
-    double buf[kAhead][6];
-#pragma unroll
-    for (int i = 0; i < kAhead; ++i)
-      if (b0 + i < nblocks)
-#pragma unroll
-        for (int k = 0; k < 6; ++k) buf[i][k] = __ldcg(partial + 6 * (size_t)(b0 + i) + k);
-#pragma unroll
-    for (int i = 0; i < kAhead; ++i)
-      if (b0 + i < nblocks) {
-        res = res + buf[i][0];
-#pragma unroll
-        for (int k = 0; k < 5; ++k) rv[k] = rv[k] + buf[i][1 + k];
-      }
-  }
   const double omega = __ldcg(&sc->omega);
   sc->omega_step = omega;  // for the update; the next stage's limiter starts afresh
   sc->omega = 1.0;
@@ -1281,9 +1286,9 @@ __device__ void ns_finalize_body(NsScalars* sc, const NsParams& P, const double*
 
 // The time discretisation of one problem with the stage's scalar tail folded in: each
 // block publishes its partial sums and limiter minimum, then counts itself in, and the
-// block that arrives last runs ns_finalize_body over all the blocks' partial sums (in
-// block order, whichever block that is, reading them from L2) and clears the count. No
-// block waits for another.
+// block that arrives last runs ns_finalize_body over all the blocks' partial sums (the same
+// tree whichever block that is, reading them from L2) and clears the count. No block waits
+// for another.
 template <bool DIFF>
 __global__ void __launch_bounds__(kTdBlock) k_ns_timedisc(DevMesh m, NsParams P, const double* __restrict__ U_rhs,
                                                           const double* __restrict__ rhs1,
@@ -1300,10 +1305,10 @@ __global__ void __launch_bounds__(kTdBlock) k_ns_timedisc(DevMesh m, NsParams P,
     last = atomicAdd(&sc->arrive, 1u) == gridDim.x - 1 ? 1 : 0;
   }
   __syncthreads();
-  if (last && threadIdx.x == 0) {
+  if (last) {
     __threadfence();
     ns_finalize_body(sc, P, partial, gridDim.x, m.status, last_stage);
-    sc->arrive = 0u;
+    if (threadIdx.x == 0) sc->arrive = 0u;
   }
 }
 
@@ -1427,12 +1432,13 @@ __global__ void __launch_bounds__(kTdBlock) kb_ns_timedisc(const NsItem* __restr
     __syncthreads();
   }
 }
-__global__ void kb_ns_finalize(const NsItem* __restrict__ it, const int* __restrict__ hdr, NsParams P,
-                               int last_stage) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= hdr[0]) return;
-  const NsItem& I = it[p];
-  ns_finalize_body(I.sc, P, I.partial, (I.m.ne + kTdBlock - 1) / kTdBlock, I.m.status, last_stage);
+__global__ void __launch_bounds__(kTdBlock) kb_ns_finalize(const NsItem* __restrict__ it, const int* __restrict__ hdr,
+                                                           NsParams P, int last_stage) {
+  for (int p = blockIdx.x; p < hdr[0]; p += gridDim.x) {  // a block per problem
+    const NsItem& I = it[p];
+    ns_finalize_body(I.sc, P, I.partial, (I.m.ne + kTdBlock - 1) / kTdBlock, I.m.status, last_stage);
+    __syncthreads();
+  }
 }
 __global__ void __launch_bounds__(128) kb_ns_apply(const NsItem* __restrict__ it, const int* __restrict__ wc,
                                                    const int* __restrict__ hdr, int stage, double a2) {
@@ -1776,7 +1782,7 @@ void launch_kb_node(const NsTable& t, const NsParams& P, cudaStream_t s, int whi
 }
 
 void launch_ns_batch_step(const NsTable& t, const NsParams& P, cudaStream_t s) {
-  const int gv = t.grid_v, gc = t.grid_c, nb = t.block_v, gp = grid_for(t.cap, 128);
+  const int gv = t.grid_v, gc = t.grid_c, nb = t.block_v;
   auto node = [&](int which, int so) { launch_kb_node(t, P, s, which, so); };
   auto rhs = [&](int which) {
     node(which, 0);
@@ -1791,7 +1797,7 @@ void launch_ns_batch_step(const NsTable& t, const NsParams& P, cudaStream_t s) {
   };
   auto stage = [&](int st, double a1, double a2, int last) {
     kb_ns_timedisc<<<gc, kTdBlock, 0, s>>>(t.items, t.wc, t.hdr, P, st, a1, a2);
-    kb_ns_finalize<<<gp, 128, 0, s>>>(t.items, t.hdr, P, last);
+    kb_ns_finalize<<<std::min(t.cap, 1184), kTdBlock, 0, s>>>(t.items, t.hdr, P, last);
     kb_ns_apply<<<gc, 128, 0, s>>>(t.items, t.wc, t.hdr, st, a2);
   };
   if (P.second_order) {
