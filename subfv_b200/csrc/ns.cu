@@ -558,14 +558,28 @@ __device__ inline double warp_sum_tree(double x) {
   return x;
 }
 
+// the primitive state of cell c, once per evaluation for the gradient kernels (a nodal
+// gradient reads it once per subface side, a slope limiter once per vertex of each
+// neighbour: up to 64 conversions of four quotients a cell)
+__device__ inline void put_prim(const double* __restrict__ U, double* __restrict__ prim, const int c) {
+  double u[5], w[5];
+  ld5(U, c, u);
+  c2p(u, w);
+  for (int k = 0; k < 5; ++k) prim[5 * (size_t)c + k] = w[k];
+}
+
 // compute_euler_flux scatter (:320-336) as a gather: rhs = 0 - corners in ascending
 // vertex order; sum_lambda = 1e-12 + corners. Block min of V / sum_lambda into *dtred.
 // called by every thread of a 128-thread block (block reduction inside)
+// With prim it also writes the cell's primitive state there (5 doubles), which the gradient
+// kernels read.
 __device__ void ns_gather_body(const DevMesh& m, const double* __restrict__ fs, double* __restrict__ rhs,
-                               NsScalars* sc, int reduce, const int c) {
+                               NsScalars* sc, int reduce, const int c, const double* __restrict__ U = nullptr,
+                               double* __restrict__ prim = nullptr) {
   if (sc && sc->done) return;
   double dmin = 1e10;
   if (c < m.ne) {
+    if (prim) put_prim(U, prim, c);
     double r[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, sl = 1e-12;
     // the corner records of four subcells at a time loaded before their sums, which run
     // in the list's order
@@ -607,8 +621,13 @@ __device__ void ns_gather_body(const DevMesh& m, const double* __restrict__ fs, 
 }
 
 __global__ void __launch_bounds__(128) k_ns_gather(DevMesh m, const double* __restrict__ fs, double* __restrict__ rhs,
-                                                   NsScalars* sc, int reduce) {
-  ns_gather_body(m, fs, rhs, sc, reduce, blockIdx.x * blockDim.x + threadIdx.x);
+                                                   NsScalars* sc, int reduce, const double* __restrict__ U,
+                                                   double* __restrict__ prim) {
+  ns_gather_body(m, fs, rhs, sc, reduce, blockIdx.x * blockDim.x + threadIdx.x, U, prim);
+}
+__global__ void __launch_bounds__(128) k_ns_prim(DevMesh m, const double* __restrict__ U, double* __restrict__ prim) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c < m.ne) put_prim(U, prim, c);
 }
 
 // The matrix of compute_nodal_grad (ns_euler_recon_module.F90:453-490) at vertex v,
@@ -643,99 +662,163 @@ __global__ void __launch_bounds__(128) k_ns_nodal_pinv(DevMesh m, double* __rest
     for (int e = 0; e < 3; ++e) npinv[9 * (size_t)v + 3 * d + e] = mat[d][e];
 }
 
-// compute_nodal_grad (ns_euler_recon_module.F90:453-490); ng[15] = g[5*d + var]. CACHED:
-// the pseudo-inverse comes from m.npinv (k_ns_nodal_pinv) instead of being formed here.
-template <bool CACHED>
-__device__ void ns_nodal_grad_body(const DevMesh& m, const double* __restrict__ U, double* __restrict__ ngrad,
-                                   const NsScalars* sc, const int v) {
+// A vertex's record of the second-order reconstruction (kNsVert doubles): its nodal gradient
+// g[5*d + var] (compute_nodal_grad, ns_euler_recon_module.F90:453-490), then what the cell
+// gradients need of it and every cell around it would compute again: per variable the
+// weight of methods 4-6 (the norm for method 3), and the extremes of the pressures and
+// densities of its cells (relaxed_maximum_principle), in the limiters' precision.
+enum { kVertWeight = 15, kVertPmin = 20, kVertPmax, kVertRmin, kVertRmax };
+static_assert(kVertRmax + 1 == kNsVert, "vertex record");
+
+// methods 4: V / (eps + |g|); 5, 6: V / (eps + |g|)^2; 3: |g|
+template <class T>
+__device__ inline double nodal_weight(int method, T vol, double g0, double g1, double g2) {
+  const T o = oi3<T>((T)g0, (T)g1, (T)g2);
+  if (method == 3) return (double)o;
+  const T q = (T)1e-3 + o;
+  return (double)(method == 4 ? vol / q : vol / (q * q));
+}
+// The folds (tmin2, tmax2) keep the first occurrence of their extreme and never take a NaN,
+// so folding a vertex's cells and then a cell's vertices returns the single fold's bits.
+template <class T>
+struct Extremes {
+  T pmin = sizeof(T) == 4 ? (T)3.0e38f : (T)1e100, pmax = 0, rmin = pmin, rmax = 0;
+  __device__ void fold(T plo, T phi, T rlo, T rhi) {
+    pmin = tmin2(pmin, plo);
+    pmax = tmax2(pmax, phi);
+    rmin = tmin2(rmin, rlo);
+    rmax = tmax2(rmax, rhi);
+  }
+  __device__ void cell(const double* __restrict__ U, const double* __restrict__ prim, const int c) {
+    if constexpr (sizeof(T) == 8) {
+      const double p = prim[5 * (size_t)c + 4], r = prim[5 * (size_t)c];
+      fold(p, p, r, r);
+    } else {
+      double u[5];
+      ld5(U, c, u);
+      T ut[5], w[5];
+      for (int k = 0; k < 5; ++k) ut[k] = (T)u[k];
+      c2p(ut, w);
+      fold(w[4], w[4], w[0], w[0]);
+    }
+  }
+};
+
+// the record's second part for a thread that holds the whole gradient o[15]
+template <class T>
+__device__ inline void put_limits(const DevMesh& m, const int method, const double* __restrict__ U,
+                                  const double* __restrict__ prim, const int v, double* o) {
+  if (method >= 3) {
+    const T vol = (T)m.vol_v[v];
+    for (int k = 0; k < 5; ++k) o[kVertWeight + k] = nodal_weight<T>(method, vol, o[k], o[5 + k], o[10 + k]);
+  }
+  Extremes<T> x;
+  for (int q = m.vel_off[v]; q < m.vel_off[v + 1]; ++q) x.cell(U, prim, m.vel[q]);
+  o[kVertPmin] = (double)x.pmin;
+  o[kVertPmax] = (double)x.pmax;
+  o[kVertRmin] = (double)x.rmin;
+  o[kVertRmax] = (double)x.rmax;
+}
+
+// the mesh's pseudo-inverses (k_ns_nodal_pinv) belong to its geometry
+__device__ inline bool has_nodal_pinv(const DevMesh& m) {
+  return m.npinv && !m.moving && m.npinv_epoch == m.geom_epoch;
+}
+
+// The vertex record, a thread per vertex; the pseudo-inverse comes from the mesh, or is
+// formed here when the mesh has none for its geometry.
+__device__ void ns_nodal_grad_body(const DevMesh& m, const NsParams& P, const double* __restrict__ U,
+                                   const double* __restrict__ prim, double* __restrict__ ngrad, const NsScalars* sc,
+                                   const int v) {
   if (sc && sc->done) return;
   if (v >= m.nv) return;
   double g[3][5] = {{0, 0, 0, 0, 0}, {0, 0, 0, 0, 0}, {0, 0, 0, 0, 0}};
-  double mat[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
   for (int p = m.vsf_off[v]; p < m.vsf_off[v + 1]; ++p) {
     const int sf = m.vsf[p];
     const int2 lr = m.flr[m.sf_face[sf]];
     if (lr.y < 0) continue;
-    double ul[5], ur[5], wl[5], wr[5];
-    ld5(U, lr.x, ul);
-    ld5(U, lr.y, ur);
-    c2p(ul, wl);
-    c2p(ur, wr);
+    const double *wl = prim + 5 * (size_t)lr.x, *wr = prim + 5 * (size_t)lr.y;
     const double4 sn = m.sfn[sf];
     const double n[3] = {sn.x, sn.y, sn.z};
-    for (int d = 0; d < 3; ++d)
-      for (int k = 0; k < 5; ++k) g[d][k] = g[d][k] + sn.w * (n[d] * (wr[k] - wl[k]));
-    if (!CACHED) {
-      const double4 cl = m.cc[lr.x], cr = m.cc[lr.y];
-      const double dxc[3] = {cr.x - cl.x, cr.y - cl.y, cr.z - cl.z};
-      for (int d = 0; d < 3; ++d)
-        for (int e = 0; e < 3; ++e) mat[d][e] = mat[d][e] + sn.w * (n[d] * dxc[e]);
+    for (int k = 0; k < 5; ++k) {
+      const double dw = wr[k] - wl[k];
+      for (int d = 0; d < 3; ++d) g[d][k] = g[d][k] + sn.w * (n[d] * dw);
     }
   }
-  if (CACHED) {
+  double mat[3][3];
+  if (has_nodal_pinv(m)) {
     for (int d = 0; d < 3; ++d)
       for (int e = 0; e < 3; ++e) mat[d][e] = m.npinv[9 * (size_t)v + 3 * d + e];
   } else {
+    nodal_grad_matrix(m, v, mat);
     pinv3(mat);
   }
   const bool bnd = m.is_bound[v] != 0;
-  double* o = ngrad + 15 * (size_t)v;
+  double* o = ngrad + kNsVert * (size_t)v;
   for (int d = 0; d < 3; ++d)
     for (int k = 0; k < 5; ++k) {
       double s = 0.0;
       for (int e = 0; e < 3; ++e) s = s + mat[d][e] * g[e][k];
       o[5 * d + k] = bnd ? 0.0 : s;
     }
+  if (P.method < 2) return;
+  if (P.precision == 2) put_limits<float>(m, P.method, U, prim, v, o);
+  else put_limits<double>(m, P.method, U, prim, v, o);
 }
 
-template <bool CACHED>
-__global__ void __launch_bounds__(128) k_ns_nodal_grad(DevMesh m, const double* __restrict__ U,
-                                                       double* __restrict__ ngrad, const NsScalars* sc) {
-  ns_nodal_grad_body<CACHED>(m, U, ngrad, sc, vert_at(m, blockIdx.x * blockDim.x + threadIdx.x));
+__global__ void __launch_bounds__(128) k_ns_nodal_grad(DevMesh m, NsParams P, const double* __restrict__ U,
+                                                       const double* __restrict__ prim, double* __restrict__ ngrad,
+                                                       const NsScalars* sc) {
+  ns_nodal_grad_body(m, P, U, prim, ngrad, sc, vert_at(m, blockIdx.x * blockDim.x + threadIdx.x));
 }
 
-// The same nodal gradient with a group of NG lanes per vertex, lane p holding the
-// vertex's p-th subface (both cells' primitives, the 15 gradient and 9 matrix terms): the
-// sums run in subface order by shuffles, each lane forming the same totals and the same
-// pseudo-inverse, and the lanes share the stores. Every lane of the warp reaches every
-// shuffle. CACHED: the pseudo-inverse comes from m.npinv and no matrix terms are formed.
-template <int NG, bool CACHED>
-__device__ void ns_nodal_grad_group(const DevMesh& m, const double* __restrict__ U, double* __restrict__ ngrad,
-                                    const NsScalars* sc, const int t, const int lane) {
+// this lane's part of the vertex's extremes, then the group's
+template <class T, int NG>
+__device__ inline void put_extremes_group(const DevMesh& m, const double* __restrict__ U, const double* __restrict__ prim,
+                                          const int v, const bool live, const int lane, double* o) {
+  Extremes<T> x;
+  if (live)
+    for (int q = m.vel_off[v] + lane; q < m.vel_off[v + 1]; q += NG) x.cell(U, prim, m.vel[q]);
+  for (int d = NG / 2; d > 0; d >>= 1)
+    x.fold(__shfl_xor_sync(0xffffffffu, x.pmin, d, NG), __shfl_xor_sync(0xffffffffu, x.pmax, d, NG),
+           __shfl_xor_sync(0xffffffffu, x.rmin, d, NG), __shfl_xor_sync(0xffffffffu, x.rmax, d, NG));
+  if (!live || lane != 5) return;
+  o[kVertPmin] = (double)x.pmin;
+  o[kVertPmax] = (double)x.pmax;
+  o[kVertRmin] = (double)x.rmin;
+  o[kVertRmax] = (double)x.rmax;
+}
+
+// The same record with a group of NG lanes per vertex, lane p holding the vertex's p-th
+// subface: the gradient's sums run in subface order by shuffles, each lane forming the
+// same totals, lane k < 5 the three components and the weight of variable k, and the lanes
+// share the cells of the extremes. Every lane of the warp reaches every shuffle.
+template <int NG>
+__device__ void ns_nodal_grad_group(const DevMesh& m, const NsParams& P, const double* __restrict__ U,
+                                    const double* __restrict__ prim, double* __restrict__ ngrad, const NsScalars* sc,
+                                    const int t, const int lane) {
   if (sc && sc->done) return;
   constexpr unsigned kAll = 0xffffffffu;
   const bool live = t < m.nv;
   const int v = vert_at(m, t);
   const int pb = live ? m.vsf_off[v] : 0, np = live ? m.vsf_off[v + 1] - pb : 0;
   const int nmax = __reduce_max_sync(kAll, np);
-  double tg[15], tm[9];
+  double tg[15];
   for (int i = 0; i < 15; ++i) tg[i] = 0.0;
-  for (int i = 0; i < 9; ++i) tm[i] = 0.0;
   int in = 0;
   if (lane < np) {
     const int sf = m.vsf[pb + lane];
     const int2 lr = m.flr[m.sf_face[sf]];
     if (lr.y >= 0) {
       in = 1;
-      double ul[5], ur[5], wl[5], wr[5];
-      ld5(U, lr.x, ul);
-      ld5(U, lr.y, ur);
-      c2p(ul, wl);
-      c2p(ur, wr);
+      const double *wl = prim + 5 * (size_t)lr.x, *wr = prim + 5 * (size_t)lr.y;
       const double4 sn = m.sfn[sf];
       const double n[3] = {sn.x, sn.y, sn.z};
       for (int d = 0; d < 3; ++d)
         for (int k = 0; k < 5; ++k) tg[5 * d + k] = sn.w * (n[d] * (wr[k] - wl[k]));
-      if (!CACHED) {
-        const double4 cl = m.cc[lr.x], cr = m.cc[lr.y];
-        const double dxc[3] = {cr.x - cl.x, cr.y - cl.y, cr.z - cl.z};
-        for (int d = 0; d < 3; ++d)
-          for (int e = 0; e < 3; ++e) tm[3 * d + e] = sn.w * (n[d] * dxc[e]);
-      }
     }
   }
   double g[3][5] = {{0, 0, 0, 0, 0}, {0, 0, 0, 0, 0}, {0, 0, 0, 0, 0}};
-  double mat[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
   for (int j = 0; j < nmax; ++j) {
     const bool add = __shfl_sync(kAll, in, j, NG) != 0;
 #pragma unroll
@@ -743,38 +826,83 @@ __device__ void ns_nodal_grad_group(const DevMesh& m, const double* __restrict__
       const double x = __shfl_sync(kAll, tg[i], j, NG);
       if (add) g[i / 5][i % 5] = g[i / 5][i % 5] + x;
     }
-    if (!CACHED)
-#pragma unroll
-      for (int i = 0; i < 9; ++i) {
-        const double x = __shfl_sync(kAll, tm[i], j, NG);
-        if (add) mat[i / 3][i % 3] = mat[i / 3][i % 3] + x;
-      }
   }
-  if (!live) return;
-  if (CACHED) {
+  double* o = ngrad + kNsVert * (size_t)v;
+  if (P.method >= 2) {
+    if (P.precision == 2) put_extremes_group<float, NG>(m, U, prim, v, live, lane, o);
+    else put_extremes_group<double, NG>(m, U, prim, v, live, lane, o);
+  }
+  if (!live || lane >= 5) return;
+  double mat[3][3];
+  if (has_nodal_pinv(m)) {
     for (int d = 0; d < 3; ++d)
       for (int e = 0; e < 3; ++e) mat[d][e] = m.npinv[9 * (size_t)v + 3 * d + e];
   } else {
+    nodal_grad_matrix(m, v, mat);
     pinv3(mat);
   }
   const bool bnd = m.is_bound[v] != 0;
-  double* o = ngrad + 15 * (size_t)v;
+  double gk[3] = {0.0, 0.0, 0.0}, r[3];
 #pragma unroll
-  for (int d = 0; d < 3; ++d)
-#pragma unroll
-    for (int k = 0; k < 5; ++k)
-      if ((5 * d + k) % NG == lane) {
-        double s = 0.0;
-        for (int e = 0; e < 3; ++e) s = s + mat[d][e] * g[e][k];
-        o[5 * d + k] = bnd ? 0.0 : s;
-      }
+  for (int k = 0; k < 5; ++k)
+    if (lane == k)
+      for (int e = 0; e < 3; ++e) gk[e] = g[e][k];
+  for (int d = 0; d < 3; ++d) {
+    double s = 0.0;
+    for (int e = 0; e < 3; ++e) s = s + mat[d][e] * gk[e];
+    r[d] = bnd ? 0.0 : s;
+    o[5 * d + lane] = r[d];
+  }
+  if (P.method >= 3) {
+    const double vol = m.vol_v[v];
+    o[kVertWeight + lane] = P.precision == 2 ? nodal_weight<float>(P.method, (float)vol, r[0], r[1], r[2])
+                                             : nodal_weight<double>(P.method, vol, r[0], r[1], r[2]);
+  }
 }
 
-template <int NG, bool CACHED>
-__global__ void __launch_bounds__(128) k_ns_nodal_grad_group(DevMesh m, const double* __restrict__ U,
+template <int NG>
+__global__ void __launch_bounds__(128) k_ns_nodal_grad_group(DevMesh m, NsParams P, const double* __restrict__ U,
+                                                             const double* __restrict__ prim,
                                                              double* __restrict__ ngrad, const NsScalars* sc) {
-  ns_nodal_grad_group<NG, CACHED>(m, U, ngrad, sc, blockIdx.x * (128 / NG) + threadIdx.x / NG,
-                                  threadIdx.x % NG);
+  ns_nodal_grad_group<NG>(m, P, U, prim, ngrad, sc, blockIdx.x * (128 / NG) + threadIdx.x / NG, threadIdx.x % NG);
+}
+
+// physical_slope_limiter's and relaxed_maximum_principle's bound on the slope factor at a
+// vertex: dw0, dw4 the density and pressure increments there
+template <class T>
+__device__ inline T slope_bound(const T* w0, T dw0, T dw4) {
+  const T tol = (T)1e-8;
+  T om = 1;
+  if (dw0 < (T)0) om = tmin2(om, tmax2((T)0, w0[0] / (tol - dw0)));
+  if (dw4 < (T)0) om = tmin2(om, tmax2((T)0, w0[4] / (tol - dw4)));
+  return om;
+}
+template <class T>
+__device__ inline T maximum_bound(const T* w0, T dw0, T dw4, const Extremes<T>& x) {  // x already relaxed
+  const T tol = (T)1e-8;
+  T om = 1;
+  if (dw0 < (T)0)
+    om = tmin2(om, tmax2((T)0, qdiv(w0[0] - x.rmin, tol - dw0)));
+  else
+    om = tmin2(om, tmax2((T)0, qdiv(-(w0[0] - x.rmax), tol + dw0)));
+  if (dw4 < (T)0)
+    om = tmin2(om, tmax2((T)0, qdiv(w0[4] - x.pmin, tol - dw4)));
+  else
+    om = tmin2(om, tmax2((T)0, qdiv(-(w0[4] - x.pmax), tol + dw4)));
+  return om;
+}
+template <class T>
+__device__ inline void relax(Extremes<T>& x) {
+  x.pmin = ((T)1.0 - (T)1e-2) * x.pmin;
+  x.rmin = ((T)1.0 - (T)1e-2) * x.rmin;
+  x.pmax = ((T)1.0 + (T)1e-2) * x.pmax;
+  x.rmax = ((T)1.0 + (T)1e-2) * x.rmax;
+}
+template <class T>
+__device__ inline T along(const T* g, const T* dx, int k) {
+  T s = 0;
+  for (int d = 0; d < 3; ++d) s = s + g[5 * d + k] * dx[d];
+  return s;
 }
 
 // compute_cell_grad_method_2..6 (:166-320) + physical_slope_limiter + relaxed_maximum_principle
@@ -789,47 +917,52 @@ __device__ void ns_cell_grad_body(const DevMesh& m, const NsParams& P, const dou
     for (int i = 0; i < 15; ++i) go[i] = 0.0;
     return;
   }
-  const T eps = (T)1e-3, tol = (T)1e-8;
+  const T eps = (T)1e-3;
   T g[15];
   T ws[5] = {0, 0, 0, 0, 0};
   for (int i = 0; i < 15; ++i) g[i] = 0;
+  Extremes<T> x;
   const int vb = m.ev_off[c], nvc = m.ev_off[c + 1] - vb;
   if (P.method == 2) {  // dual-volume average
     T dvs = 0;
     for (int j = 0; j < nvc; ++j) {
       const int v = m.ev[vb + j];
-      const double* ng = ngrad + 15 * (size_t)v;
+      const double* ng = ngrad + kNsVert * (size_t)v;
       const T vol = (T)m.vol_v[v];
       for (int i = 0; i < 15; ++i) g[i] = g[i] + vol * (T)ng[i];
       dvs = dvs + vol;
+      x.fold((T)ng[kVertPmin], (T)ng[kVertPmax], (T)ng[kVertRmin], (T)ng[kVertRmax]);
     }
     for (int i = 0; i < 15; ++i) g[i] = qdiv(g[i], dvs);
   } else if (P.method == 3) {  // the vertex gradient of smallest norm, per variable
-    const double* ng1 = ngrad + 15 * (size_t)m.ev[vb];
-    for (int i = 0; i < 15; ++i) g[i] = (T)ng1[i];
-    for (int j = 1; j < nvc; ++j) {
-      const double* ng = ngrad + 15 * (size_t)m.ev[vb + j];
-      for (int k = 0; k < 5; ++k)
-        if (oi3<T>((T)ng[k], (T)ng[5 + k], (T)ng[10 + k]) < oi3<T>(g[k], g[5 + k], g[10 + k]))
+    for (int j = 0; j < nvc; ++j) {
+      const double* ng = ngrad + kNsVert * (size_t)m.ev[vb + j];
+      for (int k = 0; k < 5; ++k) {
+        const T o = (T)ng[kVertWeight + k];
+        if (j == 0 || o < ws[k]) {
+          ws[k] = o;
           for (int d = 0; d < 3; ++d) g[5 * d + k] = (T)ng[5 * d + k];
+        }
+      }
+      x.fold((T)ng[kVertPmin], (T)ng[kVertPmax], (T)ng[kVertRmin], (T)ng[kVertRmax]);
     }
   } else {  // 4: V / (eps + |g|); 5, 6: V / (eps + |g|)^2 (6 adds the central average)
     T cg[15], cws = 0;
     for (int i = 0; i < 15; ++i) cg[i] = 0;
     for (int j = 0; j < nvc; ++j) {
       const int v = m.ev[vb + j];
-      const double* ng = ngrad + 15 * (size_t)v;
-      const T vol = (T)m.vol_v[v];
+      const double* ng = ngrad + kNsVert * (size_t)v;
       for (int k = 0; k < 5; ++k) {
-        const T q = eps + oi3<T>((T)ng[k], (T)ng[5 + k], (T)ng[10 + k]);
-        const T w = P.method == 4 ? vol / q : vol / (q * q);
+        const T w = (T)ng[kVertWeight + k];
         for (int d = 0; d < 3; ++d) g[5 * d + k] = g[5 * d + k] + w * (T)ng[5 * d + k];
         ws[k] = ws[k] + w;
       }
       if (P.method == 6) {
+        const T vol = (T)m.vol_v[v];
         for (int i = 0; i < 15; ++i) cg[i] = cg[i] + vol * (T)ng[i];
         cws = cws + vol;
       }
+      x.fold((T)ng[kVertPmin], (T)ng[kVertPmax], (T)ng[kVertRmin], (T)ng[kVertRmax]);
     }
     if (P.method == 6) {  // OI of the (3, 5) central gradient: the norm of its first column
       for (int i = 0; i < 15; ++i) cg[i] = qdiv(cg[i], cws);
@@ -851,48 +984,15 @@ __device__ void ns_cell_grad_body(const DevMesh& m, const NsParams& P, const dou
   for (int j = 0; j < nvc; ++j) {  // physical_slope_limiter
     const double4 xv = m.x[m.ev[vb + j]];
     const T dx[3] = {(T)(xv.x - ce.x), (T)(xv.y - ce.y), (T)(xv.z - ce.z)};
-    T dw0 = 0, dw4 = 0;
-    for (int d = 0; d < 3; ++d) dw0 = dw0 + g[5 * d] * dx[d];
-    for (int d = 0; d < 3; ++d) dw4 = dw4 + g[5 * d + 4] * dx[d];
-    if (dw0 < (T)0) omega = tmin2(omega, tmax2((T)0, w0[0] / (tol - dw0)));
-    if (dw4 < (T)0) omega = tmin2(omega, tmax2((T)0, w0[4] / (tol - dw4)));
+    omega = tmin2(omega, slope_bound(w0, along(g, dx, 0), along(g, dx, 4)));
   }
   for (int i = 0; i < 15; ++i) g[i] = omega * g[i];
-  T rmin = (T)1e100, rmax = 0, pmin = (T)1e100, pmax = 0;  // relaxed_maximum_principle
-  if (sizeof(T) == 4) rmin = pmin = (T)3.0e38f;
-  for (int j = 0; j < nvc; ++j) {
-    const int v = m.ev[vb + j];
-    for (int q = m.vel_off[v]; q < m.vel_off[v + 1]; ++q) {
-      double un[5];
-      ld5(U, m.vel[q], un);
-      T ut[5], w[5];
-      for (int k = 0; k < 5; ++k) ut[k] = (T)un[k];
-      c2p(ut, w);
-      pmin = tmin2(pmin, w[4]);
-      pmax = tmax2(pmax, w[4]);
-      rmin = tmin2(rmin, w[0]);
-      rmax = tmax2(rmax, w[0]);
-    }
-  }
-  pmin = ((T)1.0 - (T)1e-2) * pmin;
-  rmin = ((T)1.0 - (T)1e-2) * rmin;
-  pmax = ((T)1.0 + (T)1e-2) * pmax;
-  rmax = ((T)1.0 + (T)1e-2) * rmax;
+  relax(x);
   omega = 1;
   for (int j = 0; j < nvc; ++j) {
     const double4 xv = m.x[m.ev[vb + j]];
     const T dx[3] = {(T)(xv.x - ce.x), (T)(xv.y - ce.y), (T)(xv.z - ce.z)};
-    T dw0 = 0, dw4 = 0;
-    for (int d = 0; d < 3; ++d) dw0 = dw0 + g[5 * d] * dx[d];
-    for (int d = 0; d < 3; ++d) dw4 = dw4 + g[5 * d + 4] * dx[d];
-    if (dw0 < (T)0)
-      omega = tmin2(omega, tmax2((T)0, qdiv(w0[0] - rmin, tol - dw0)));
-    else
-      omega = tmin2(omega, tmax2((T)0, qdiv(-(w0[0] - rmax), tol + dw0)));
-    if (dw4 < (T)0)
-      omega = tmin2(omega, tmax2((T)0, qdiv(w0[4] - pmin, tol - dw4)));
-    else
-      omega = tmin2(omega, tmax2((T)0, qdiv(-(w0[4] - pmax), tol + dw4)));
+    omega = tmin2(omega, maximum_bound(w0, along(g, dx, 0), along(g, dx, 4), x));
   }
   for (int i = 0; i < 15; ++i) go[i] = (double)(omega * g[i]);
 }
@@ -906,14 +1006,11 @@ __global__ void __launch_bounds__(128) k_ns_cell_grad(DevMesh m, NsParams P, con
 
 // The same cell gradient with a group of kCellLanes lanes per cell, lane j holding the
 // cell's j-th vertex, for small meshes where a thread per cell leaves most SMs idle and
-// each cell's chain sets the kernel's length. Per-vertex terms (weights, their products,
-// the limiters' candidates, the neighbour states' primitives) are formed in parallel;
-// every sum is taken in vertex order by shuffles, each lane forming the same totals from
-// the same operands, so the sums have the thread-per-cell kernel's bits. The min / max
-// folds (tmin2, tmax2) run over each lane's own list from the initial value, then over
-// the lanes' results in vertex order: a fold keeps the first occurrence of its extreme
-// among the values strictly past the initial one and never takes a NaN, so the two-level
-// fold returns the single fold's bits. Every lane of the warp reaches every shuffle.
+// each cell's chain sets the kernel's length. Per-vertex terms (the weighted gradients, the
+// limiters' candidates) are formed in parallel; every sum is taken in vertex order by
+// shuffles, each lane forming the same totals from the same operands, so the sums have the
+// thread-per-cell kernel's bits; the folds have theirs (Extremes). Every lane of the warp
+// reaches every shuffle.
 template <class T>
 __device__ void ns_cell_grad_group(const DevMesh& m, const NsParams& P, const double* __restrict__ U,
                                    const double* __restrict__ ngrad, double* __restrict__ grad,
@@ -926,46 +1023,20 @@ __device__ void ns_cell_grad_group(const DevMesh& m, const NsParams& P, const do
     return;
   }
   constexpr unsigned kAll = 0xffffffffu;
-  const T eps = (T)1e-3, tol = (T)1e-8;
+  const T eps = (T)1e-3;
   const int vb = live ? m.ev_off[c] : 0, nvc = live ? m.ev_off[c + 1] - vb : 0;
   const int nmax = __reduce_max_sync(kAll, nvc);
   const bool own = lane < nvc;
   const int v = own ? m.ev[vb + lane] : 0;
-  T ng[15], vol = 0;
+  T ng[15], w[5] = {0, 0, 0, 0, 0}, vol = 0;
   for (int i = 0; i < 15; ++i) ng[i] = 0;
+  Extremes<T> x;
   if (own) {
-    const double* src = ngrad + 15 * (size_t)v;
+    const double* src = ngrad + kNsVert * (size_t)v;
     for (int i = 0; i < 15; ++i) ng[i] = (T)src[i];
+    for (int k = 0; k < 5; ++k) w[k] = (T)src[kVertWeight + k];
+    x.fold((T)src[kVertPmin], (T)src[kVertPmax], (T)src[kVertRmin], (T)src[kVertRmax]);
     vol = (T)m.vol_v[v];
-  }
-  // relaxed_maximum_principle, this lane's part: the states of the cells around its
-  // vertex do not depend on the gradient, so their folds run first, their loads issued
-  // four cells at a time (the folds in the list's order)
-  T lrmin = (T)1e100, lrmax = 0, lpmin = (T)1e100, lpmax = 0;
-  if (sizeof(T) == 4) lrmin = lpmin = (T)3.0e38f;
-  if (own) {
-    constexpr int kAhead = 4;
-    const int qb = m.vel_off[v + 1];
-    for (int q0 = m.vel_off[v]; q0 < qb; q0 += kAhead) {
-      int id[kAhead];
-#pragma unroll
-      for (int i = 0; i < kAhead; ++i) id[i] = q0 + i < qb ? m.vel[q0 + i] : 0;
-      double un[kAhead][5];
-#pragma unroll
-      for (int i = 0; i < kAhead; ++i)
-        if (q0 + i < qb) ld5(U, id[i], un[i]);
-#pragma unroll
-      for (int i = 0; i < kAhead; ++i)
-        if (q0 + i < qb) {
-          T ut[5], w[5];
-          for (int k = 0; k < 5; ++k) ut[k] = (T)un[i][k];
-          c2p(ut, w);
-          lpmin = tmin2(lpmin, w[4]);
-          lpmax = tmax2(lpmax, w[4]);
-          lrmin = tmin2(lrmin, w[0]);
-          lrmax = tmax2(lrmax, w[0]);
-        }
-    }
   }
   // the cell's primitive state and this lane's vertex offset, for both limiters
   T w0[5] = {0, 0, 0, 0, 0}, dx[3] = {0, 0, 0};
@@ -990,43 +1061,39 @@ __device__ void ns_cell_grad_group(const DevMesh& m, const NsParams& P, const do
     for (int j = 0; j < nmax; ++j) {
       const bool in = j < nvc;
       for (int i = 0; i < 15; ++i) {
-        const T x = __shfl_sync(kAll, t[i], j, kCellLanes);
-        if (in) g[i] = g[i] + x;
+        const T y = __shfl_sync(kAll, t[i], j, kCellLanes);
+        if (in) g[i] = g[i] + y;
       }
-      const T x = __shfl_sync(kAll, vol, j, kCellLanes);
-      if (in) dvs = dvs + x;
+      const T y = __shfl_sync(kAll, vol, j, kCellLanes);
+      if (in) dvs = dvs + y;
     }
     for (int i = 0; i < 15; ++i) g[i] = qdiv(g[i], dvs);
   } else if (P.method == 3) {  // the vertex gradient of smallest norm, per variable
     for (int k = 0; k < 5; ++k) {
-      const T o = oi3<T>(ng[k], ng[5 + k], ng[10 + k]);
-      T best = __shfl_sync(kAll, o, 0, kCellLanes);
+      T best = __shfl_sync(kAll, w[k], 0, kCellLanes);
       int sel = 0;
       for (int j = 1; j < nmax; ++j) {
-        const T x = __shfl_sync(kAll, o, j, kCellLanes);
-        if (j < nvc && x < best) {
-          best = x;
+        const T y = __shfl_sync(kAll, w[k], j, kCellLanes);
+        if (j < nvc && y < best) {
+          best = y;
           sel = j;
         }
       }
       for (int d = 0; d < 3; ++d) g[5 * d + k] = __shfl_sync(kAll, ng[5 * d + k], sel, kCellLanes);
     }
   } else {  // 4: V / (eps + |g|); 5, 6: V / (eps + |g|)^2 (6 adds the central average)
-    T w[5], t[15];
-    for (int k = 0; k < 5; ++k) {
-      const T q = eps + oi3<T>(ng[k], ng[5 + k], ng[10 + k]);
-      w[k] = P.method == 4 ? vol / q : vol / (q * q);
+    T t[15];
+    for (int k = 0; k < 5; ++k)
       for (int d = 0; d < 3; ++d) t[5 * d + k] = w[k] * ng[5 * d + k];
-    }
     for (int j = 0; j < nmax; ++j) {
       const bool in = j < nvc;
       for (int i = 0; i < 15; ++i) {
-        const T x = __shfl_sync(kAll, t[i], j, kCellLanes);
-        if (in) g[i] = g[i] + x;
+        const T y = __shfl_sync(kAll, t[i], j, kCellLanes);
+        if (in) g[i] = g[i] + y;
       }
       for (int k = 0; k < 5; ++k) {
-        const T x = __shfl_sync(kAll, w[k], j, kCellLanes);
-        if (in) ws[k] = ws[k] + x;
+        const T y = __shfl_sync(kAll, w[k], j, kCellLanes);
+        if (in) ws[k] = ws[k] + y;
       }
     }
     if (P.method == 6) {  // OI of the (3, 5) central gradient: the norm of its first column
@@ -1038,11 +1105,11 @@ __device__ void ns_cell_grad_group(const DevMesh& m, const NsParams& P, const do
       for (int j = 0; j < nmax; ++j) {
         const bool in = j < nvc;
         for (int i = 0; i < 15; ++i) {
-          const T x = __shfl_sync(kAll, t[i], j, kCellLanes);
-          if (in) cg[i] = cg[i] + x;
+          const T y = __shfl_sync(kAll, t[i], j, kCellLanes);
+          if (in) cg[i] = cg[i] + y;
         }
-        const T x = __shfl_sync(kAll, vol, j, kCellLanes);
-        if (in) cws = cws + x;
+        const T y = __shfl_sync(kAll, vol, j, kCellLanes);
+        if (in) cws = cws + y;
       }
       for (int i = 0; i < 15; ++i) cg[i] = qdiv(cg[i], cws);
       const T q = eps + oi3<T>(cg[0], cg[5], cg[10]);
@@ -1053,55 +1120,18 @@ __device__ void ns_cell_grad_group(const DevMesh& m, const NsParams& P, const do
     for (int k = 0; k < 5; ++k)
       for (int d = 0; d < 3; ++d) g[5 * d + k] = qdiv(g[5 * d + k], ws[k]);
   }
-  T om = 1;  // physical_slope_limiter: this lane's vertex
-  {
-    T dw0 = 0, dw4 = 0;
-    for (int d = 0; d < 3; ++d) dw0 = dw0 + g[5 * d] * dx[d];
-    for (int d = 0; d < 3; ++d) dw4 = dw4 + g[5 * d + 4] * dx[d];
-    if (dw0 < (T)0) om = tmin2(om, tmax2((T)0, w0[0] / (tol - dw0)));
-    if (dw4 < (T)0) om = tmin2(om, tmax2((T)0, w0[4] / (tol - dw4)));
-  }
-  T omega = 1;
-  for (int j = 0; j < nmax; ++j) {
-    const T x = __shfl_sync(kAll, om, j, kCellLanes);
-    if (j < nvc) omega = tmin2(omega, x);
-  }
+  // the least of the group's bounds; a lane without a vertex holds 1
+  auto least = [&](T om) {
+    for (int d = kCellLanes / 2; d > 0; d >>= 1) om = tmin2(om, __shfl_xor_sync(kAll, om, d, kCellLanes));
+    return om;
+  };
+  T omega = least(own ? slope_bound(w0, along(g, dx, 0), along(g, dx, 4)) : (T)1);
   for (int i = 0; i < 15; ++i) g[i] = omega * g[i];
-  T rmin = (T)1e100, rmax = 0, pmin = (T)1e100, pmax = 0;  // relaxed_maximum_principle
-  if (sizeof(T) == 4) rmin = pmin = (T)3.0e38f;
-  for (int j = 0; j < nmax; ++j) {
-    const T a = __shfl_sync(kAll, lpmin, j, kCellLanes), b = __shfl_sync(kAll, lpmax, j, kCellLanes);
-    const T e = __shfl_sync(kAll, lrmin, j, kCellLanes), f = __shfl_sync(kAll, lrmax, j, kCellLanes);
-    if (j < nvc) {
-      pmin = tmin2(pmin, a);
-      pmax = tmax2(pmax, b);
-      rmin = tmin2(rmin, e);
-      rmax = tmax2(rmax, f);
-    }
-  }
-  pmin = ((T)1.0 - (T)1e-2) * pmin;
-  rmin = ((T)1.0 - (T)1e-2) * rmin;
-  pmax = ((T)1.0 + (T)1e-2) * pmax;
-  rmax = ((T)1.0 + (T)1e-2) * rmax;
-  om = 1;
-  {
-    T dw0 = 0, dw4 = 0;
-    for (int d = 0; d < 3; ++d) dw0 = dw0 + g[5 * d] * dx[d];
-    for (int d = 0; d < 3; ++d) dw4 = dw4 + g[5 * d + 4] * dx[d];
-    if (dw0 < (T)0)
-      om = tmin2(om, tmax2((T)0, qdiv(w0[0] - rmin, tol - dw0)));
-    else
-      om = tmin2(om, tmax2((T)0, qdiv(-(w0[0] - rmax), tol + dw0)));
-    if (dw4 < (T)0)
-      om = tmin2(om, tmax2((T)0, qdiv(w0[4] - pmin, tol - dw4)));
-    else
-      om = tmin2(om, tmax2((T)0, qdiv(-(w0[4] - pmax), tol + dw4)));
-  }
-  omega = 1;
-  for (int j = 0; j < nmax; ++j) {
-    const T x = __shfl_sync(kAll, om, j, kCellLanes);
-    if (j < nvc) omega = tmin2(omega, x);
-  }
+  for (int d = kCellLanes / 2; d > 0; d >>= 1)
+    x.fold(__shfl_xor_sync(kAll, x.pmin, d, kCellLanes), __shfl_xor_sync(kAll, x.pmax, d, kCellLanes),
+           __shfl_xor_sync(kAll, x.rmin, d, kCellLanes), __shfl_xor_sync(kAll, x.rmax, d, kCellLanes));
+  relax(x);
+  omega = least(own ? maximum_bound(w0, along(g, dx, 0), along(g, dx, 4), x) : (T)1);
   if (live)
 #pragma unroll
     for (int i = 0; i < 15; ++i)
@@ -1389,22 +1419,24 @@ __global__ void __launch_bounds__(kNodeGroupThreads, kNodeGroupMinBlocks) kb_ns_
   }
 }
 __global__ void __launch_bounds__(128) kb_ns_gather(const NsItem* __restrict__ it, const int* __restrict__ wc,
-                                                    const int* __restrict__ hdr, int second) {
+                                                    const int* __restrict__ hdr, int which, int second, int so) {
   const int n = hdr[0];
   for (int w = blockIdx.x; w < wc[n]; w += gridDim.x) {
     const int p = item_of(wc, n, w);
     const NsItem& I = it[p];
-    ns_gather_body(I.m, I.fs, second ? I.rhs2 : I.rhs1, I.sc, second ? 0 : 1, (w - wc[p]) * 128 + threadIdx.x);
+    ns_gather_body(I.m, I.fs, second ? I.rhs2 : I.rhs1, I.sc, second ? 0 : 1, (w - wc[p]) * 128 + threadIdx.x,
+                   which ? I.U1 : I.U0, so && !second ? I.delta : nullptr);
     __syncthreads();  // the block-reduction scratch is reused by the next work block
   }
 }
 __global__ void __launch_bounds__(256) kb_ns_nodal_grad(const NsItem* __restrict__ it, const int* __restrict__ wv,
-                                                        const int* __restrict__ hdr, int which) {
+                                                        const int* __restrict__ hdr, NsParams P, int which) {
   const int n = hdr[0];
   for (int w = blockIdx.x; w < wv[n]; w += gridDim.x) {
     const int p = item_of(wv, n, w);
     const NsItem& I = it[p];
-    ns_nodal_grad_body<false>(I.m, which ? I.U1 : I.U0, I.ngrad, I.sc, vert_at(I.m, (w - wv[p]) * blockDim.x + threadIdx.x));
+    ns_nodal_grad_body(I.m, P, which ? I.U1 : I.U0, I.delta, I.ngrad, I.sc,
+                       vert_at(I.m, (w - wv[p]) * blockDim.x + threadIdx.x));
   }
 }
 template <class T>
@@ -1786,13 +1818,13 @@ void launch_ns_batch_step(const NsTable& t, const NsParams& P, cudaStream_t s) {
   auto node = [&](int which, int so) { launch_kb_node(t, P, s, which, so); };
   auto rhs = [&](int which) {
     node(which, 0);
-    kb_ns_gather<<<gc, 128, 0, s>>>(t.items, t.wc, t.hdr, 0);
+    kb_ns_gather<<<gc, 128, 0, s>>>(t.items, t.wc, t.hdr, which, 0, P.second_order);
     if (P.second_order) {
-      kb_ns_nodal_grad<<<gv, nb, 0, s>>>(t.items, t.wv, t.hdr, which);
+      kb_ns_nodal_grad<<<gv, nb, 0, s>>>(t.items, t.wv, t.hdr, P, which);
       if (P.precision == 2) kb_ns_cell_grad<float><<<gc, 128, 0, s>>>(t.items, t.wc, t.hdr, P, which);
       else kb_ns_cell_grad<double><<<gc, 128, 0, s>>>(t.items, t.wc, t.hdr, P, which);
       node(which, 1);
-      kb_ns_gather<<<gc, 128, 0, s>>>(t.items, t.wc, t.hdr, 1);
+      kb_ns_gather<<<gc, 128, 0, s>>>(t.items, t.wc, t.hdr, which, 1, P.second_order);
     }
   };
   auto stage = [&](int st, double a1, double a2, int last) {
@@ -1887,24 +1919,19 @@ void launch_node(const DevMesh& m, const NsParams& P, const double* U, const dou
   else launch_node_tl<double, double>(m, P, U, grad, fs, so, sc);
 }
 
-// The nodal gradient: a group of 8, 16 or 32 lanes per vertex (the fewest that hold
-// every vertex's subfaces) along with the grouped node kernel, else a thread per vertex.
-template <bool CACHED>
-void launch_nodal_grad_t(const DevMesh& m, const NsParams& P, const double* U, double* ngrad, const NsScalars* sc) {
+// The vertex records: a group of 8, 16 or 32 lanes per vertex (the fewest that hold every
+// vertex's subfaces) along with the grouped node kernel, else a thread per vertex.
+void launch_nodal_grad(const DevMesh& m, const NsParams& P, const double* U, const double* prim, double* ngrad,
+                       const NsScalars* sc) {
   const int k = m.max_vsf, ng = k <= 8 ? 8 : k <= 16 ? 16 : k <= 32 ? 32 : 0;
   if (P.node_group && ng) {
     const int g = grid_for(m.nv, 128 / ng);
-    if (ng == 8) k_ns_nodal_grad_group<8, CACHED><<<g, 128, 0, m.stream>>>(m, U, ngrad, sc);
-    else if (ng == 16) k_ns_nodal_grad_group<16, CACHED><<<g, 128, 0, m.stream>>>(m, U, ngrad, sc);
-    else k_ns_nodal_grad_group<32, CACHED><<<g, 128, 0, m.stream>>>(m, U, ngrad, sc);
+    if (ng == 8) k_ns_nodal_grad_group<8><<<g, 128, 0, m.stream>>>(m, P, U, prim, ngrad, sc);
+    else if (ng == 16) k_ns_nodal_grad_group<16><<<g, 128, 0, m.stream>>>(m, P, U, prim, ngrad, sc);
+    else k_ns_nodal_grad_group<32><<<g, 128, 0, m.stream>>>(m, P, U, prim, ngrad, sc);
     return;
   }
-  k_ns_nodal_grad<CACHED><<<grid_for(m.nv, 128), 128, 0, m.stream>>>(m, U, ngrad, sc);
-}
-// with the mesh's cached pseudo-inverses when they belong to its current geometry
-void launch_nodal_grad(const DevMesh& m, const NsParams& P, const double* U, double* ngrad, const NsScalars* sc) {
-  if (m.npinv && m.npinv_epoch == m.geom_epoch) launch_nodal_grad_t<true>(m, P, U, ngrad, sc);
-  else launch_nodal_grad_t<false>(m, P, U, ngrad, sc);
+  k_ns_nodal_grad<<<grid_for(m.nv, 128), 128, 0, m.stream>>>(m, P, U, prim, ngrad, sc);
 }
 
 int ensure_nodal_pinv(DevMesh* m) {
@@ -1941,15 +1968,15 @@ void launch_cell_grad(const DevMesh& m, const NsParams& P, const double* U, cons
 }
 
 void launch_ns_rhs(const DevMesh& m, const NsParams& P, const double* U, double* fs, double* rhs1, double* rhs2,
-                   double* ngrad, double* grad, NsScalars* sc) {
+                   double* ngrad, double* grad, NsScalars* sc, double* prim) {
   const int gc = grid_for(m.ne, 128);
   launch_node(m, P, U, grad, fs, 0, sc);
-  k_ns_gather<<<gc, 128, 0, m.stream>>>(m, fs, rhs1, sc, sc ? 1 : 0);
+  k_ns_gather<<<gc, 128, 0, m.stream>>>(m, fs, rhs1, sc, sc ? 1 : 0, U, P.second_order ? prim : nullptr);
   if (P.second_order) {
-    launch_nodal_grad(m, P, U, ngrad, sc);
+    launch_nodal_grad(m, P, U, prim, ngrad, sc);
     launch_cell_grad(m, P, U, ngrad, grad, sc);
     launch_node(m, P, U, grad, fs, 1, sc);
-    k_ns_gather<<<gc, 128, 0, m.stream>>>(m, fs, rhs2, sc, 0);
+    k_ns_gather<<<gc, 128, 0, m.stream>>>(m, fs, rhs2, sc, 0, nullptr, nullptr);
   }
 }
 
@@ -1978,13 +2005,14 @@ void launch_ns_timedisc(const DevMesh& m, const NsParams& P, const double* U_rhs
 void launch_ns_euler_flux(const DevMesh& m, const NsParams& P, const double* U, const double* grad, double* fs,
                           double* rhs, int second_order, NsScalars* sc) {
   launch_node(m, P, U, grad, fs, second_order ? 1 : 0, sc);
-  k_ns_gather<<<grid_for(m.ne, 128), 128, 0, m.stream>>>(m, fs, rhs, sc, 0);
+  k_ns_gather<<<grid_for(m.ne, 128), 128, 0, m.stream>>>(m, fs, rhs, sc, 0, nullptr, nullptr);
 }
 
 // compute_cell_grad_from_nodal_grad (ns_euler_recon_module.F90:8-59)
 void launch_ns_cell_grads(const DevMesh& m, const NsParams& P, const double* U, double* ngrad, double* grad,
-                          NsScalars* sc) {
-  launch_nodal_grad(m, P, U, ngrad, sc);
+                          NsScalars* sc, double* prim) {
+  k_ns_prim<<<grid_for(m.ne, 128), 128, 0, m.stream>>>(m, U, prim);
+  launch_nodal_grad(m, P, U, prim, ngrad, sc);
   launch_cell_grad(m, P, U, ngrad, grad, sc);
 }
 

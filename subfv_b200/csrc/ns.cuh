@@ -8,6 +8,7 @@ namespace subfv {
 
 constexpr int kNsMaxSf = 32;  // subfaces around a vertex (a 3-D hex vertex has 12)
 constexpr int kNsFs = 6;      // per-subcell record: five corner flux sums and the wave-speed sum
+constexpr int kNsVert = 24;    // per-vertex record of the second-order reconstruction (ns.cu)
 constexpr int kCellLanes = 8;  // lanes per cell of the grouped cell gradient (cells of up to 8 vertices)
 
 struct NsParams {
@@ -89,9 +90,10 @@ void launch_ns_batch_step(const NsTable& t, const NsParams& P, cudaStream_t s);
 NsParams ns_params_from(const subfv_ns_cfg& c);
 
 // One residual evaluation at state U (records of kRec doubles): rhs1/sl (first order),
-// and for second order ngrad, grad, rhs2. rhs records: kRhs doubles (5 + sum_lambda).
+// and for second order ngrad (kNsVert doubles a vertex), grad, rhs2, with prim (5 doubles a
+// cell, free until the time discretisation: its delta) as scratch. rhs records: kRhs doubles (5 + sum_lambda).
 void launch_ns_rhs(const DevMesh& m, const NsParams& P, const double* U, double* fs, double* rhs1, double* rhs2,
-                   double* ngrad, double* grad, NsScalars* sc);
+                   double* ngrad, double* grad, NsScalars* sc, double* prim);
 // flux limiting + add_timedisc_and_solve + update (stage coefficients a1, a2)
 // (dterm: the diffusion corner records when P.diff, else null)
 void launch_ns_timedisc(const DevMesh& m, const NsParams& P, const double* U_rhs, const double* rhs1,
@@ -118,7 +120,7 @@ int ns_partial_blocks(const DevMesh& m);
 void launch_ns_euler_flux(const DevMesh& m, const NsParams& P, const double* U, const double* grad, double* fs,
                           double* rhs, int second_order, NsScalars* sc);
 void launch_ns_cell_grads(const DevMesh& m, const NsParams& P, const double* U, double* ngrad, double* grad,
-                          NsScalars* sc);
+                          NsScalars* sc, double* prim);
 void launch_proc_dtmin(const DevMesh& m, const double* sl, double* slot);
 void launch_proc_flux_limiting(const DevMesh& m, const double* sol5, double* rhs5, const double* rhso2_5,
                                const double* sl, double dt);

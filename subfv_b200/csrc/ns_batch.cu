@@ -31,6 +31,7 @@ struct Slot {
   double *U0 = nullptr, *U1 = nullptr, *fs = nullptr, *rhs1 = nullptr, *rhs2 = nullptr;
   double *ngrad = nullptr, *grad = nullptr, *delta = nullptr, *partial = nullptr;
   int64_t bytes = 0;       // state + mesh bytes charged against the budget
+  unsigned long long seen_epoch = 0;  // the mesh geometry the table's copy of the mesh belongs to
   unsigned long long first_snap = 0;  // the first snapshot that includes this problem
   double t0 = 0.0;
 };
@@ -48,7 +49,8 @@ struct Snapshot {
 int64_t state_bytes(const DevMesh& d, int second_order) {
   const int64_t ne = d.ne, nv = d.nv, nse = d.nse;
   const int64_t o1 = kRec * ne + kNsFs * nse + kRhs * ne + 5 * ne + 6 * (int64_t)ns_partial_blocks(d);
-  const int64_t o2 = kRec * ne + kRhs * ne + 15 * nv + 15 * ne;
+  // the mesh's pseudo-inverses are the mesh's once they exist
+  const int64_t o2 = kRec * ne + kRhs * ne + kNsVert * nv + 15 * ne + (d.npinv || d.moving ? 0 : 9 * nv);
   return 8 * (o1 + (second_order ? o2 : 0)) + node_codes_bytes(d);
 }
 
@@ -121,6 +123,18 @@ int graph_for(subfv_ns_batch* b, int steps) {
 
 // Rewrite the device table from the live slots (stream-ordered on the batch stream).
 int table_upload(subfv_ns_batch* b) {
+  for (int i : b->order) {  // a mesh whose vertices moved since the table was written
+    Slot& q = b->slots[i];
+    DevMesh& d = q.mesh->d;
+    if (q.seen_epoch == d.geom_epoch) continue;
+    if (b->P.second_order) {
+      if (ensure_nodal_pinv(&d)) return -1;
+      SUBFV_CUDA(cudaEventRecord(q.free_ev, d.stream));
+      SUBFV_CUDA(cudaStreamWaitEvent(b->stream, q.free_ev, 0));
+    }
+    q.seen_epoch = d.geom_epoch;
+    b->dirty = true;
+  }
   if (!b->dirty) return 0;
   const int k = b->stage_cur;
   SUBFV_CUDA(cudaEventSynchronize(b->stage_ev[k]));  // the staging copy issued two updates ago
@@ -321,7 +335,9 @@ int subfv_ns_batch_add(subfv_ns_batch* b, subfv_mesh* m, int take_mesh, const do
     set_error("subfv_ns_batch_add: null argument");
     return -2;
   }
-  if (handle_ensure_full_geometry(m->d) || ensure_node_codes(&m->d)) return -1;
+  if (handle_ensure_full_geometry(m->d) || ensure_node_codes(&m->d) ||
+      (b->P.second_order && ensure_nodal_pinv(&m->d)))
+    return -1;
   const DevMesh& d = m->d;
   if (ns_node_lanes(d) == 0) {
     set_error("subfv_ns_batch_add: a vertex has more than 32 subfaces or subcells");
@@ -346,7 +362,7 @@ int subfv_ns_batch_add(subfv_ns_batch* b, subfv_mesh* m, int take_mesh, const do
       dalloc_async(&q.rhs1, kRhs * ne, s) || dalloc_async(&q.delta, 5 * ne, s) ||
       dalloc_async(&q.partial, 6 * (size_t)ns_partial_blocks(d), s) ||
       (o2 && (dalloc_async(&q.U1, kRec * ne, s) || dalloc_async(&q.rhs2, kRhs * ne, s) ||
-              dalloc_async(&q.ngrad, 15 * nv, s) || dalloc_async(&q.grad, 15 * ne, s))) ||
+              dalloc_async(&q.ngrad, kNsVert * nv, s) || dalloc_async(&q.grad, 15 * ne, s))) ||
       pool_alloc((void**)&stage, 5 * ne * sizeof(double), s)) {
     slot_free_state(q, s);
     return -1;
@@ -376,6 +392,7 @@ int subfv_ns_batch_add(subfv_ns_batch* b, subfv_mesh* m, int take_mesh, const do
   q.bytes = need;
   q.first_snap = b->snap_count + 1;
   q.t0 = t0;
+  q.seen_epoch = d.geom_epoch;
   b->used += need;
   b->order.push_back(k);
   b->dirty = true;

@@ -101,7 +101,7 @@ void enqueue_ns_step(subfv_ns_state* s) {
   const DevMesh& d = s->m->d;
   const NsParams& P = s->P;
   auto rhs = [&](const double* U) {
-    launch_ns_rhs(d, P, U, s->fs, s->rhs1, s->rhs2, s->ngrad, s->grad, s->sc);
+    launch_ns_rhs(d, P, U, s->fs, s->rhs1, s->rhs2, s->ngrad, s->grad, s->sc, s->delta);
     if (P.diff) launch_ns_diffusion(d, s->D, U, s->dterm, s->mu0c);
   };
   if (P.second_order) {
@@ -235,7 +235,7 @@ int subfv_ns_state_create(subfv_mesh* m, const subfv_ns_cfg* cfg, const double* 
   mem.add(&s->fs, kNsFs * nse);
   mem.add(&s->rhs1, kRhs * ne);
   mem.add(&s->rhs2, kRhs * ne);
-  mem.add(&s->ngrad, 15 * nv);
+  mem.add(&s->ngrad, kNsVert * nv);
   mem.add(&s->grad, 15 * ne);
   mem.add(&s->delta, 5 * ne);
   mem.add(&s->partial, 6 * (size_t)ns_partial_blocks(d));
@@ -540,7 +540,7 @@ int implicit_assemble(subfv_ns_state* s, double cfl_implicit, double dt_force, d
   h.omega = 1.0;
   h.done = 0;
   SUBFV_CUDA(cudaMemcpyAsync(s->sc, &h, sizeof(h), cudaMemcpyHostToDevice, d.stream));
-  launch_ns_rhs(d, Q, s->U0, s->fs, s->rhs1, s->rhs2, s->ngrad, s->grad, s->sc);
+  launch_ns_rhs(d, Q, s->U0, s->fs, s->rhs1, s->rhs2, s->ngrad, s->grad, s->sc, s->delta);
   double dtred = 0.0;
   SUBFV_CUDA(cudaMemcpyAsync(&dtred, &s->sc->dtred, sizeof(double), cudaMemcpyDeviceToHost, d.stream));
   SUBFV_CUDA(cudaStreamSynchronize(d.stream));
@@ -670,7 +670,7 @@ int subfv_compute_rhs_ns_ex(subfv_mesh* m, const subfv_ns_cfg* cfg, const double
       st = -1;
       break;
     }
-    launch_ns_rhs(d, s->P, s->U0, s->fs, s->rhs1, s->rhs2, s->ngrad, s->grad, s->sc);
+    launch_ns_rhs(d, s->P, s->U0, s->fs, s->rhs1, s->rhs2, s->ngrad, s->grad, s->sc, s->delta);
     if (s->P.second_order) launch_ns_flux_limiting(d, s->P, s->U0, s->rhs1, s->rhs2, s->sc);
     double* ddiag = nullptr;
     if (s->P.diff) {
@@ -752,10 +752,10 @@ void grad_from_ref(const double* f, double* g, size_t n) {
     for (int dd = 0; dd < 3; ++dd)
       for (int k = 0; k < 5; ++k) g[15 * c + 5 * dd + k] = f[15 * c + dd + 3 * k];
 }
-void grad_to_ref(const double* g, double* f, size_t n) {
+void grad_to_ref(const double* g, double* f, size_t n, size_t stride = 15) {
   for (size_t c = 0; c < n; ++c)
     for (int dd = 0; dd < 3; ++dd)
-      for (int k = 0; k < 5; ++k) f[15 * c + dd + 3 * k] = g[15 * c + 5 * dd + k];
+      for (int k = 0; k < 5; ++k) f[15 * c + dd + 3 * k] = g[stride * c + 5 * dd + k];
 }
 
 // device scratch of one call, released on the mesh's stream
@@ -826,15 +826,15 @@ int subfv_compute_cell_grad_from_nodal_grad(subfv_mesh* m, const subfv_ns_cfg* c
   if (rc) return rc;
   DevMesh& d = m->d;
   if (reset_scalars(h.s)) return -1;
-  launch_ns_cell_grads(d, h.s->P, h.s->U0, h.s->ngrad, h.s->grad, h.s->sc);
-  std::vector<double> g(15 * (size_t)d.ne), ng(nodal_grad ? 15 * (size_t)d.nv : 0);
+  launch_ns_cell_grads(d, h.s->P, h.s->U0, h.s->ngrad, h.s->grad, h.s->sc, h.s->delta);
+  std::vector<double> g(15 * (size_t)d.ne), ng(nodal_grad ? kNsVert * (size_t)d.nv : 0);
   SUBFV_CUDA(cudaMemcpyAsync(g.data(), h.s->grad, g.size() * sizeof(double), cudaMemcpyDeviceToHost, d.stream));
   if (nodal_grad)
     SUBFV_CUDA(cudaMemcpyAsync(ng.data(), h.s->ngrad, ng.size() * sizeof(double), cudaMemcpyDeviceToHost, d.stream));
   const int st = handle_check_status(d);
   SUBFV_CUDA(cudaGetLastError());
   grad_to_ref(g.data(), grad, d.ne);
-  if (nodal_grad) grad_to_ref(ng.data(), nodal_grad, d.nv);
+  if (nodal_grad) grad_to_ref(ng.data(), nodal_grad, d.nv, kNsVert);
   return st;
 }
 
