@@ -88,12 +88,16 @@ int ensure_scratch(subfv_mesh* m) {
 int ensure_lag_arrays(DevMesh& d) {
   if (d.frec) return 0;
   SUBFV_CUDA(cudaMallocAsync((void**)&d.frec, 6 * (size_t)d.nf * sizeof(double), d.stream));
-  SUBFV_CUDA(cudaMallocAsync((void**)&d.centry, std::max<size_t>(d.ncsf, 1) * sizeof(int4), d.stream));
+  const size_t tiles = (d.ne + 31) / 32, entries = std::max<size_t>(32 * tiles * d.max_csf, 1),
+               pairs = std::max<size_t>(32 * tiles * d.max_pairs, 1);
+  SUBFV_CUDA(cudaMallocAsync((void**)&d.centry, entries * sizeof(int4), d.stream));
+  SUBFV_CUDA(cudaMemsetAsync(d.centry, 0xff, entries * sizeof(int4), d.stream));
   SUBFV_CUDA(cudaMallocAsync((void**)&d.fS, (size_t)d.nf * sizeof(double4), d.stream));
-  SUBFV_CUDA(cudaMallocAsync((void**)&d.gface, 8 * (size_t)d.ne * sizeof(uint16_t), d.stream));
+  SUBFV_CUDA(cudaMallocAsync((void**)&d.cinfo, (size_t)d.ne * sizeof(uint32_t), d.stream));
+  SUBFV_CUDA(cudaMallocAsync((void**)&d.gpair, pairs * sizeof(uint32_t), d.stream));
   SUBFV_CUDA(cudaMallocAsync((void**)&d.gsub, (size_t)d.nse * sizeof(uint32_t), d.stream));
-  d.bytes += 6 * (size_t)d.nf * sizeof(double) + std::max<size_t>(d.ncsf, 1) * sizeof(int4) +
-             (size_t)d.nf * sizeof(double4) + 8 * (size_t)d.ne * sizeof(uint16_t) + (size_t)d.nse * sizeof(uint32_t);
+  d.bytes += 6 * (size_t)d.nf * sizeof(double) + entries * sizeof(int4) + (size_t)d.nf * sizeof(double4) +
+             (pairs + (size_t)d.ne + (size_t)d.nse) * sizeof(uint32_t);
   launch_build_cell_entries(d);
   launch_build_geom_codes(d);
   SUBFV_CUDA(cudaGetLastError());
@@ -334,7 +338,7 @@ int subfv_compute_rhs_lagrange(subfv_mesh* m, const double* sol, double* vp, dou
   d.b2d = b2d;
   if (load_sol(m, sol, mass)) return -1;
   launch_lag_node(d, m->sol6, nullptr, 0);
-  launch_lag_cell(d, m->sol6, m->rhs6, nullptr, nullptr, 0, 1);
+  launch_lag_cell(d, m->sol6, m->rhs6, nullptr, nullptr, 1);
   launch_unpack6(d, d.ne, kRhs, m->rhs6, m->stage);
   SUBFV_CUDA(cudaMemcpyAsync(rhs, m->stage, 5 * (size_t)d.ne * sizeof(double), cudaMemcpyDeviceToHost, d.stream));
   std::vector<double4> h(d.nv);
@@ -360,7 +364,7 @@ int subfv_compute_rhs_lagrange_sidil(subfv_mesh* m, const double* sol, double* v
   d.b2d = b2d;
   if (load_sol(m, sol, mass)) return -1;
   launch_lag_sidil_node(d, m->sol6, nullptr, method_length);
-  launch_lag_cell(d, m->sol6, m->rhs6, nullptr, nullptr, 0, 5);
+  launch_lag_cell(d, m->sol6, m->rhs6, nullptr, nullptr, 5);
   launch_unpack6(d, d.ne, kRhs, m->rhs6, m->stage);
   SUBFV_CUDA(cudaMemcpyAsync(rhs, m->stage, 5 * (size_t)d.ne * sizeof(double), cudaMemcpyDeviceToHost, d.stream));
   std::vector<double4> h(d.nv);
@@ -401,7 +405,7 @@ int subfv_compute_dt(subfv_mesh* m, const double* sol, double cfl, const double*
   launch_vp_in(d, m->stage);
   double* slot = &m->sc->dtmin;
   launch_set_scalar(d, slot, 1e6);
-  launch_lag_cell(d, m->sol6, nullptr, nullptr, slot, 0, 2);
+  launch_lag_cell(d, m->sol6, nullptr, nullptr, slot, 2);
   double h = 0;
   SUBFV_CUDA(cudaMemcpyAsync(&h, slot, sizeof(double), cudaMemcpyDeviceToHost, d.stream));
   SUBFV_CUDA(cudaStreamSynchronize(d.stream));
@@ -622,7 +626,7 @@ int subfv_lag_profile_steps(subfv_lag_state* s, int n_steps, double* kernel_ms) 
     SUBFV_CUDA(cudaEventRecord(ev[1], d.stream));
     launch_lag_node_only(d, s->sc, s->precision);
     SUBFV_CUDA(cudaEventRecord(ev[2], d.stream));
-    launch_lag_cell(d, s->sol6, s->rhs6, s->sc, &s->sc->dtmin, s->precision, 3);
+    launch_lag_cell(d, s->sol6, s->rhs6, s->sc, &s->sc->dtmin, 3);
     SUBFV_CUDA(cudaEventRecord(ev[3], d.stream));
     launch_lag_finalize(d, s->sc);
     SUBFV_CUDA(cudaEventRecord(ev[4], d.stream));

@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "handles.cuh"
+#include "geom_body.cuh"
 #include "lagrange.cuh"
 #include "pool.cuh"
 
@@ -118,6 +119,24 @@ int table_upload(subfv_lag_batch* b) {
   int* hdr = wc + (b->cap + 1);
   const int n = (int)b->order.size();
   wf[0] = wv[0] = wc[0] = 0;
+  int max_csf = 0, max_pairs = 0;
+  int64_t cells = 0;
+  for (int i = 0; i < n; ++i) {
+    cells += b->slots[b->order[i]].mesh->d.ne;
+    max_csf = std::max(max_csf, b->slots[b->order[i]].mesh->d.max_csf);
+    max_pairs = std::max(max_pairs, b->slots[b->order[i]].mesh->d.max_pairs);
+  }
+  const int small = cells <= geo::kTileCells;
+  if (n && (max_csf != b->tab.max_csf || max_pairs != b->tab.max_pairs || small != b->tab.small)) {
+    if (b->graph) {  // the captured step loop launches the cell kernels chosen for the old sizes
+      SUBFV_CUDA(cudaStreamSynchronize(b->stream));
+      cudaGraphExecDestroy(b->graph);
+      b->graph = nullptr;
+    }
+    b->tab.max_csf = max_csf;
+    b->tab.max_pairs = max_pairs;
+    b->tab.small = small;
+  }
   for (int i = 0; i < n; ++i) {
     Slot& q = b->slots[b->order[i]];
     LagItem& I = it[i];

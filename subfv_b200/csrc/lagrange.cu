@@ -7,12 +7,14 @@
 //                  per face; the node and cell kernels read them from the face record
 //   k_lag_node     one thread per vertex: nodal 3x3 system (Mp, Rp, Bp) over the
 //                  vertex's subfaces, inverse_3_by_3, vp
-//   k_lag_cell     one thread per cell: deterministic gather of the subface fluxes in
-//                  the reference's scatter order (no float atomics) -> rhs, and the
-//                  cell's CFL terms -> block min -> one atomicMin on the bit pattern
+//   k_lag_cell     one thread per cell (a tile of 32 cells per block on small meshes):
+//                  deterministic gather of the subface fluxes in the reference's scatter
+//                  order (no float atomics) -> rhs, and the cells' CFL terms -> minimum ->
+//                  atomicMin on the bit pattern
 //   k_lag_finalize one thread: dt = cfl*min, clip to t_max, t += dt
 //   k_lag_move     x += dt*vp
-//   k_geom<0>      geometry of the moved mesh, one thread per cell (mesh_dev.cu), fused
+//   k_geom<0>      geometry of the moved mesh, one thread per cell or a tile of
+//                  32 cells per block (mesh_dev.cu), fused
 //                  with sol += dt*rhs
 //
 // precision 0 (plain FP64) evaluates every expression in the reference's order and is
@@ -81,7 +83,7 @@ __device__ inline double lam_wall(double p_me, double tau_me) {
 // interior (xb = v_bar of :75), 1 a z-face of a one-layer slab (b2d), 2 a wall
 // (xb = p_l + l1 v_l).
 constexpr int kFrec = 6;
-constexpr int kNodeChunk = 4, kCellChunk = 2;
+constexpr int kNodeChunk = 4;
 
 template <int P>
 __device__ inline void lag_face_body(const DevMesh& m, const double* __restrict__ sol6, const int f) {
@@ -347,10 +349,132 @@ __device__ inline double warp_min(double x) {
   return x;
 }
 
-// mode bit 1: rhs, bit 2: CFL terms, bit 4: the rhs of scheme "sidil" (the nodal
-// pressure vp.w in place of the face's star pressures); every thread of the block calls
-// (block reduction)
-template <int P>
+// The cells' residuals and CFL terms in tiles of 32 cells: lane = cell, the entries of the
+// cell's list (one per subface it touches, 18 for a prism) spread over the warps, their five
+// flux terms in shared memory and summed in entry order by a warp per component.
+// mode bit 1: rhs, bit 2: CFL terms, bit 4: the rhs of scheme "sidil" (the nodal pressure
+// vp.w in place of the face's star pressures); every thread of the block calls.
+// The star pressures and the flux are FP64 at every precision: at precision 1 lambda is the
+// FP32 wave speed (stored as a double), the same value the nodal solve used, so sum over a
+// node of A (p*_L - p*_R) n = R - M v* closes to FP64 rounding and the totals stay conserved.
+// What bounds it: the gathers' latency. One thread per cell walked its entries two at a
+// time at 16 warps an SM (180,000 prisms 87 us, 3,000 prisms 19 us).
+constexpr int kCellEntries = 24, kCellWarps = 12;
+// two entries a warp, and at least the six warps of the summed components
+inline int lag_cell_warps(int entries) { return entries <= 12 ? 6 : entries <= 18 ? 9 : kCellWarps; }
+
+struct CellTile {
+  double term[5][kCellEntries][32];
+  double cell[4][32];  // pressure, sound speed, mass, 1 / mass
+  double dmin[kCellWarps];
+};
+
+__device__ inline void lag_cell_tile(const DevMesh& m, const double* __restrict__ sol6, double* __restrict__ rhs6,
+                                     double* dt_slot, const int mode, const int tile, CellTile& s) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, W = blockDim.x >> 5;
+  const int c = 32 * tile + lane, Q = m.max_csf;
+  const bool live = c < m.ne;
+  const int n = live ? m.csf_off[c + 1] - m.csf_off[c] : 0;
+  const int4* list = m.centry + ((size_t)tile * Q) * 32 + lane;  // entry q at list[32 q]
+  if (w == 0 && live) {
+    const U5 me = ld_u(sol6, c);
+    const double mass = ld_mass(sol6, c);
+    s.cell[0][lane] = me.p;
+    s.cell[1][lane] = sqrt(kGamma * me.p * me.t);
+    s.cell[2][lane] = mass;
+    s.cell[3][lane] = 1.0 / mass;
+  }
+  int4 E = w < n ? list[32 * w] : make_int4(-1, 0, 0, 0);
+  const double vse_c = live ? m.vol_se[c < m.nse ? c : 0] : 0.0;  // sub_elem(i) with i the cell (reference quirk)
+  __syncthreads();
+  double r = 0.0, dtloc = 1e6, dlo = 1e300, dhi = 0.0;
+  bool bad = false, any = false;
+  for (int base = 0; base < Q; base += kCellEntries) {
+    if (base) __syncthreads();  // the sums before the next terms
+    for (int q = base + w; q < min(base + kCellEntries, n); q += W) {
+      const double4 fn = m.fn[E.y];
+      const double area = m.sfa[E.x];
+      const int node = E.z & 0x3fffffff;
+      const bool right = (E.z >> 30) & 1;
+      const double4 vp = m.vp[node];
+      const double vsub = (mode & 2) && E.w >= 0 ? m.vol_se[E.w] : 0.0;
+      const int sub = E.w, sf = E.x;
+      double2 ll = make_double2(0.0, 0.0), vv = ll;
+      if ((mode & 5) == 1) {
+        const double2* fr = reinterpret_cast<const double2*>(m.frec + kFrec * (size_t)E.y);
+        ll = fr[0];
+        vv = fr[1];
+      }
+      if (q + W < n) E = list[32 * (q + W)];  // the next entry while this one's terms form
+      if (mode & 1) {
+        const double v_et = dot3(vp.x, vp.y, vp.z, fn.x, fn.y, fn.z);
+        const double am = div_by(area, s.cell[2][lane], s.cell[3][lane]);
+        double ps;
+        if (mode & 4) {  // sidil: flux (-v.n, pp n, pp v.n) of the vertex
+          ps = vp.w;
+        } else {  // lambda and v.n of this cell's side
+          const double lam = right ? ll.y : ll.x, vme = right ? vv.y : vv.x, x = lam * (v_et - vme);
+          ps = right ? s.cell[0][lane] + x : s.cell[0][lane] - x;
+        }
+        const double sg = right ? 1.0 : -1.0;  // r - t and r + (-t) are the same
+        double* t = &s.term[0][q - base][lane];
+        constexpr int tc = kCellEntries * 32;
+        t[0] = sg * (am * (-v_et));
+        t[tc] = sg * (am * (ps * fn.x));
+        t[2 * tc] = sg * (am * (ps * fn.y));
+        t[3 * tc] = sg * (am * (ps * fn.z));
+        t[4 * tc] = sg * (am * (ps * v_et));
+      }
+      if (mode & 2) {  // compute_dt terms for (cell, subface)
+        const double sg = right ? -1.0 : 1.0;
+        // the subface's own vertex (the owning node unless the node list is a periodic extension)
+        const double4 vps = m.vsf_identity ? vp : m.vp[m.sf_vert[sf]];
+        const double d = area * s.cell[1][lane];  // vse_c / d, least where d is largest: divided once below
+        bad = bad || !(d >= 0.0) || (d == 0.0 && vse_c == 0.0);
+        dlo = d < dlo ? d : dlo;
+        dhi = d > dhi ? d : dhi;
+        any = true;
+        const double vn = dot3(vps.x, vps.y, vps.z, sg * fn.x, sg * fn.y, sg * fn.z);
+        const double t2 = sub >= 0 ? qdiv(0.8 * vsub, 1e-8 + fabs(vn) * fn.w) : 1e6;
+        if (t2 < dtloc) dtloc = t2;
+        bad = bad || !(t2 >= 0.0);
+      }
+    }
+    if (mode & 1) {
+      __syncthreads();
+      if (w < 5)
+        for (int q = base; q < min(base + kCellEntries, n); ++q) r = r + s.term[w][q - base][lane];
+    }
+  }
+  if ((mode & 1) && w < 6 && live) rhs6[kRhs * (size_t)c + w] = r;  // the sixth is the pad, 0
+  if (mode & 2) {
+    if (any) {
+      const double t1 = vse_c / (vse_c < 0.0 ? dlo : dhi);
+      if (t1 < dtloc) dtloc = t1;
+      bad = bad || !(t1 >= 0.0);
+    }
+    const double x = warp_min(dtloc);
+    if (lane == 0) s.dmin[w] = x;
+    __syncthreads();
+    if (w == 0) {
+      const double y = warp_min(lane < W ? s.dmin[lane] : 1e6);
+      if (lane == 0) atomic_min_pos(dt_slot, y);
+    }
+  }
+  if (bad) atomicOr(m.status, kErrNonFinite);
+}
+__global__ void __launch_bounds__(32 * kCellWarps) k_lag_cell_tile(DevMesh m, const double* __restrict__ sol6,
+                                                                   double* __restrict__ rhs6, LagScalars* sc,
+                                                                   double* dt_slot, int mode) {
+  if (sc && sc->done) return;
+  __shared__ CellTile s;
+  lag_cell_tile(m, sol6, rhs6, dt_slot, mode, blockIdx.x, s);
+}
+
+// The same, one thread per cell, for meshes that fill the GPU this way: fewer instructions
+// (no terms through shared memory, the cell's values in registers), while the entries of a
+// cell are one chain. Whole warps call.
+constexpr int kCellChunk = 2;
 __device__ inline void lag_cell_body(const DevMesh& m, const double* __restrict__ sol6, double* __restrict__ rhs6,
                                      double* dt_slot, const int mode, const int c) {
   double dtloc = 1e6;
@@ -362,14 +486,15 @@ __device__ inline void lag_cell_body(const DevMesh& m, const double* __restrict_
     double r0 = 0, r1 = 0, r2 = 0, r3 = 0, r4 = 0;
     bool bad = false;
     const double vse_c = m.vol_se[c < m.nse ? c : 0];  // sub_elem(i) with i the cell (reference quirk)
-    const int q1 = m.csf_off[c + 1];
+    const int q1 = m.csf_off[c + 1] - m.csf_off[c];
+    const int4* list = m.centry + geo::tile_entry(c, m.max_csf, 0);  // entry q at list[32 q]
     // entries in chunks of kCellChunk: the chunk's loads are issued together, then the
     // sums run in entry order; the next chunk's entries are loaded while they run
-    int q = m.csf_off[c];
+    int q = 0;
     int4 Ec[kCellChunk];
 #pragma unroll
     for (int u = 0; u < kCellChunk; ++u)
-      if (q + u < q1) Ec[u] = m.centry[q + u];
+      if (q + u < q1) Ec[u] = list[32 * (q + u)];
     for (; q < q1; q += kCellChunk) {
       double4 fnc[kCellChunk], vpc[kCellChunk];
       double2 llc[kCellChunk], vvc[kCellChunk];
@@ -392,7 +517,7 @@ __device__ inline void lag_cell_body(const DevMesh& m, const double* __restrict_
       int4 En[kCellChunk];
 #pragma unroll
       for (int u = 0; u < kCellChunk; ++u)
-        if (q + kCellChunk + u < q1) En[u] = m.centry[q + kCellChunk + u];
+        if (q + kCellChunk + u < q1) En[u] = list[32 * (q + kCellChunk + u)];
 #pragma unroll
       for (int u = 0; u < kCellChunk; ++u) {
         if (q + u >= q1) break;
@@ -421,10 +546,6 @@ __device__ inline void lag_cell_body(const DevMesh& m, const double* __restrict_
           double v_et = dot3(vpn.x, vpn.y, vpn.z, fn.x, fn.y, fn.z);
           double am = area / mass;
           const double2 ll = llc[u], vv = vvc[u];
-          // The star pressures and the flux in FP64 at every precision: at precision 1
-          // lambda is the FP32 wave speed (stored as a double), the same value the nodal
-          // solve used, so sum over a node of A (p*_L - p*_R) n = R - M v* closes to FP64
-          // rounding and the totals stay conserved.
           if (side == 0) {  // this cell is the face's left neighbour: lambda of its side, v.n
             double lam = ll.x, vme = vv.x;
             double ps = pme - lam * (v_et - vme);
@@ -466,26 +587,17 @@ __device__ inline void lag_cell_body(const DevMesh& m, const double* __restrict_
     }
     if (bad) atomicOr(m.status, kErrNonFinite);
   }
-  if (mode & 2) {
-    __shared__ double wmin[32];
-    double x = warp_min(dtloc);
-    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) wmin[wid] = x;
-    __syncthreads();
-    if (wid == 0) {
-      int nw = (blockDim.x + 31) >> 5;
-      x = lane < nw ? wmin[lane] : 1e6;
-      x = warp_min(x);
-      if (lane == 0) atomic_min_pos(dt_slot, x);
-    }
+  if (mode & 2) {  // a warp's minimum goes to the slot only where it lowers it
+    const double x = warp_min(dtloc);
+    if ((threadIdx.x & 31) == 0 && x < *(volatile double*)dt_slot) atomic_min_pos(dt_slot, x);
   }
 }
-template <int P>
 __global__ void __launch_bounds__(128) k_lag_cell(DevMesh m, const double* __restrict__ sol6, double* __restrict__ rhs6,
                                                   LagScalars* sc, double* dt_slot, int mode) {
   if (sc && sc->done) return;
-  lag_cell_body<P>(m, sol6, rhs6, dt_slot, mode, blockIdx.x * blockDim.x + threadIdx.x);
+  lag_cell_body(m, sol6, rhs6, dt_slot, mode, blockIdx.x * blockDim.x + threadIdx.x);
 }
+
 
 // dt = cfl*dt; if (t + dt > t_max) dt = t_max - t; t = t + dt (lagrange_main.F90:102-116)
 __device__ inline void lag_finalize_body(LagScalars* sc) {
@@ -552,16 +664,28 @@ __global__ void __launch_bounds__(kLagVertBlock) kb_lag_node(const LagItem* __re
     lag_node_body<P>(I.m, (w - wv[p]) * kLagVertBlock + threadIdx.x);
   }
 }
-template <int P>
-__global__ void __launch_bounds__(kLagCellBlock) kb_lag_cell(const LagItem* __restrict__ it,
-                                                             const int* __restrict__ wc, const int* __restrict__ hdr) {
+__global__ void __launch_bounds__(32 * kCellWarps) kb_lag_cell_tile(const LagItem* __restrict__ it,
+                                                                    const int* __restrict__ wc,
+                                                                    const int* __restrict__ hdr) {
+  __shared__ CellTile s;
   const int n = hdr[0];
   for (int w = blockIdx.x; w < wc[n]; w += gridDim.x) {
     const int p = lag_item_of(wc, n, w);
     const LagItem& I = it[p];
     if (I.sc->done) continue;
-    lag_cell_body<P>(I.m, I.sol6, I.rhs6, &I.sc->dtmin, 3, (w - wc[p]) * kLagCellBlock + threadIdx.x);
-    __syncthreads();  // the block-reduction scratch is reused by the next work block
+    lag_cell_tile(I.m, I.sol6, I.rhs6, &I.sc->dtmin, 3, w - wc[p], s);
+    __syncthreads();  // the shared memory is reused by the next tile
+  }
+}
+// a warp per tile
+__global__ void __launch_bounds__(64) kb_lag_cell(const LagItem* __restrict__ it, const int* __restrict__ wc,
+                                                  const int* __restrict__ hdr) {
+  const int n = hdr[0];
+  for (int w = 2 * blockIdx.x + (threadIdx.x >> 5); w < wc[n]; w += 2 * gridDim.x) {
+    const int p = lag_item_of(wc, n, w);
+    const LagItem& I = it[p];
+    if (I.sc->done) continue;
+    lag_cell_body(I.m, I.sol6, I.rhs6, &I.sc->dtmin, 3, 32 * (w - wc[p]) + (threadIdx.x & 31));
   }
 }
 __global__ void kb_lag_finalize(const LagItem* __restrict__ it, const int* __restrict__ hdr) {
@@ -588,16 +712,29 @@ __global__ void __launch_bounds__(kLagFaceBlock) kb_face_geom(const LagItem* __r
     geo::face_geom_body<0>(I.m, face_at(I.m, (w - wf[p]) * kLagFaceBlock + threadIdx.x));
   }
 }
-__global__ void __launch_bounds__(geo::kGeoBlock) kb_geom_step(const LagItem* __restrict__ it,
-                                                               const int* __restrict__ wc,
-                                                               const int* __restrict__ hdr) {
-  static_assert(geo::kGeoBlock == kLagCellBlock, "cell work blocks");
+__global__ void __launch_bounds__(geo::kGeoThreads) kb_geom_step_tile(const LagItem* __restrict__ it,
+                                                                      const int* __restrict__ wc,
+                                                                      const int* __restrict__ hdr) {
+  extern __shared__ __align__(16) char smem[];
   const int n = hdr[0];
   for (int w = blockIdx.x; w < wc[n]; w += gridDim.x) {
     const int p = lag_item_of(wc, n, w);
     const LagItem& I = it[p];
     if (I.sc->skip) continue;
-    geo::geom_step_body(I.m, I.sol6, I.rhs6, I.sc->dt, (w - wc[p]) * kLagCellBlock + threadIdx.x);
+    geo::geom_step_tile(I.m, I.sol6, I.rhs6, I.sc->dt, w - wc[p], *reinterpret_cast<geo::GeoTile*>(smem));
+    __syncthreads();
+  }
+}
+
+__global__ void __launch_bounds__(geo::kGeoBlock) kb_geom_step(const LagItem* __restrict__ it,
+                                                               const int* __restrict__ wc,
+                                                               const int* __restrict__ hdr) {
+  const int n = hdr[0];
+  for (int w = 2 * blockIdx.x + (threadIdx.x >> 5); w < wc[n]; w += 2 * gridDim.x) {
+    const int p = lag_item_of(wc, n, w);
+    const LagItem& I = it[p];
+    if (I.sc->skip) continue;
+    geo::geom_step_body(I.m, I.sol6, I.rhs6, I.sc->dt, 32 * (w - wc[p]) + (threadIdx.x & 31));
   }
 }
 
@@ -636,19 +773,23 @@ __global__ void k_set_scalar(double* p, double v) { *p = v; }
 // position p (bit 30: side) and the cell's subcell on the subface; one 16-byte record
 // instead of four dependent lookups in k_lag_cell.
 __global__ void k_build_cell_entries(DevMesh m) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= m.ncsf) return;
-  const int e = m.csf[q];
-  const int p = e >> 1, side = e & 1;
-  const int sf = m.vsf_identity ? p : m.vsf[p];
-  const int node = m.vsf_identity ? m.sf_vert[sf] : m.p_node[p];
-  const int2 se = m.sf_se[sf];
-  m.centry[q] = make_int4(sf, m.sf_face[sf], node | (side << 30), side == 0 ? se.x : se.y);
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= m.ne) return;
+  const int q0 = m.csf_off[c], n = m.csf_off[c + 1] - q0;
+  for (int q = 0; q < n; ++q) {
+    const int e = m.csf[q0 + q];
+    const int p = e >> 1, side = e & 1;
+    const int sf = m.vsf_identity ? p : m.vsf[p];
+    const int node = m.vsf_identity ? m.sf_vert[sf] : m.p_node[p];
+    const int2 se = m.sf_se[sf];
+    m.centry[geo::tile_entry(c, m.max_csf, q)] =
+        make_int4(sf, m.sf_face[sf], node | (side << 30), side == 0 ? se.x : se.y);
+  }
 }
 
 }  // namespace
 
-constexpr int kBlkNode = 128, kBlkCell = 128, kBlkVert = 256;
+constexpr int kBlkNode = 128, kBlkVert = 256;
 
 void launch_lag_node(const DevMesh& m, const double* sol6, const LagScalars* sc, int precision) {
   if (precision == 1) {
@@ -671,12 +812,12 @@ void launch_lag_sidil_node(const DevMesh& m, const double* sol6, const LagScalar
   launch_vert_volume(m);  // V_p of the current (moved) mesh
   k_lag_sidil_node<<<grid_for(m.nv, kBlkNode), kBlkNode, 0, m.stream>>>(m, sol6, sc, method);
 }
-void launch_lag_cell(const DevMesh& m, const double* sol6, double* rhs6, LagScalars* sc, double* dt_slot,
-                     int precision, int mode) {
-  if (precision == 1)
-    k_lag_cell<1><<<grid_for(m.ne, kBlkCell), kBlkCell, 0, m.stream>>>(m, sol6, rhs6, sc, dt_slot, mode);
+void launch_lag_cell(const DevMesh& m, const double* sol6, double* rhs6, LagScalars* sc, double* dt_slot, int mode) {
+  if (m.ne <= geo::kTileCells)
+    k_lag_cell_tile<<<grid_for(m.ne, 32), 32 * lag_cell_warps(m.max_csf), 0, m.stream>>>(m, sol6, rhs6, sc, dt_slot,
+                                                                                         mode);
   else
-    k_lag_cell<0><<<grid_for(m.ne, kBlkCell), kBlkCell, 0, m.stream>>>(m, sol6, rhs6, sc, dt_slot, mode);
+    k_lag_cell<<<grid_for(m.ne, 128), 128, 0, m.stream>>>(m, sol6, rhs6, sc, dt_slot, mode);
 }
 void launch_lag_finalize(const DevMesh& m, LagScalars* sc) { k_lag_finalize<<<1, 1, 0, m.stream>>>(sc); }
 void launch_lag_move(const DevMesh& m, const LagScalars* sc, double dt_host) {
@@ -692,7 +833,7 @@ void launch_vp_out(const DevMesh& m, double* out) { k_vp_out<<<grid_for(m.nv, 25
 void launch_vp_in(const DevMesh& m, const double* in) { k_vp_in<<<grid_for(m.nv, 256), 256, 0, m.stream>>>(m.nv, in, m.vp); }
 void launch_set_scalar(const DevMesh& m, double* p, double v) { k_set_scalar<<<1, 1, 0, m.stream>>>(p, v); }
 void launch_build_cell_entries(const DevMesh& m) {
-  k_build_cell_entries<<<grid_for(m.ncsf, 256), 256, 0, m.stream>>>(m);
+  k_build_cell_entries<<<grid_for(m.ne, 128), 128, 0, m.stream>>>(m);
 }
 
 void launch_lag_batch_step(const LagTable& t, int precision, cudaStream_t s) {
@@ -700,16 +841,22 @@ void launch_lag_batch_step(const LagTable& t, int precision, cudaStream_t s) {
   if (precision == 1) {
     kb_lag_face<1><<<g, kLagFaceBlock, 0, s>>>(t.items, t.wf, t.hdr);
     kb_lag_node<1><<<g, kLagVertBlock, 0, s>>>(t.items, t.wv, t.hdr);
-    kb_lag_cell<1><<<g, kLagCellBlock, 0, s>>>(t.items, t.wc, t.hdr);
   } else {
     kb_lag_face<0><<<g, kLagFaceBlock, 0, s>>>(t.items, t.wf, t.hdr);
     kb_lag_node<0><<<g, kLagVertBlock, 0, s>>>(t.items, t.wv, t.hdr);
-    kb_lag_cell<0><<<g, kLagCellBlock, 0, s>>>(t.items, t.wc, t.hdr);
   }
+  if (t.small) kb_lag_cell_tile<<<g, 32 * lag_cell_warps(t.max_csf), 0, s>>>(t.items, t.wc, t.hdr);
+  else kb_lag_cell<<<g, 64, 0, s>>>(t.items, t.wc, t.hdr);
   kb_lag_finalize<<<gp, 128, 0, s>>>(t.items, t.hdr);
   kb_lag_move<<<g, kLagVertBlock, 0, s>>>(t.items, t.wv, t.hdr);
   kb_face_geom<<<g, kLagFaceBlock, 0, s>>>(t.items, t.wf, t.hdr);
-  kb_geom_step<<<g, geo::kGeoBlock, 0, s>>>(t.items, t.wc, t.hdr);
+  if (t.small) {
+    constexpr int smem = (int)sizeof(geo::GeoTile);
+    cudaFuncSetAttribute(kb_geom_step_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    kb_geom_step_tile<<<g, 32 * geo::geo_warps(t.max_pairs), smem, s>>>(t.items, t.wc, t.hdr);
+  } else {
+    kb_geom_step<<<g, geo::kGeoBlock, 0, s>>>(t.items, t.wc, t.hdr);
+  }
 }
 
 // One full time step of lagrange_main.F90:89-127 (graph-capturable: no host sync);
@@ -718,10 +865,10 @@ void enqueue_lag_step_head(const DevMesh& m, double* sol6, double* rhs6, LagScal
                            int method) {
   if (scheme == 1) {
     launch_lag_sidil_node(m, sol6, sc, method);
-    launch_lag_cell(m, sol6, rhs6, sc, &sc->dtmin, 0, 7);
+    launch_lag_cell(m, sol6, rhs6, sc, &sc->dtmin, 7);
   } else {
     launch_lag_node(m, sol6, sc, precision);
-    launch_lag_cell(m, sol6, rhs6, sc, &sc->dtmin, precision, 3);
+    launch_lag_cell(m, sol6, rhs6, sc, &sc->dtmin, 3);
   }
   launch_lag_finalize(m, sc);
 }

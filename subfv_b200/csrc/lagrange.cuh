@@ -11,8 +11,7 @@ void launch_lag_node(const DevMesh& m, const double* sol6, const LagScalars* sc,
 void launch_lag_face_only(const DevMesh& m, const double* sol6, const LagScalars* sc, int precision);
 void launch_lag_node_only(const DevMesh& m, const LagScalars* sc, int precision);
 // mode bit 1: rhs into rhs6; bit 2: CFL terms min-reduced into *dt_slot
-void launch_lag_cell(const DevMesh& m, const double* sol6, double* rhs6, LagScalars* sc, double* dt_slot,
-                     int precision, int mode);
+void launch_lag_cell(const DevMesh& m, const double* sol6, double* rhs6, LagScalars* sc, double* dt_slot, int mode);
 void launch_lag_finalize(const DevMesh& m, LagScalars* sc);
 void launch_lag_move(const DevMesh& m, const LagScalars* sc, double dt_host);
 void launch_pack6(const DevMesh& m, int n, const double* s5, const double* mass, double* s6);
@@ -21,7 +20,7 @@ void launch_unpack6(const DevMesh& m, int n, int stride, const double* s6, doubl
 void launch_vp_out(const DevMesh& m, double* out);
 void launch_vp_in(const DevMesh& m, const double* in);
 void launch_set_scalar(const DevMesh& m, double* p, double v);
-// fills m.centry (allocated by the caller, ncsf records) from the cell CSR
+// fills m.centry (allocated by the caller, all bits set) from the cell CSR
 void launch_build_cell_entries(const DevMesh& m);
 // scheme 0 "classic", 1 "sidil" (method_length `method`, FP64)
 // the step up to lagrange_finalize (nodal solve, fluxes, dt); the rest is move_mesh and
@@ -43,11 +42,13 @@ struct LagItem {
 // Table of in-flight problems: items, work-block prefixes over faces (wf, kLagFaceBlock
 // faces per block), vertices (wv, kLagVertBlock) and cells (wc, kLagCellBlock), and
 // hdr[0] = the number of problems; persistent grids of `grid` blocks.
-constexpr int kLagFaceBlock = 128, kLagVertBlock = 128, kLagCellBlock = 64;
+constexpr int kLagFaceBlock = 128, kLagVertBlock = 128, kLagCellBlock = 32;
 struct LagTable {
   LagItem* items = nullptr;
   int *wf = nullptr, *wv = nullptr, *wc = nullptr, *hdr = nullptr;
   int cap = 0, grid = 1;
+  int max_csf = 0, max_pairs = 0;  // the largest of any problem's mesh (the cell kernels' warps)
+  int small = 0;                   // the table's cells are few enough for the tiled cell kernels
 };
 // One step of lagrange_main.F90:89-127 for every problem of the table, in shared launches.
 void launch_lag_batch_step(const LagTable& t, int precision, cudaStream_t s);

@@ -283,6 +283,12 @@ int devmesh_create(const subfv_mesh_desc* d, DevMesh* m) {
     }
   }
   m->ncsf = csf_off[ne];
+  for (int c = 0; c < ne; ++c) {
+    m->max_csf = std::max(m->max_csf, csf_off[c + 1] - csf_off[c]);
+    int pairs = 0;
+    for (int k = 0; k < 8 && ef8[8 * (size_t)c + k] >= 0; ++k) pairs += fvert[ef8[8 * (size_t)c + k]].w < 0 ? 3 : 4;
+    m->max_pairs = std::max(m->max_pairs, std::min(pairs, geo::kGeoPairs));
+  }
   std::vector<int> vel_off(nv + 1, 0), vel;
   if (d->vert_elem_off && d->vert_elem) {
     for (int v = 0; v <= nv; ++v) vel_off[v] = d->vert_elem_off[v];
@@ -388,7 +394,7 @@ void devmesh_free(DevMesh* m) {
                   m->sf_face, m->sf_vert, m->sf_se, m->sf_loc, m->sfn, m->sfa, m->se_elem, m->se_vert, m->se_loc,
                   m->se_sf, m->vol_se, m->ev_off, m->ev, m->ef8, m->ekind, m->cc, m->vol, m->vsf_off,
                   m->vsf, m->p_node, m->vse_off, m->vse, m->csf_off, m->csf, m->status,
-                  m->vel_off, m->vel, m->cse_sorted, m->frec, m->centry, m->fS, m->fpos, m->gface, m->gsub, m->forder, m->vorder,
+                  m->vel_off, m->vel, m->cse_sorted, m->frec, m->centry, m->fS, m->fpos, m->cinfo, m->gpair, m->gsub, m->forder, m->vorder,
                   m->dsf_off, m->dsf, m->dsf_se, m->dsf_seloc, m->dse_off, m->dse, m->dse_sfloc,
                   m->dcache, m->dcache_off, m->npinv, m->vslot, m->vcorner};
   diffusion_cache_forget(m);
@@ -523,6 +529,13 @@ __global__ void __launch_bounds__(128) k_face_geom(DevMesh m, const LagScalars* 
   geo::face_geom_body<FULL>(m, face_at(m, blockIdx.x * blockDim.x + threadIdx.x));
 }
 
+__global__ void __launch_bounds__(geo::kGeoThreads) k_geom_step_tile(DevMesh m, double* sol6, const double* rhs6,
+                                                                     const LagScalars* sc) {
+  if (sc && sc->skip) return;
+  extern __shared__ __align__(16) char smem[];
+  geo::geom_step_tile(m, sol6, rhs6, sol6 ? sc->dt : 0.0, blockIdx.x, *reinterpret_cast<geo::GeoTile*>(smem));
+}
+
 __global__ void __launch_bounds__(geo::kGeoBlock) k_geom_step(DevMesh m, double* sol6, const double* rhs6,
                                                               const LagScalars* sc) {
   if (sc && sc->skip) return;
@@ -577,7 +590,13 @@ void launch_face_geometry_step(const DevMesh& m, const LagScalars* sc) {
   k_face_geom<0><<<grid_for(m.nf, 128), 128, 0, m.stream>>>(m, sc);
 }
 void launch_cell_geometry_step(const DevMesh& m, double* sol6, const double* rhs6, const LagScalars* sc) {
-  k_geom_step<<<grid_for(m.ne, geo::kGeoBlock), geo::kGeoBlock, 0, m.stream>>>(m, sol6, rhs6, sc);
+  if (m.ne <= geo::kTileCells) {
+    constexpr int smem = (int)sizeof(geo::GeoTile);
+    cudaFuncSetAttribute(k_geom_step_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    k_geom_step_tile<<<grid_for(m.ne, 32), 32 * geo::geo_warps(m.max_pairs), smem, m.stream>>>(m, sol6, rhs6, sc);
+  } else {
+    k_geom_step<<<grid_for(m.ne, geo::kGeoBlock), geo::kGeoBlock, 0, m.stream>>>(m, sol6, rhs6, sc);
+  }
 }
 void launch_lag_update(const DevMesh& m, double* sol6, const double* rhs6, const LagScalars* sc) {
   k_lag_update<<<grid_for(m.ne, 256), 256, 0, m.stream>>>(m, sol6, rhs6, sc);

@@ -30,6 +30,7 @@ struct DevMesh {
   int vsf_identity = 0;  // vsf[p] == p for every p (no periodic extension)
   int max_vsf = 0, max_vse = 0;  // the most subfaces / subcells around one vertex
   int max_evc = 0;               // the most vertices of one cell
+  int max_csf = 0, max_pairs = 0;  // the most entries (csf) and (face, vertex) pairs of one cell
   // vertices
   double4* x = nullptr;
   double4* vp = nullptr;
@@ -51,17 +52,20 @@ struct DevMesh {
   // Lagrangian face records (6 doubles per face, allocated on first Lagrangian use):
   // wave speeds and normal velocities of the face's two sides for the current state
   double* frec = nullptr;
-  // per cell-CSR entry: subface, face, owning node | side << 30, subcell (Lagrangian
-  // cell kernel; built on first Lagrangian use)
+  // per cell and position q of its list of node-ordered subface entries (csf): subface (-1:
+  // none), face, owning node | side << 30, subcell; in tiles of 32 cells, entry q of cell c
+  // at centry[((c / 32) max_csf + q) 32 + c % 32], so that a warp's lanes, one cell each,
+  // read consecutive records (Lagrangian cell kernel; built on first Lagrangian use)
   int4* centry = nullptr;
   // per face: sum of area * unit normal over its subfaces (Lagrangian step's mesh check)
   double4* fS = nullptr;
   // Static local topology for the geometry kernels (the topology never changes, so the
   // per-step kernels need no id searches; layouts in geom_body.cuh). fpos: per face,
-  // built at creation; gface (8 per cell, face slot order of ef8) and gsub (per subcell):
-  // built on first Lagrangian use.
+  // built at creation; cinfo (per cell), gpair (per cell and pair of face and vertex, in
+  // tiles of 32 cells as centry) and gsub (per subcell): built on first Lagrangian use.
   uint8_t* fpos = nullptr;
-  uint16_t* gface = nullptr;
+  uint32_t* cinfo = nullptr;
+  uint32_t* gpair = nullptr;
   uint32_t* gsub = nullptr;
   // Launch orders (built at creation): the faces grouped by vertex count and interior /
   // boundary, the vertices by subface count, subcell count and boundary subfaces, each
@@ -175,8 +179,8 @@ void launch_cell_geometry_step(const DevMesh& m, double* sol6, const double* rhs
 // sol += dt*rhs alone (the update launch_geometry otherwise fuses in)
 void launch_lag_update(const DevMesh& m, double* sol6, const double* rhs6, const LagScalars* sc);
 void launch_vert_volume(const DevMesh& m);
-// the static local-topology codes of the Lagrangian geometry kernel (gface, gsub must be
-// allocated: 8 per cell, one per subcell)
+// the static local-topology codes of the Lagrangian geometry kernel (cinfo, gpair and gsub
+// must be allocated)
 void launch_build_geom_codes(const DevMesh& m);
 void launch_vert_is_bound(const DevMesh& m);
 
