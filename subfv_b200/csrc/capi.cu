@@ -9,6 +9,7 @@
 #include "handles.cuh"
 #include "lagrange.cuh"
 #include "mesh_dev.cuh"
+#include "pool.cuh"
 #include "topology.h"
 
 namespace subfv {
@@ -114,6 +115,25 @@ int ensure_full_geometry(DevMesh& d) {
   SUBFV_CUDA(cudaStreamSynchronize(d.stream));
   SUBFV_CUDA(cudaGetLastError());
   d.geom_partial = 0;
+  return 0;
+}
+// a vertex array to or from the host's (3, n_vert), converted on the device
+int xyz_to_host(DevMesh& d, const double4* a, double* out) {
+  double* t = nullptr;
+  if (pool_alloc((void**)&t, 3 * (size_t)d.nv * sizeof(double), d.stream)) return -1;
+  launch_xyz_out(d, a, t);
+  const cudaError_t e = cudaMemcpyAsync(out, t, 3 * (size_t)d.nv * sizeof(double), cudaMemcpyDeviceToHost, d.stream);
+  cudaFreeAsync(t, d.stream);
+  SUBFV_CUDA(e);
+  return 0;
+}
+int xyz_from_host(DevMesh& d, const double* in, double4* a) {
+  double* t = nullptr;
+  if (pool_alloc((void**)&t, 3 * (size_t)d.nv * sizeof(double), d.stream)) return -1;
+  const cudaError_t e = cudaMemcpyAsync(t, in, 3 * (size_t)d.nv * sizeof(double), cudaMemcpyHostToDevice, d.stream);
+  if (e == cudaSuccess) launch_xyz_in(d, t, a);
+  cudaFreeAsync(t, d.stream);
+  SUBFV_CUDA(e);
   return 0;
 }
 int load_sol(subfv_mesh* m, const double* sol, const double* mass) {
@@ -259,23 +279,17 @@ int64_t subfv_mesh_device_bytes(const subfv_mesh* m) { return (int64_t)m->d.byte
 
 int subfv_mesh_set_coords(subfv_mesh* m, const double* c) {
   DevMesh& d = m->d;
-  std::vector<double4> x(d.nv);
-  for (int i = 0; i < d.nv; ++i) x[i] = make_double4(c[3 * i], c[3 * i + 1], c[3 * i + 2], 0.0);
-  SUBFV_CUDA(cudaMemcpyAsync(d.x, x.data(), x.size() * sizeof(double4), cudaMemcpyHostToDevice, d.stream));
+  if (xyz_from_host(d, c, d.x)) return -1;
   SUBFV_CUDA(cudaStreamSynchronize(d.stream));
+  SUBFV_CUDA(cudaGetLastError());
   ++d.geom_epoch;
   return 0;
 }
 int subfv_mesh_get_coords(subfv_mesh* m, double* c) {
   DevMesh& d = m->d;
-  std::vector<double4> x(d.nv);
-  SUBFV_CUDA(cudaMemcpyAsync(x.data(), d.x, x.size() * sizeof(double4), cudaMemcpyDeviceToHost, d.stream));
+  if (xyz_to_host(d, d.x, c)) return -1;
   SUBFV_CUDA(cudaStreamSynchronize(d.stream));
-  for (int i = 0; i < d.nv; ++i) {
-    c[3 * i] = x[i].x;
-    c[3 * i + 1] = x[i].y;
-    c[3 * i + 2] = x[i].z;
-  }
+  SUBFV_CUDA(cudaGetLastError());
   return 0;
 }
 
@@ -341,14 +355,8 @@ int subfv_compute_rhs_lagrange(subfv_mesh* m, const double* sol, double* vp, dou
   launch_lag_cell(d, m->sol6, m->rhs6, nullptr, nullptr, 1);
   launch_unpack6(d, d.ne, kRhs, m->rhs6, m->stage);
   SUBFV_CUDA(cudaMemcpyAsync(rhs, m->stage, 5 * (size_t)d.ne * sizeof(double), cudaMemcpyDeviceToHost, d.stream));
-  std::vector<double4> h(d.nv);
-  SUBFV_CUDA(cudaMemcpyAsync(h.data(), d.vp, d.nv * sizeof(double4), cudaMemcpyDeviceToHost, d.stream));
+  if (xyz_to_host(d, d.vp, vp)) return -1;
   SUBFV_CUDA(cudaStreamSynchronize(d.stream));
-  for (int i = 0; i < d.nv; ++i) {
-    vp[3 * i] = h[i].x;
-    vp[3 * i + 1] = h[i].y;
-    vp[3 * i + 2] = h[i].z;
-  }
   SUBFV_CUDA(cudaGetLastError());
   return check_status(d);
 }
@@ -367,14 +375,8 @@ int subfv_compute_rhs_lagrange_sidil(subfv_mesh* m, const double* sol, double* v
   launch_lag_cell(d, m->sol6, m->rhs6, nullptr, nullptr, 5);
   launch_unpack6(d, d.ne, kRhs, m->rhs6, m->stage);
   SUBFV_CUDA(cudaMemcpyAsync(rhs, m->stage, 5 * (size_t)d.ne * sizeof(double), cudaMemcpyDeviceToHost, d.stream));
-  std::vector<double4> h(d.nv);
-  SUBFV_CUDA(cudaMemcpyAsync(h.data(), d.vp, d.nv * sizeof(double4), cudaMemcpyDeviceToHost, d.stream));
+  if (xyz_to_host(d, d.vp, vp)) return -1;
   SUBFV_CUDA(cudaStreamSynchronize(d.stream));
-  for (int i = 0; i < d.nv; ++i) {
-    vp[3 * i] = h[i].x;
-    vp[3 * i + 1] = h[i].y;
-    vp[3 * i + 2] = h[i].z;
-  }
   SUBFV_CUDA(cudaGetLastError());
   return check_status(d);
 }
@@ -402,7 +404,7 @@ int subfv_compute_dt(subfv_mesh* m, const double* sol, double cfl, const double*
   if (ensure_scratch(m) || clear_status(d)) return -1;
   if (load_sol(m, sol, nullptr)) return -1;
   SUBFV_CUDA(cudaMemcpyAsync(m->stage, vp, 3 * (size_t)d.nv * sizeof(double), cudaMemcpyHostToDevice, d.stream));
-  launch_vp_in(d, m->stage);
+  launch_xyz_in(d, m->stage, d.vp);
   double* slot = &m->sc->dtmin;
   launch_set_scalar(d, slot, 1e6);
   launch_lag_cell(d, m->sol6, nullptr, nullptr, slot, 2);
@@ -419,7 +421,7 @@ int subfv_move_mesh(subfv_mesh* m, const double* vp, double dt) {
   ++d.geom_epoch;
   if (ensure_scratch(m)) return -1;
   SUBFV_CUDA(cudaMemcpyAsync(m->stage, vp, 3 * (size_t)d.nv * sizeof(double), cudaMemcpyHostToDevice, d.stream));
-  launch_vp_in(d, m->stage);
+  launch_xyz_in(d, m->stage, d.vp);
   launch_lag_move(d, nullptr, dt);
   SUBFV_CUDA(cudaStreamSynchronize(d.stream));
   SUBFV_CUDA(cudaGetLastError());
@@ -552,14 +554,8 @@ int subfv_lag_set_sol(subfv_lag_state* s, const double* sol) {
 }
 int subfv_lag_get_vp(subfv_lag_state* s, double* vp) {
   DevMesh& d = s->m->d;
-  std::vector<double4> h(d.nv);
-  SUBFV_CUDA(cudaMemcpyAsync(h.data(), d.vp, d.nv * sizeof(double4), cudaMemcpyDeviceToHost, d.stream));
+  if (xyz_to_host(d, d.vp, vp)) return -1;
   SUBFV_CUDA(cudaStreamSynchronize(d.stream));
-  for (int i = 0; i < d.nv; ++i) {
-    vp[3 * i] = h[i].x;
-    vp[3 * i + 1] = h[i].y;
-    vp[3 * i + 2] = h[i].z;
-  }
   return 0;
 }
 int subfv_lag_last_dt(subfv_lag_state* s, double* dt) {

@@ -767,6 +767,19 @@ __global__ void k_vp_in(int n, const double* __restrict__ in, double4* __restric
   if (v >= n) return;
   vp[v] = make_double4(in[3 * (size_t)v], in[3 * (size_t)v + 1], in[3 * (size_t)v + 2], 0.0);
 }
+// one component of each record, and grad(3, 5, n) from records whose first 15 doubles are
+// g[5 d + var]
+__global__ void k_component_out(int n, int stride, int k, const double* __restrict__ rec, double* __restrict__ out) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c < n) out[c] = rec[stride * (size_t)c + k];
+}
+__global__ void k_grad_out(int n, int stride, const double* __restrict__ rec, double* __restrict__ out) {
+  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= 15L * n) return;
+  const long c = i / 15;
+  const int e = (int)(i - 15 * c);
+  out[i] = rec[stride * c + 5 * (e % 3) + e / 3];
+}
 __global__ void k_set_scalar(double* p, double v) { *p = v; }
 
 // Per cell-CSR entry (csf = 2p + side): the subface, its face, the node that owns
@@ -829,8 +842,18 @@ void launch_pack6(const DevMesh& m, int n, const double* s5, const double* mass,
 void launch_unpack6(const DevMesh& m, int n, int stride, const double* s6, double* s5) {
   k_unpack6<<<grid_for(n, 256), 256, 0, m.stream>>>(n, stride, s6, s5);
 }
-void launch_vp_out(const DevMesh& m, double* out) { k_vp_out<<<grid_for(m.nv, 256), 256, 0, m.stream>>>(m.nv, m.vp, out); }
-void launch_vp_in(const DevMesh& m, const double* in) { k_vp_in<<<grid_for(m.nv, 256), 256, 0, m.stream>>>(m.nv, in, m.vp); }
+void launch_xyz_out(const DevMesh& m, const double4* a, double* out) {
+  k_vp_out<<<grid_for(m.nv, 256), 256, 0, m.stream>>>(m.nv, a, out);
+}
+void launch_xyz_in(const DevMesh& m, const double* in, double4* a) {
+  k_vp_in<<<grid_for(m.nv, 256), 256, 0, m.stream>>>(m.nv, in, a);
+}
+void launch_component_out(const DevMesh& m, int n, int stride, int k, const double* rec, double* out) {
+  k_component_out<<<grid_for(n, 256), 256, 0, m.stream>>>(n, stride, k, rec, out);
+}
+void launch_grad_out(const DevMesh& m, int n, int stride, const double* rec, double* out) {
+  k_grad_out<<<grid_for(15LL * n, 256), 256, 0, m.stream>>>(n, stride, rec, out);
+}
 void launch_set_scalar(const DevMesh& m, double* p, double v) { k_set_scalar<<<1, 1, 0, m.stream>>>(p, v); }
 void launch_build_cell_entries(const DevMesh& m) {
   k_build_cell_entries<<<grid_for(m.ne, 128), 128, 0, m.stream>>>(m);

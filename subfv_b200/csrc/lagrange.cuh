@@ -17,8 +17,12 @@ void launch_lag_move(const DevMesh& m, const LagScalars* sc, double dt_host);
 void launch_pack6(const DevMesh& m, int n, const double* s5, const double* mass, double* s6);
 // record (stride doubles per cell) -> (5, n) host layout
 void launch_unpack6(const DevMesh& m, int n, int stride, const double* s6, double* s5);
-void launch_vp_out(const DevMesh& m, double* out);
-void launch_vp_in(const DevMesh& m, const double* in);
+// a vertex array (double4) <-> (3, n_vert); one component of n records; grad(3, 5, n) from
+// records that start with g[5 d + var]
+void launch_xyz_out(const DevMesh& m, const double4* a, double* out);
+void launch_xyz_in(const DevMesh& m, const double* in, double4* a);
+void launch_component_out(const DevMesh& m, int n, int stride, int k, const double* rec, double* out);
+void launch_grad_out(const DevMesh& m, int n, int stride, const double* rec, double* out);
 void launch_set_scalar(const DevMesh& m, double* p, double v);
 // fills m.centry (allocated by the caller, all bits set) from the cell CSR
 void launch_build_cell_entries(const DevMesh& m);

@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "handles.cuh"
+#include "lagrange.cuh"
 #include "ns.cuh"
 #include "pool.cuh"
 
@@ -550,11 +551,14 @@ int subfv_ns_batch_get_sol(subfv_ns_batch* b, int slot, double* sol) {
     SUBFV_CUDA(cudaStreamWaitEvent(d.stream, e, 0));
     cudaEventDestroy(e);
   }
-  std::vector<double> rec(kRec * (size_t)d.ne);
-  SUBFV_CUDA(cudaMemcpyAsync(rec.data(), q.U0, rec.size() * sizeof(double), cudaMemcpyDeviceToHost, d.stream));
+  double* t = nullptr;
+  if (pool_alloc((void**)&t, 5 * (size_t)d.ne * sizeof(double), d.stream)) return -1;
+  launch_unpack6(d, d.ne, kRec, q.U0, t);
+  const cudaError_t e = cudaMemcpyAsync(sol, t, 5 * (size_t)d.ne * sizeof(double), cudaMemcpyDeviceToHost, d.stream);
+  cudaFreeAsync(t, d.stream);
+  SUBFV_CUDA(e);
   SUBFV_CUDA(cudaStreamSynchronize(d.stream));
-  for (int c = 0; c < d.ne; ++c)
-    for (int k = 0; k < 5; ++k) sol[5 * (size_t)c + k] = rec[kRec * (size_t)c + k];
+  SUBFV_CUDA(cudaGetLastError());
   return 0;
 }
 

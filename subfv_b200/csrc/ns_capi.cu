@@ -7,6 +7,7 @@
 
 #include "bcsr.cuh"
 #include "handles.cuh"
+#include "lagrange.cuh"
 #include "ns.cuh"
 #include "ns_diffusion.cuh"
 #include "pool.cuh"
@@ -366,11 +367,10 @@ int subfv_ns_advance(subfv_ns_state* s, int n_steps, int* steps_done, double* t)
 
 int subfv_ns_get_sol(subfv_ns_state* s, double* sol) {
   DevMesh& d = s->m->d;
-  std::vector<double> rec(kRec * (size_t)d.ne);
-  SUBFV_CUDA(cudaMemcpyAsync(rec.data(), s->U0, rec.size() * sizeof(double), cudaMemcpyDeviceToHost, d.stream));
+  launch_unpack6(d, d.ne, kRec, s->U0, s->stage);
+  SUBFV_CUDA(cudaMemcpyAsync(sol, s->stage, 5 * (size_t)d.ne * sizeof(double), cudaMemcpyDeviceToHost, d.stream));
   SUBFV_CUDA(cudaStreamSynchronize(d.stream));
-  for (int c = 0; c < d.ne; ++c)
-    for (int k = 0; k < 5; ++k) sol[5 * (size_t)c + k] = rec[kRec * (size_t)c + k];
+  SUBFV_CUDA(cudaGetLastError());
   return 0;
 }
 
@@ -643,6 +643,34 @@ int subfv_ns_be_jacobian(subfv_ns_state* s, double dt, int32_t* row, int32_t* co
   return (int)c->col1.size();
 }
 
+}  // extern "C"
+
+namespace {
+// A residual's outputs in the reference's layouts, converted on the device into one pool
+// buffer and queued for copying on the mesh's stream (vp and cell_grad may be null).
+int outputs_to_host(subfv_ns_state* s, double* rhs, double* sum_lambda, double* vp, double* cell_grad) {
+  DevMesh& d = s->m->d;
+  const size_t ne = d.ne, nv = d.nv;
+  double* t = nullptr;
+  if (pool_alloc((void**)&t, (21 * ne + 3 * nv) * sizeof(double), d.stream)) return -1;
+  double *tl = t + 5 * ne, *tg = tl + ne, *tv = tg + 15 * ne;
+  launch_unpack6(d, d.ne, kRhs, s->rhs1, t);
+  launch_component_out(d, d.ne, kRhs, 5, s->rhs1, tl);
+  if (cell_grad) launch_grad_out(d, d.ne, 15, s->grad, tg);
+  if (vp) launch_xyz_out(d, d.vp, tv);
+  cudaError_t e = cudaMemcpyAsync(rhs, t, 5 * ne * sizeof(double), cudaMemcpyDeviceToHost, d.stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(sum_lambda, tl, ne * sizeof(double), cudaMemcpyDeviceToHost, d.stream);
+  if (e == cudaSuccess && cell_grad)
+    e = cudaMemcpyAsync(cell_grad, tg, 15 * ne * sizeof(double), cudaMemcpyDeviceToHost, d.stream);
+  if (e == cudaSuccess && vp) e = cudaMemcpyAsync(vp, tv, 3 * nv * sizeof(double), cudaMemcpyDeviceToHost, d.stream);
+  cudaFreeAsync(t, d.stream);
+  SUBFV_CUDA(e);
+  return 0;
+}
+}  // namespace
+
+extern "C" {
+
 int subfv_compute_rhs_ns(subfv_mesh* m, const subfv_ns_cfg* cfg, const double* sol, double* rhs, double* sum_lambda,
                          double* vp, double* cell_grad) {
   return subfv_compute_rhs_ns_ex(m, cfg, sol, rhs, sum_lambda, vp, cell_grad, nullptr);
@@ -681,36 +709,16 @@ int subfv_compute_rhs_ns_ex(subfv_mesh* m, const subfv_ns_cfg* cfg, const double
       }
       launch_ns_diffusion_apply(d, s->dterm, s->D.kd, s->rhs1, ddiag);
     }
-    std::vector<double> r(kRhs * (size_t)d.ne);
-    if (cudaMemcpyAsync(r.data(), s->rhs1, r.size() * sizeof(double), cudaMemcpyDeviceToHost, d.stream) !=
-        cudaSuccess) {
+    if (outputs_to_host(s, rhs, sum_lambda, vp, cell_grad)) {
       st = -1;
       break;
     }
-    std::vector<double> g(cell_grad ? 15 * (size_t)d.ne : 0);
-    if (cell_grad) cudaMemcpyAsync(g.data(), s->grad, g.size() * sizeof(double), cudaMemcpyDeviceToHost, d.stream);
-    std::vector<double4> vph(vp ? d.nv : 0);
-    if (vp) cudaMemcpyAsync(vph.data(), d.vp, vph.size() * sizeof(double4), cudaMemcpyDeviceToHost, d.stream);
     if (mat_diag) {  // mat_diag(5, 5, n): the diffusion blocks (zero without diffusion)
       if (ddiag) cudaMemcpyAsync(mat_diag, ddiag, 25 * sizeof(double) * d.ne, cudaMemcpyDeviceToHost, d.stream);
       else std::memset(mat_diag, 0, 25 * sizeof(double) * d.ne);
     }
     if (ddiag) cudaFreeAsync(ddiag, d.stream);
     st = handle_check_status(d);
-    for (int c = 0; c < d.ne; ++c) {
-      for (int k = 0; k < 5; ++k) rhs[5 * (size_t)c + k] = r[kRhs * (size_t)c + k];
-      sum_lambda[c] = r[kRhs * (size_t)c + 5];
-    }
-    if (cell_grad)  // device g[5*d + var] -> Fortran grad(3, 5, n): index d + 3*var
-      for (int c = 0; c < d.ne; ++c)
-        for (int dd = 0; dd < 3; ++dd)
-          for (int k = 0; k < 5; ++k) cell_grad[15 * (size_t)c + dd + 3 * k] = g[15 * (size_t)c + 5 * dd + k];
-    if (vp)
-      for (int v = 0; v < d.nv; ++v) {
-        vp[3 * (size_t)v] = vph[v].x;
-        vp[3 * (size_t)v + 1] = vph[v].y;
-        vp[3 * (size_t)v + 2] = vph[v].z;
-      }
   } while (0);
   subfv_ns_state_destroy(s);
   return st;
@@ -797,21 +805,9 @@ int subfv_compute_euler_flux(subfv_mesh* m, const subfv_ns_cfg* cfg, const doubl
     SUBFV_CUDA(cudaMemcpyAsync(h.s->grad, g.data(), g.size() * sizeof(double), cudaMemcpyHostToDevice, d.stream));
   }
   launch_ns_euler_flux(d, h.s->P, h.s->U0, h.s->grad, h.s->fs, h.s->rhs1, second_order, h.s->sc);
-  std::vector<double> r(kRhs * (size_t)d.ne);
-  SUBFV_CUDA(cudaMemcpyAsync(r.data(), h.s->rhs1, r.size() * sizeof(double), cudaMemcpyDeviceToHost, d.stream));
-  std::vector<double4> vph(vp ? d.nv : 0);
-  if (vp) SUBFV_CUDA(cudaMemcpyAsync(vph.data(), d.vp, vph.size() * sizeof(double4), cudaMemcpyDeviceToHost, d.stream));
+  if (outputs_to_host(h.s, rhs, sum_lambda, vp, nullptr)) return -1;
   const int st = handle_check_status(d);
   SUBFV_CUDA(cudaGetLastError());
-  for (int c = 0; c < d.ne; ++c) {
-    for (int k = 0; k < 5; ++k) rhs[5 * (size_t)c + k] = r[kRhs * (size_t)c + k];
-    sum_lambda[c] = r[kRhs * (size_t)c + 5];
-  }
-  for (int v = 0; vp && v < d.nv; ++v) {
-    vp[3 * (size_t)v] = vph[v].x;
-    vp[3 * (size_t)v + 1] = vph[v].y;
-    vp[3 * (size_t)v + 2] = vph[v].z;
-  }
   return st;
 }
 
