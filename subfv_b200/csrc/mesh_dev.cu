@@ -595,7 +595,26 @@ void launch_cell_geometry_step(const DevMesh& m, double* sol6, const double* rhs
     cudaFuncSetAttribute(k_geom_step_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     k_geom_step_tile<<<grid_for(m.ne, 32), 32 * geo::geo_warps(m.max_pairs), smem, m.stream>>>(m, sol6, rhs6, sc);
   } else {
-    k_geom_step<<<grid_for(m.ne, geo::kGeoBlock), geo::kGeoBlock, 0, m.stream>>>(m, sol6, rhs6, sc);
+    // The kernel is bound by the latency of its gathers, and the cache that shortens them is
+    // what the shared memory leaves: the default split makes room for ten blocks of 22 KB an
+    // SM and leaves L1 next to nothing, 60% makes room for seven. Fewer blocks with the cache
+    // win as soon as the grid needs several waves (2 n^2 cells; default against 60%: n = 222
+    // 58.6 against 49.2 us, 512 229 against 190, 700 406 against 338) and where it needs one
+    // either way (n = 130 25.6 against 22.7, 176 35.1 against 31.7). Between seven and ten
+    // blocks an SM the default's one wave is the shorter (n = 184 37.0 against 41.1, 217 46.0
+    // against 48.8). The split is asked for at the launch, so no other launch sees it.
+    constexpr int kSms = 148;
+    const int grid = grid_for(m.ne, geo::kGeoBlock);
+    cudaLaunchAttribute split{};
+    split.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    split.val.sharedMemCarveout = 60;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(geo::kGeoBlock);
+    cfg.stream = m.stream;
+    cfg.attrs = &split;
+    cfg.numAttrs = grid <= 7 * kSms || grid > 10 * kSms ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, k_geom_step, m, sol6, rhs6, sc);
   }
 }
 void launch_lag_update(const DevMesh& m, double* sol6, const double* rhs6, const LagScalars* sc) {
