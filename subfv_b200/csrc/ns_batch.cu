@@ -16,7 +16,6 @@
 #include <vector>
 
 #include "handles.cuh"
-#include "lagrange.cuh"
 #include "ns.cuh"
 #include "pool.cuh"
 
@@ -551,14 +550,11 @@ int subfv_ns_batch_get_sol(subfv_ns_batch* b, int slot, double* sol) {
     SUBFV_CUDA(cudaStreamWaitEvent(d.stream, e, 0));
     cudaEventDestroy(e);
   }
-  double* t = nullptr;
-  if (pool_alloc((void**)&t, 5 * (size_t)d.ne * sizeof(double), d.stream)) return -1;
-  launch_unpack6(d, d.ne, kRec, q.U0, t);
-  const cudaError_t e = cudaMemcpyAsync(sol, t, 5 * (size_t)d.ne * sizeof(double), cudaMemcpyDeviceToHost, d.stream);
-  cudaFreeAsync(t, d.stream);
-  SUBFV_CUDA(e);
+  std::vector<double> rec(kRec * (size_t)d.ne);
+  SUBFV_CUDA(cudaMemcpyAsync(rec.data(), q.U0, rec.size() * sizeof(double), cudaMemcpyDeviceToHost, d.stream));
   SUBFV_CUDA(cudaStreamSynchronize(d.stream));
-  SUBFV_CUDA(cudaGetLastError());
+  for (int c = 0; c < d.ne; ++c)
+    for (int k = 0; k < 5; ++k) sol[5 * (size_t)c + k] = rec[kRec * (size_t)c + k];
   return 0;
 }
 
