@@ -324,7 +324,10 @@ int subfv_ns_get_sol(subfv_ns_state* s, double* sol);
  * per-vertex sums formed in shared memory (the default on smaller meshes); 8, 16 or 32:
  * a group of at least that many lanes. With a group layout the second-order cell
  * gradient also runs a group of 8 lanes per cell (one per vertex) when no cell has more
- * than 8 vertices. Results are bit-identical in every layout. */
+ * than 8 vertices. The multi_point and two_wave schemes run in tiles of vertices whatever
+ * the layout (unless boundary vertices are excluded or a vertex has more than 32
+ * subfaces): there it is the layout of the gradients alone. Results are bit-identical in
+ * every layout. */
 int subfv_ns_state_set_node_kernel(subfv_ns_state* s, int lanes);
 /* res = sum of |delta|_2 and res_vect(5) of the last add_timedisc_and_solve call */
 int subfv_ns_residuals(subfv_ns_state* s, double* res, double* res_vect, double* dt);

@@ -226,7 +226,10 @@ __device__ inline void state_update(const DevMesh& m, double* sol6, const double
 //   the cell's volume and tests, and the state's update.
 // What bounds it: FP64 issue. One thread per cell ran the 5,500 instructions of a prism as
 // one chain, at 16 warps an SM (180,000 prisms 85 us, 3,000 prisms 20 us).
-// Above kTileCells cells (of a mesh, or of a batch's table) one thread per cell is faster.
+// Above kTileCells cells (of a mesh, or of a batch's table) one thread per cell is as fast
+// or faster (both cell kernels together: tiles 38.7 us at 16,200 prisms, 43.4 at 21,632,
+// 45.3 at 27,848; a thread per cell 44.6 at 28,322, 46.6 at 33,800, and its time hardly
+// falls on smaller meshes).
 constexpr int kTileCells = 28000;
 constexpr int kGeoWarps = 12, kGeoThreads = 32 * kGeoWarps;
 // two pairs a warp; at least the warps that share the vertices and the summed components

@@ -18,8 +18,9 @@
 //   k_ns_nodal_grad  one thread per vertex: least-squares gradient, 3x3 pseudo-inverse
 //   k_ns_cell_grad   one thread per cell: method-4 weighting, physical slope limiter,
 //                    relaxed maximum principle
-//   (on small meshes the node kernel and both gradients run a group of lanes per
-//   vertex or cell instead: k_ns_node_group, k_ns_nodal_grad_group, k_ns_cell_grad_group)
+//   (on small meshes the other schemes' node kernel and both gradients run a group of lanes
+//   per vertex or cell instead: k_ns_node_group, k_ns_nodal_grad_group,
+//   k_ns_cell_grad_group)
 // then per stage k_ns_timedisc (flux limiting blend, diagonal solve, positivity limiter,
 // residual partial sums; its last block to finish runs the stage's scalar tail) and
 // k_ns_apply (batched problems: kb_ns_timedisc, kb_ns_finalize, kb_ns_apply).

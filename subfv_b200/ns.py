@@ -308,8 +308,10 @@ class NsState:
     def set_node_kernel(self, lanes: int):
         """0: one thread per vertex; 1: a group of lanes per vertex (8/16/32 as the mesh
         needs); 8, 16, 32: a group of at least that many lanes. A group layout also runs
-        the cell gradient with 8 lanes per cell (cells of up to 8 vertices). Same results
-        in all."""
+        the cell gradient with 8 lanes per cell (cells of up to 8 vertices). multi_point
+        and two_wave run in tiles of vertices in every layout (meshes of up to 32
+        subfaces a vertex), which then is that of the gradients alone. Same results in
+        all."""
         check(_lib.load().subfv_ns_state_set_node_kernel(self._h, int(lanes)), "subfv_ns_state_set_node_kernel")
 
     def residuals(self):
@@ -434,7 +436,8 @@ class NsBatch:
 
     def set_node_kernel(self, lanes: int):
         """0: one thread per vertex; 1: a group of lanes per vertex (8/16/32 as the mesh
-        needs); 8, 16, 32: a group of at least that many lanes. Same results in all."""
+        needs); 8, 16, 32: a group of at least that many lanes. multi_point and two_wave
+        run in tiles of vertices in every layout. Same results in all."""
         check(_lib.load().subfv_ns_batch_set_node_kernel(self._h, int(lanes)), "subfv_ns_batch_set_node_kernel")
 
     def close(self):
