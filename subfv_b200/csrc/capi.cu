@@ -216,6 +216,7 @@ int subfv_mesh_create(const subfv_mesh_desc* desc, subfv_mesh** out) {
     delete m;
     return rc;
   }
+  m->life->stream = m->d.stream;
   *out = m;
   return 0;
 }
@@ -263,7 +264,18 @@ int subfv_mesh_create_from_topology(const subfv_topology* tp, int b2d, subfv_mes
 
 int subfv_mesh_destroy(subfv_mesh* m) {
   if (!m) return 0;
-  *m->alive = false;
+  {
+    std::lock_guard<std::mutex> lock(m->life->mu);
+    // a state still holds the mesh: it frees its buffers after this event. Without one the
+    // queued work is waited for here.
+    if (m->life->stream && m->life.use_count() > 1 &&
+        (cudaEventCreateWithFlags(&m->life->last, cudaEventDisableTiming) != cudaSuccess ||
+         cudaEventRecord(m->life->last, m->d.stream) != cudaSuccess)) {
+      cudaGetLastError();
+      cudaStreamSynchronize(m->d.stream);
+    }
+    m->life->stream = nullptr;
+  }
   // scratch of the stateless calls (allocated on first use only); a mesh that never
   // needed it is released without any device-wide synchronisation
   void* scratch[] = {m->stage, m->sol6, m->rhs6, m->mass, m->sc};

@@ -1,11 +1,25 @@
 // Opaque handle types of the C-ABI, shared by the translation units that implement it.
 #pragma once
-#include <atomic>
 #include <memory>
+#include <mutex>
 
 #include "../../include/subfv.h"
 #include "common.cuh"
 #include "mesh_dev.cuh"
+
+// What a state keeps of its mesh, so that either may be destroyed first, also from another
+// thread. While the mesh lives, `stream` is its stream. Destroying it clears `stream` and
+// leaves in `last` the end of the work queued by then, which may still write the state's
+// buffers: freed memory of the pool can belong to another state at once, and neither
+// cudaFree nor the stream's destruction waits for that work.
+struct MeshLife {
+  std::mutex mu;
+  cudaStream_t stream = nullptr;
+  cudaEvent_t last = nullptr;
+  ~MeshLife() {
+    if (last) cudaEventDestroy(last);
+  }
+};
 
 // A device mesh plus the scratch buffers the stateless reference-shaped calls need.
 struct subfv_mesh {
@@ -18,8 +32,7 @@ struct subfv_mesh {
   // the backward-Euler Jacobian's host pattern, built on first use and kept with the mesh
   void* imp_pattern = nullptr;
   void (*imp_pattern_free)(void*) = nullptr;
-  // false once the mesh is destroyed: a state that outlives it has no stream to free on
-  std::shared_ptr<std::atomic<bool>> alive = std::make_shared<std::atomic<bool>>(true);
+  std::shared_ptr<MeshLife> life = std::make_shared<MeshLife>();
 };
 
 namespace subfv {

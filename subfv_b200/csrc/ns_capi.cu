@@ -28,7 +28,7 @@ struct ImplicitCtx {
 
 struct subfv_ns_state {
   subfv_mesh* m = nullptr;
-  std::shared_ptr<std::atomic<bool>> mesh_alive;
+  std::shared_ptr<MeshLife> mesh_life;
   char* arena = nullptr;  // one allocation that holds every buffer below
   NsParams P{};
   double *U0 = nullptr, *U1 = nullptr, *fs = nullptr, *rhs1 = nullptr, *rhs2 = nullptr;
@@ -228,7 +228,7 @@ int subfv_ns_state_create(subfv_mesh* m, const subfv_ns_cfg* cfg, const double* 
   // per vertex (one per subface) shortens each vertex's serial chain (Gresho 64x64: 0.39
   // against 0.48 ms per iteration); subfv_ns_state_set_node_kernel overrides it
   if (d.nv < kSmallMeshVertices) s->P.node_group = 1;
-  s->mesh_alive = m->alive;
+  s->mesh_life = m->life;
   const size_t ne = d.ne, nv = d.nv, nse = d.nse;
   Arena mem;
   mem.add(&s->U0, kRec * ne);
@@ -319,11 +319,16 @@ int subfv_ns_state_destroy(subfv_ns_state* s) {
     delete c;
   }
   if (s->graph) cudaGraphExecDestroy(s->graph);
-  if (s->arena) {
-    // after the work queued on the mesh's stream; cudaFree waits for it when the mesh, and
-    // its stream, went first
-    if (*s->mesh_alive) cudaFreeAsync(s->arena, s->m->d.stream);
-    else cudaFree(s->arena);
+  if (s->arena) {  // after the work queued on the mesh's stream
+    MeshLife& life = *s->mesh_life;
+    std::unique_lock<std::mutex> lock(life.mu);
+    if (life.stream) {
+      cudaFreeAsync(s->arena, life.stream);
+    } else {
+      lock.unlock();
+      if (life.last) cudaEventSynchronize(life.last);
+      cudaFree(s->arena);
+    }
   }
   delete s;
   return 0;
