@@ -485,6 +485,11 @@ int subfv_bcsr_gmres_ex(subfv_bcsr* A, double* x, const double* b, double tol, i
 int subfv_bcsr_gmres_refine(subfv_bcsr* A, double* x, const double* b, double rel_tol, int m, int* conv,
                             int* outer, double* rho);
 /* Device time of one SpMV (FP64 or FP32 matrix), averaged over n_iter launches. */
+/* For checks of the solver's Gram-Schmidt kernel on one handle: at most `blocks` blocks
+ * (0: one launch per projection instead, as where the device cannot hold the grid;
+ * negative: as the device has), whose waits give up after `polls` polls (0: the default,
+ * about a second) and make the solve return an error. */
+int subfv_probe_gram_schmidt(subfv_bcsr* h, int blocks, int polls);
 int subfv_bcsr_profile_spmv(subfv_bcsr* A, int n_iter, int fp32, double* ms_per_spmv);
 
 #ifdef __cplusplus

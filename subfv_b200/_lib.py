@@ -131,6 +131,7 @@ SIGNATURES = {
     "subfv_bcsr_gmres": (c_int, [P, PD, PD, c_dbl, c_int, C.POINTER(c_int), C.POINTER(c_int), PD]),
     "subfv_bcsr_gmres_ex": (c_int, [P, PD, PD, c_dbl, c_int, c_int, C.POINTER(c_int), C.POINTER(c_int), PD, PD]),
     "subfv_bcsr_gmres_refine": (c_int, [P, PD, PD, c_dbl, c_int, C.POINTER(c_int), C.POINTER(c_int), PD]),
+    "subfv_probe_gram_schmidt": (c_int, [P, c_int, c_int]),
     "subfv_bcsr_profile_spmv": (c_int, [P, c_int, c_int, PD]),
     "subfv_mesh_stream": (P, [P]),
 }

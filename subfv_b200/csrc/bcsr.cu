@@ -399,7 +399,6 @@ __global__ void __launch_bounds__(kRedThreads) k_normalize(const double* src, do
 constexpr unsigned long long kNoPartial = ~0ull;
 constexpr int kMgsThreads = 1024;
 constexpr int kMgsSharedMax = 27;       // 216 KB of the SM's shared memory
-constexpr int kMgsSpin = 2000000;       // polls of an L2 word: about a second
 constexpr int kMgsLaneSlots = 5;        // block 0's lanes read the partials of up to 160 blocks
 constexpr int kMgsStride = 32 * kMgsLaneSlots + 16;  // a sum's words: the partials, then the total on a line of its own
 
@@ -408,7 +407,7 @@ __device__ inline unsigned long long mgs_word(double v) {  // never the mark: an
   return bits == kNoPartial ? 0x7ff8000000000000ull : bits;
 }
 
-__device__ inline double mgs_sum(double s, unsigned long long* slots, unsigned* fail, bool* ok) {
+__device__ inline double mgs_sum(double s, unsigned long long* slots, const int polls, unsigned* fail, bool* ok) {
   __shared__ double part[32];
   __shared__ unsigned long long total;
   volatile unsigned long long* all = slots;
@@ -420,10 +419,10 @@ __device__ inline double mgs_sum(double s, unsigned long long* slots, unsigned* 
     const double v = warp_tree(part[threadIdx.x]);
     if (blockIdx.x == 0) {
       // all of a lane's slots in flight at once, until each holds a value
-      unsigned long long bits[kMgsLaneSlots];
+      unsigned long long bits[kMgsLaneSlots] = {};
       const unsigned long long own = __shfl_sync(0xffffffffu, mgs_word(v), 0);
       bool late = true;
-      for (int spin = 0; spin < kMgsSpin && late; ++spin) {
+      for (int spin = 0; spin < polls && late; ++spin) {
 #pragma unroll
         for (int u = 0; u < kMgsLaneSlots; ++u) {
           const int q = threadIdx.x + 32 * u;
@@ -445,7 +444,7 @@ __device__ inline double mgs_sum(double s, unsigned long long* slots, unsigned* 
     } else if (threadIdx.x == 0) {
       all[blockIdx.x] = mgs_word(v);
       unsigned long long t = kNoPartial;
-      for (int spin = 0; spin < kMgsSpin && t == kNoPartial; ++spin) t = *sum;
+      for (int spin = 0; spin < polls && t == kNoPartial; ++spin) t = *sum;
       total = t;
     }
     if (threadIdx.x == 0 && total == kNoPartial) *fail = 1u;
@@ -459,7 +458,8 @@ __device__ inline double mgs_sum(double s, unsigned long long* slots, unsigned* 
 
 template <int E, bool KEEP>
 __global__ void __launch_bounds__(kMgsThreads, 1) k_mgs_column(double* V, long n, int jj, double* __restrict__ hcol,
-                                                               unsigned long long* slots, int nes, unsigned* fail) {
+                                                               unsigned long long* slots, int nes, int polls,
+                                                               unsigned* fail) {
   extern __shared__ double ws[];  // [nes][kMgsThreads]
   const long T = (long)gridDim.x * kMgsThreads, k0 = (long)blockIdx.x * kMgsThreads + threadIdx.x;
   double* wv = V + (size_t)(jj - 1) * n;
@@ -486,7 +486,7 @@ __global__ void __launch_bounds__(kMgsThreads, 1) k_mgs_column(double* V, long n
       if (k < n) s = s + x * V[k];
     }
   }
-  double h = mgs_sum(s, slots, fail, &ok);
+  double h = mgs_sum(s, slots, polls, fail, &ok);
   for (int i = 1; i <= jj - 1; ++i) {
     if (!ok) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) hcol[i - 1] = h;
@@ -524,7 +524,7 @@ __global__ void __launch_bounds__(kMgsThreads, 1) k_mgs_column(double* V, long n
         }
       }
     }
-    h = mgs_sum(s, slots + (size_t)i * kMgsStride, fail, &ok);
+    h = mgs_sum(s, slots + (size_t)i * kMgsStride, polls, fail, &ok);
   }
   if (!ok) return;
   const double nrm = sqrt(h);
@@ -633,9 +633,57 @@ void bcsr_free(DevBcsr* A) {
 namespace {
 // projections and norms of a cycle: jj sums in column jj = 2 .. krylov + 1
 size_t mgs_slots(int krylov) { return (size_t)krylov * (krylov + 3) / 2; }
+
+// a block's dynamic shared memory: the elements beyond the E in registers
+template <int E, bool KEEP>
+size_t mgs_smem(const GmresWork& W) {
+  const int nes = W.mgs_per > E ? W.mgs_per - E : 0;
+  if (nes) cudaFuncSetAttribute(k_mgs_column<E, KEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                kMgsSharedMax * kMgsThreads * (int)sizeof(double));
+  return (size_t)nes * kMgsThreads * sizeof(double);
+}
+template <int E, bool KEEP>
+bool mgs_resident_e(const GmresWork& W) {
+  int per_sm = 0;
+  const bool ok = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mgs_column<E, KEEP>, kMgsThreads,
+                                                                mgs_smem<E, KEEP>(W)) == cudaSuccess;
+  if (!ok) cudaGetLastError();
+  return ok && per_sm >= 1;
+}
+bool mgs_resident(const GmresWork& W) {
+  return W.mgs_per <= 1 ? mgs_resident_e<1, true>(W) : W.mgs_per <= 2 ? mgs_resident_e<2, true>(W)
+       : W.mgs_per <= 4 ? mgs_resident_e<4, true>(W) : W.mgs_per <= 8 ? mgs_resident_e<8, true>(W)
+                                                                      : mgs_resident_e<16, false>(W);
+}
+
+// k_mgs_column's grid: one block per SM, at most `most` (negative: no limit), where all of
+// them can be resident and hold the vector. mgs_per stays 0 where they cannot, or where its
+// slots find no room, and one launch per projection serves.
+int mgs_plan(GmresWork* W, int most, int polls) {
+  int dev = 0, sms = 0, coop = 0;
+  SUBFV_CUDA(cudaGetDevice(&dev));
+  SUBFV_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  SUBFV_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+  W->mgs_per = 0;
+  W->mgs_polls = polls;
+  sms = coop ? std::min(sms, 32 * kMgsLaneSlots) : 0;
+  if (most >= 0) sms = std::min(sms, most);
+  W->mgs_blocks = (int)std::min<long>(sms, (W->n + kMgsThreads - 1) / kMgsThreads);
+  if (W->mgs_blocks < 1) return 0;
+  const long T = (long)W->mgs_blocks * kMgsThreads, per = (W->n + T - 1) / T;
+  if (per > 16 + kMgsSharedMax) return 0;
+  W->mgs_per = (int)per;
+  if (!mgs_resident(*W) ||
+      cudaMalloc(&W->slots, mgs_slots(W->krylov) * kMgsStride * sizeof(unsigned long long)) != cudaSuccess) {
+    cudaGetLastError();
+    W->slots = nullptr;
+    W->mgs_per = 0;
+  }
+  return 0;
+}
 }  // namespace
 
-int gmres_work_alloc(GmresWork* W, long n, int krylov) {
+int gmres_work_alloc(GmresWork* W, long n, int krylov, int mgs_most, int mgs_polls) {
   W->n = n;
   W->krylov = krylov;
   SUBFV_CUDA(cudaMalloc(&W->V, (size_t)n * (krylov + 1) * sizeof(double)));
@@ -648,14 +696,8 @@ int gmres_work_alloc(GmresWork* W, long n, int krylov) {
   SUBFV_CUDA(cudaMalloc(&W->z, (krylov + 2) * sizeof(double)));
   SUBFV_CUDA(cudaMalloc(&W->partial, 2 * kRedBlocks * sizeof(double)));
   SUBFV_CUDA(cudaMalloc(&W->H, ((size_t)(krylov + 1) * krylov + 1) * sizeof(double)));  // and the fail word
-  int dev = 0, sms = 0;
-  SUBFV_CUDA(cudaGetDevice(&dev));
-  SUBFV_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  W->mgs_blocks = (int)std::min<long>(std::min(sms, 32 * kMgsLaneSlots), (n + kMgsThreads - 1) / kMgsThreads);
-  const long per = (n + (long)W->mgs_blocks * kMgsThreads - 1) / ((long)W->mgs_blocks * kMgsThreads);
-  W->mgs_per = per <= 16 + kMgsSharedMax ? (int)per : 0;
-  if (W->mgs_per) SUBFV_CUDA(cudaMalloc(&W->slots, mgs_slots(krylov) * kMgsStride * sizeof(unsigned long long)));
   SUBFV_CUDA(cudaMalloc(&W->scal, 8 * sizeof(double)));
+  if (mgs_plan(W, mgs_most, mgs_polls)) return -1;
   W->bytes = (size_t)n * (krylov + 7) * 8;
   return 0;
 }
@@ -797,10 +839,8 @@ int bcsr_set_colors(DevBcsr* A, int ncs, const int* color) {
 namespace {
 template <int E, bool KEEP>
 cudaError_t launch_mgs_e(GmresWork& W, int jj, double* hcol, unsigned long long* slots, unsigned* fail, cudaStream_t s) {
-  const int nes = W.mgs_per > E ? W.mgs_per - E : 0;
-  const size_t smem = (size_t)nes * kMgsThreads * sizeof(double);
-  if (smem) cudaFuncSetAttribute(k_mgs_column<E, KEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kMgsSharedMax * kMgsThreads * (int)sizeof(double));
+  const size_t smem = mgs_smem<E, KEEP>(W);
+  const int nes = (int)(smem / (kMgsThreads * sizeof(double)));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(W.mgs_blocks);
   cfg.blockDim = dim3(kMgsThreads);
@@ -811,7 +851,7 @@ cudaError_t launch_mgs_e(GmresWork& W, int jj, double* hcol, unsigned long long*
   a.val.cooperative = 1;
   cfg.attrs = &a;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_mgs_column<E, KEEP>, W.V, W.n, jj, hcol, slots, nes, fail);
+  return cudaLaunchKernelEx(&cfg, k_mgs_column<E, KEEP>, W.V, W.n, jj, hcol, slots, nes, W.mgs_polls, fail);
 }
 // the fewest registers that hold a thread's elements (and its basis vector elements up to 8)
 cudaError_t launch_mgs(GmresWork& W, int jj, double* hcol, unsigned long long* slots, unsigned* fail, cudaStream_t s) {
@@ -873,19 +913,28 @@ int run_arnoldi_cycle(const DevBcsr& A, GmresWork& W, int precond, bool fp32) {
     cudaGraphExecDestroy(W.cycle);
     W.cycle = nullptr;
   }
+  cudaError_t e = cudaSuccess;
   if (!W.cycle) {
     cudaGraph_t g = nullptr;
     SUBFV_CUDA(cudaStreamBeginCapture(A.stream, cudaStreamCaptureModeThreadLocal));
-    const cudaError_t le = arnoldi_cycle(A, W, precond, fp32);
+    e = arnoldi_cycle(A, W, precond, fp32);
     const cudaError_t ce = cudaStreamEndCapture(A.stream, &g);
-    SUBFV_CUDA(le);
-    SUBFV_CUDA(ce);
-    const cudaError_t ie = cudaGraphInstantiate(&W.cycle, g, 0);
-    cudaGraphDestroy(g);
-    SUBFV_CUDA(ie);
+    if (e == cudaSuccess) e = ce;
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&W.cycle, g, 0);
+    if (g) cudaGraphDestroy(g);
+    if (e != cudaSuccess) W.cycle = nullptr;
     std::memcpy(W.cycle_key, key, sizeof(key));
   }
-  SUBFV_CUDA(cudaGraphLaunch(W.cycle, A.stream));
+  if (e == cudaSuccess) e = cudaGraphLaunch(W.cycle, A.stream);
+  if (W.mgs_per && (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported)) {
+    // a process limited to part of the SMs: its grid cannot be resident after all
+    cudaGetLastError();
+    if (W.cycle) cudaGraphExecDestroy(W.cycle);
+    W.cycle = nullptr;
+    W.mgs_per = 0;
+    return run_arnoldi_cycle(A, W, precond, fp32);
+  }
+  SUBFV_CUDA(e);
   return 0;
 }
 }  // namespace

@@ -47,9 +47,9 @@ struct GmresWork {
   double *partial = nullptr, *H = nullptr, *scal = nullptr;
   double *d = nullptr, *rr = nullptr;  // refinement correction and residual
   double* ty = nullptr;                 // the LU-SGS forward sweep
-  // k_mgs_column: its blocks, the elements a thread holds (0: the vector does not fit), and
-  // the blocks' partial sums of a cycle
-  int mgs_blocks = 0, mgs_per = 0;
+  // k_mgs_column: its blocks, the elements a thread holds (0: one launch per projection
+  // instead), the polls of a wait before it gives up, and the blocks' partial sums of a cycle
+  int mgs_blocks = 0, mgs_per = 0, mgs_polls = 0;
   unsigned long long* slots = nullptr;
   size_t bytes = 0;
   cudaGraphExec_t cycle = nullptr;  // the captured Arnoldi cycle and what it was captured for
@@ -59,7 +59,9 @@ struct GmresWork {
 int bcsr_upload(DevBcsr* A, int m, int bs, const int* row1, const int* col1, const double* v, cudaStream_t s);
 int bcsr_set_values(DevBcsr* A, const double* v_dev_or_host, bool on_device);
 void bcsr_free(DevBcsr* A);
-int gmres_work_alloc(GmresWork* W, long n, int krylov);
+constexpr int kMgsPolls = 2000000;  // of an L2 word: about a second
+// mgs_most: at most that many blocks for k_mgs_column (0: none, negative: as the device has)
+int gmres_work_alloc(GmresWork* W, long n, int krylov, int mgs_most = -1, int mgs_polls = kMgsPolls);
 void gmres_work_free(GmresWork* W);
 
 void launch_bcsr_spmv(const DevBcsr& A, const double* x, double* y, bool fp32_matrix);

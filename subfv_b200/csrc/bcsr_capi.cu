@@ -11,6 +11,7 @@ struct subfv_bcsr {
   DevBcsr A;
   GmresWork W;
   double *x = nullptr, *b = nullptr, *y = nullptr;
+  int mgs_most = -1, mgs_polls = kMgsPolls;
 };
 
 namespace {
@@ -25,7 +26,9 @@ int ensure_vecs(subfv_bcsr* h) {
 int ensure_work(subfv_bcsr* h, int krylov) {
   if (h->W.V && h->W.krylov == krylov) return 0;
   gmres_work_free(&h->W);
-  return gmres_work_alloc(&h->W, (long)h->A.m * h->A.bs, krylov);
+  const int rc = gmres_work_alloc(&h->W, (long)h->A.m * h->A.bs, krylov, h->mgs_most, h->mgs_polls);
+  if (rc) gmres_work_free(&h->W);  // what there was room for: the next call starts afresh
+  return rc;
 }
 }  // namespace
 
@@ -176,6 +179,18 @@ int subfv_bcsr_gmres_refine(subfv_bcsr* h, double* x, const double* b, double re
   if (outer) *outer = st.outer;
   if (rho) *rho = st.rho;
   return st.conv ? 0 : SUBFV_ERR_GMRES;
+}
+
+int subfv_probe_gram_schmidt(subfv_bcsr* h, int blocks, int polls) {
+  if (!h || polls < 0) {
+    set_error("subfv_probe_gram_schmidt: bad argument");
+    return -2;
+  }
+  SUBFV_CUDA(cudaStreamSynchronize(h->A.stream));
+  h->mgs_most = blocks;
+  h->mgs_polls = polls > 0 ? polls : kMgsPolls;
+  gmres_work_free(&h->W);
+  return 0;
 }
 
 int subfv_bcsr_profile_spmv(subfv_bcsr* h, int n_iter, int fp32, double* ms_per_spmv) {
