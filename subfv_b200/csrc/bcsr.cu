@@ -969,7 +969,9 @@ int gmres_device(const DevBcsr& A, GmresWork& W, double* x, const double* b, dou
     SUBFV_CUDA(cudaMemcpyAsync(H.data(), W.H, H.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
     SUBFV_CUDA(cudaStreamSynchronize(s));
     SUBFV_CUDA(cudaGetLastError());
-    if (H.back() != 0.0) {
+    uint64_t fail = 0;  // the word's bits: as a double 1 is a subnormal, which a caller may flush to zero
+    std::memcpy(&fail, &H.back(), sizeof(fail));
+    if (fail) {
       set_error("gmres: a block of the Gram-Schmidt kernel waited too long for the others");
       return -1;
     }

@@ -47,3 +47,22 @@ def test_gram_schmidt_with_fewer_blocks(native, cuda_ok, blocks, n):
         np.testing.assert_allclose(H.T, _arnoldi(mul, b, m), rtol=0, atol=4 * 1e-11)
     else:
         np.testing.assert_allclose(H[0, 0], mul(np.ones(n))[0], rtol=1e-14)
+
+
+@pytest.mark.parametrize("flush", [False, True])
+def test_wait_that_runs_out_is_an_error(native, cuda_ok, flush):
+    """Blocks that give up after one poll (an answer takes several times as long) make the
+    solve return an error, also in a process that flushes subnormals to zero; the next solve
+    on the handle is sound."""
+    import torch
+    A, mul, b = _tridiagonal(5000)
+    _limit(A, -1, polls=1)
+    assert torch.set_flush_denormal(flush)
+    try:
+        with pytest.raises(RuntimeError, match="waited too long"):
+            A.gmres(b, 1e-300, 5, precond=False)
+    finally:
+        torch.set_flush_denormal(False)
+    _limit(A, -1)
+    *_, H = A.gmres(b, 1e-300, 5, precond=False, want_h=True)
+    np.testing.assert_allclose(H.T, _arnoldi(mul, b, 5), rtol=0, atol=4 * 1e-11)
