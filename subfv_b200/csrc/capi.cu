@@ -123,7 +123,7 @@ int xyz_to_host(DevMesh& d, const double4* a, double* out) {
   if (pool_alloc((void**)&t, 3 * (size_t)d.nv * sizeof(double), d.stream)) return -1;
   launch_xyz_out(d, a, t);
   const cudaError_t e = cudaMemcpyAsync(out, t, 3 * (size_t)d.nv * sizeof(double), cudaMemcpyDeviceToHost, d.stream);
-  cudaFreeAsync(t, d.stream);
+  pool_free(t, d.stream);
   SUBFV_CUDA(e);
   return 0;
 }
@@ -132,7 +132,7 @@ int xyz_from_host(DevMesh& d, const double* in, double4* a) {
   if (pool_alloc((void**)&t, 3 * (size_t)d.nv * sizeof(double), d.stream)) return -1;
   const cudaError_t e = cudaMemcpyAsync(t, in, 3 * (size_t)d.nv * sizeof(double), cudaMemcpyHostToDevice, d.stream);
   if (e == cudaSuccess) launch_xyz_in(d, t, a);
-  cudaFreeAsync(t, d.stream);
+  pool_free(t, d.stream);
   SUBFV_CUDA(e);
   return 0;
 }

@@ -82,8 +82,8 @@ struct subfv_lag_batch {
 namespace {
 
 void slot_free_state(Slot& q, cudaStream_t s) {
-  if (q.sol6) cudaFreeAsync(q.sol6, s);
-  if (q.rhs6) cudaFreeAsync(q.rhs6, s);
+  pool_free(q.sol6, s);
+  pool_free(q.rhs6, s);
   q.sol6 = q.rhs6 = nullptr;
 }
 
@@ -313,6 +313,7 @@ int subfv_lag_batch_add(subfv_lag_batch* b, subfv_mesh* m, int take_mesh, const 
       pool_alloc((void**)&stage, 5 * ne * sizeof(double), s) ||
       pool_alloc((void**)&mstage, ne * sizeof(double), s)) {
     slot_free_state(q, s);
+    pool_free(stage, s);
     set_error("subfv_lag_batch_add: device allocation failed");
     return -1;
   }
@@ -329,8 +330,8 @@ int subfv_lag_batch_add(subfv_lag_batch* b, subfv_mesh* m, int take_mesh, const 
   SUBFV_CUDA(cudaMemcpyAsync(b->sc + k, &h, sizeof(h), cudaMemcpyHostToDevice, s));
   SUBFV_CUDA(cudaMemcpyAsync(b->status + k, &zero, sizeof(zero), cudaMemcpyHostToDevice, s));
   launch_pack6(d, (int)ne, stage, mstage, q.sol6);
-  SUBFV_CUDA(cudaFreeAsync(stage, s));
-  SUBFV_CUDA(cudaFreeAsync(mstage, s));
+  pool_free(stage, s);
+  pool_free(mstage, s);
   cudaEvent_t ready;
   SUBFV_CUDA(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
   SUBFV_CUDA(cudaEventRecord(ready, s));
@@ -486,7 +487,7 @@ int subfv_lag_batch_get_sol(subfv_lag_batch* b, int slot, double* sol) {
   if (pool_alloc((void**)&t, 5 * (size_t)d.ne * sizeof(double), d.stream)) return -1;
   launch_unpack6(d, d.ne, kRec, q.sol6, t);
   const cudaError_t e = cudaMemcpyAsync(sol, t, 5 * (size_t)d.ne * sizeof(double), cudaMemcpyDeviceToHost, d.stream);
-  cudaFreeAsync(t, d.stream);
+  pool_free(t, d.stream);
   SUBFV_CUDA(e);
   SUBFV_CUDA(cudaStreamSynchronize(d.stream));
   SUBFV_CUDA(cudaGetLastError());

@@ -96,8 +96,7 @@ int dalloc_async(T** p, size_t n, cudaStream_t s) {
 
 void slot_free_state(Slot& q, cudaStream_t s) {
   double* bufs[] = {q.U0, q.U1, q.fs, q.rhs1, q.rhs2, q.ngrad, q.grad, q.delta, q.partial};
-  for (double* b : bufs)
-    if (b) cudaFreeAsync(b, s);
+  for (double* b : bufs) pool_free(b, s);
   q.U0 = q.U1 = q.fs = q.rhs1 = q.rhs2 = q.ngrad = q.grad = q.delta = q.partial = nullptr;
 }
 
@@ -379,7 +378,7 @@ int subfv_ns_batch_add(subfv_ns_batch* b, subfv_mesh* m, int take_mesh, const do
   SUBFV_CUDA(cudaMemcpyAsync(b->sc + k, &h, sizeof(h), cudaMemcpyHostToDevice, s));
   SUBFV_CUDA(cudaMemcpyAsync(b->status + k, &zero, sizeof(zero), cudaMemcpyHostToDevice, s));
   launch_ns_pack(d, stage, q.U0);
-  SUBFV_CUDA(cudaFreeAsync(stage, s));
+  pool_free(stage, s);
   cudaEvent_t ready;
   SUBFV_CUDA(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
   SUBFV_CUDA(cudaEventRecord(ready, s));

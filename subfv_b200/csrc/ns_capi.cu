@@ -323,11 +323,11 @@ int subfv_ns_state_destroy(subfv_ns_state* s) {
     MeshLife& life = *s->mesh_life;
     std::unique_lock<std::mutex> lock(life.mu);
     if (life.stream) {
-      cudaFreeAsync(s->arena, life.stream);
+      pool_free(s->arena, life.stream);
     } else {
       lock.unlock();
       if (life.last) cudaEventSynchronize(life.last);
-      cudaFree(s->arena);
+      pool_free_idle(s->arena);
     }
   }
   delete s;
@@ -668,7 +668,7 @@ int outputs_to_host(subfv_ns_state* s, double* rhs, double* sum_lambda, double* 
   if (e == cudaSuccess && cell_grad)
     e = cudaMemcpyAsync(cell_grad, tg, 15 * ne * sizeof(double), cudaMemcpyDeviceToHost, d.stream);
   if (e == cudaSuccess && vp) e = cudaMemcpyAsync(vp, tv, 3 * nv * sizeof(double), cudaMemcpyDeviceToHost, d.stream);
-  cudaFreeAsync(t, d.stream);
+  pool_free(t, d.stream);
   SUBFV_CUDA(e);
   return 0;
 }

@@ -8,7 +8,13 @@
 // synchronisations, and leaves the ordering between streams and threads to the runtime.
 // A residual of 480 cells through compute_rhs_ns took 0.9 ms and more of which 0.1 ms on
 // the device.
+//
+// The runtime's release threshold counts what the pool holds, memory in use included. So it
+// follows the bytes in use, in steps of kStep: at a fixed threshold a program whose states
+// pass it would keep nothing, and map and unmap memory with each state and each read-back
+// through a staging buffer (1-3 ms a problem).
 #include <mutex>
+#include <unordered_map>
 
 #include "common.cuh"
 #include "pool.cuh"
@@ -17,11 +23,52 @@ namespace subfv {
 
 namespace {
 constexpr int kMaxDevices = 64;
-constexpr unsigned long long kKept = 512ull << 20;
-std::mutex g_pool_mutex;
-cudaMemPool_t g_pool[kMaxDevices] = {};
+constexpr unsigned long long kKept = 512ull << 20, kStep = 64ull << 20;
 
-int device_pool(cudaMemPool_t* out) {
+struct Pool {
+  cudaMemPool_t pool = nullptr;
+  unsigned long long used = 0, threshold = 0;
+};
+struct Block {
+  int dev;
+  size_t bytes;
+};
+std::mutex g_pool_mutex;
+Pool g_pool[kMaxDevices];
+std::unordered_map<void*, Block> g_blocks;  // the allocations in use
+
+// the bytes in use rounded up, and kKept more
+void follow_use(Pool& p) {
+  unsigned long long keep = (p.used + kStep - 1) / kStep * kStep + kKept;
+  if (keep == p.threshold) return;
+  p.threshold = keep;
+  cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+}
+
+int device_pool(int dev) {
+  Pool& p = g_pool[dev];
+  if (p.pool) return 0;
+  cudaMemPoolProps props{};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  SUBFV_CUDA(cudaMemPoolCreate(&p.pool, &props));
+  return 0;
+}
+
+// the block leaves the books (before it is freed: afterwards its address may be another's)
+void forget(void* ptr) {
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  auto it = g_blocks.find(ptr);
+  if (it == g_blocks.end()) return;
+  Pool& p = g_pool[it->second.dev];
+  p.used -= it->second.bytes;
+  g_blocks.erase(it);
+  follow_use(p);
+}
+}  // namespace
+
+int pool_alloc(void** ptr, size_t bytes, cudaStream_t s) {
   int dev = 0;
   SUBFV_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= kMaxDevices) {
@@ -29,27 +76,25 @@ int device_pool(cudaMemPool_t* out) {
     return -1;
   }
   std::lock_guard<std::mutex> lock(g_pool_mutex);
-  if (!g_pool[dev]) {
-    cudaMemPoolProps props{};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = dev;
-    cudaMemPool_t p = nullptr;
-    SUBFV_CUDA(cudaMemPoolCreate(&p, &props));
-    unsigned long long kept = kKept;
-    SUBFV_CUDA(cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &kept));
-    g_pool[dev] = p;
-  }
-  *out = g_pool[dev];
+  if (device_pool(dev)) return -1;
+  Pool& p = g_pool[dev];
+  SUBFV_CUDA(cudaMallocFromPoolAsync(ptr, bytes, p.pool, s));
+  g_blocks[*ptr] = {dev, bytes};
+  p.used += bytes;
+  follow_use(p);
   return 0;
 }
-}  // namespace
 
-int pool_alloc(void** p, size_t bytes, cudaStream_t s) {
-  cudaMemPool_t pool = nullptr;
-  if (device_pool(&pool)) return -1;
-  SUBFV_CUDA(cudaMallocFromPoolAsync(p, bytes, pool, s));
-  return 0;
+void pool_free(void* ptr, cudaStream_t s) {
+  if (!ptr) return;
+  forget(ptr);
+  cudaFreeAsync(ptr, s);
+}
+
+void pool_free_idle(void* ptr) {
+  if (!ptr) return;
+  forget(ptr);
+  cudaFree(ptr);
 }
 
 }  // namespace subfv

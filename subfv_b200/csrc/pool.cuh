@@ -6,7 +6,10 @@
 
 namespace subfv {
 
-// *p: `bytes` of device memory usable on s from here on; released with cudaFreeAsync
-int pool_alloc(void** p, size_t bytes, cudaStream_t s);
+// *ptr: `bytes` of the current device's memory, usable on s from here on
+int pool_alloc(void** ptr, size_t bytes, cudaStream_t s);
+// gives it back after the work queued on s, or (idle) when no work uses it any more
+void pool_free(void* ptr, cudaStream_t s);
+void pool_free_idle(void* ptr);
 
 }  // namespace subfv
