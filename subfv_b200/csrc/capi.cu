@@ -117,10 +117,17 @@ int ensure_full_geometry(DevMesh& d) {
   d.geom_partial = 0;
   return 0;
 }
-// a vertex array to or from the host's (3, n_vert), converted on the device
+// A vertex array to or from the host's (3, n_vert), converted on the device. Without room for
+// the staging buffer the copy itself takes three of each vertex's four doubles: slow, row
+// by row, but without device memory (the fourth double of a position is always 0).
 int xyz_to_host(DevMesh& d, const double4* a, double* out) {
   double* t = nullptr;
-  if (pool_alloc((void**)&t, 3 * (size_t)d.nv * sizeof(double), d.stream)) return -1;
+  if (pool_alloc((void**)&t, 3 * (size_t)d.nv * sizeof(double), d.stream)) {
+    cudaGetLastError();
+    SUBFV_CUDA(cudaMemcpy2DAsync(out, 3 * sizeof(double), a, sizeof(double4), 3 * sizeof(double), d.nv,
+                                 cudaMemcpyDeviceToHost, d.stream));
+    return 0;
+  }
   launch_xyz_out(d, a, t);
   const cudaError_t e = cudaMemcpyAsync(out, t, 3 * (size_t)d.nv * sizeof(double), cudaMemcpyDeviceToHost, d.stream);
   pool_free(t, d.stream);
@@ -129,7 +136,12 @@ int xyz_to_host(DevMesh& d, const double4* a, double* out) {
 }
 int xyz_from_host(DevMesh& d, const double* in, double4* a) {
   double* t = nullptr;
-  if (pool_alloc((void**)&t, 3 * (size_t)d.nv * sizeof(double), d.stream)) return -1;
+  if (pool_alloc((void**)&t, 3 * (size_t)d.nv * sizeof(double), d.stream)) {
+    cudaGetLastError();
+    SUBFV_CUDA(cudaMemcpy2DAsync(a, sizeof(double4), in, 3 * sizeof(double), 3 * sizeof(double), d.nv,
+                                 cudaMemcpyHostToDevice, d.stream));
+    return 0;
+  }
   const cudaError_t e = cudaMemcpyAsync(t, in, 3 * (size_t)d.nv * sizeof(double), cudaMemcpyHostToDevice, d.stream);
   if (e == cudaSuccess) launch_xyz_in(d, t, a);
   pool_free(t, d.stream);

@@ -484,11 +484,16 @@ int subfv_lag_batch_get_sol(subfv_lag_batch* b, int slot, double* sol) {
     cudaEventDestroy(e);
   }
   double* t = nullptr;
-  if (pool_alloc((void**)&t, 5 * (size_t)d.ne * sizeof(double), d.stream)) return -1;
-  launch_unpack6(d, d.ne, kRec, q.sol6, t);
-  const cudaError_t e = cudaMemcpyAsync(sol, t, 5 * (size_t)d.ne * sizeof(double), cudaMemcpyDeviceToHost, d.stream);
-  pool_free(t, d.stream);
-  SUBFV_CUDA(e);
+  if (pool_alloc((void**)&t, 5 * (size_t)d.ne * sizeof(double), d.stream)) {
+    cudaGetLastError();  // no room for the staging buffer: the copy takes five doubles of each record
+    SUBFV_CUDA(cudaMemcpy2DAsync(sol, 5 * sizeof(double), q.sol6, kRec * sizeof(double), 5 * sizeof(double), d.ne,
+                                 cudaMemcpyDeviceToHost, d.stream));
+  } else {
+    launch_unpack6(d, d.ne, kRec, q.sol6, t);
+    const cudaError_t e = cudaMemcpyAsync(sol, t, 5 * (size_t)d.ne * sizeof(double), cudaMemcpyDeviceToHost, d.stream);
+    pool_free(t, d.stream);
+    SUBFV_CUDA(e);
+  }
   SUBFV_CUDA(cudaStreamSynchronize(d.stream));
   SUBFV_CUDA(cudaGetLastError());
   return 0;

@@ -651,14 +651,14 @@ int subfv_ns_be_jacobian(subfv_ns_state* s, double dt, int32_t* row, int32_t* co
 }  // extern "C"
 
 namespace {
-// A residual's outputs in the reference's layouts, converted on the device into one pool
-// buffer and queued for copying on the mesh's stream (vp and cell_grad may be null).
+// A residual's outputs in the reference's layouts, converted on the device and queued for
+// copying on the mesh's stream (vp and cell_grad may be null). They are staged in the state's
+// buffers that the residual leaves behind: the corner sums hold the gradients (15 doubles a
+// cell in 6 for each of its four subcells and more), the vertex records the velocities.
 int outputs_to_host(subfv_ns_state* s, double* rhs, double* sum_lambda, double* vp, double* cell_grad) {
   DevMesh& d = s->m->d;
   const size_t ne = d.ne, nv = d.nv;
-  double* t = nullptr;
-  if (pool_alloc((void**)&t, (21 * ne + 3 * nv) * sizeof(double), d.stream)) return -1;
-  double *tl = t + 5 * ne, *tg = tl + ne, *tv = tg + 15 * ne;
+  double *t = s->stage, *tl = s->delta, *tg = s->fs, *tv = s->ngrad;
   launch_unpack6(d, d.ne, kRhs, s->rhs1, t);
   launch_component_out(d, d.ne, kRhs, 5, s->rhs1, tl);
   if (cell_grad) launch_grad_out(d, d.ne, 15, s->grad, tg);
@@ -668,7 +668,6 @@ int outputs_to_host(subfv_ns_state* s, double* rhs, double* sum_lambda, double* 
   if (e == cudaSuccess && cell_grad)
     e = cudaMemcpyAsync(cell_grad, tg, 15 * ne * sizeof(double), cudaMemcpyDeviceToHost, d.stream);
   if (e == cudaSuccess && vp) e = cudaMemcpyAsync(vp, tv, 3 * nv * sizeof(double), cudaMemcpyDeviceToHost, d.stream);
-  pool_free(t, d.stream);
   SUBFV_CUDA(e);
   return 0;
 }
