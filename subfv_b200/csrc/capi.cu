@@ -121,6 +121,7 @@ int ensure_full_geometry(DevMesh& d) {
 // the staging buffer the copy itself takes three of each vertex's four doubles: slow, row
 // by row, but without device memory (the fourth double of a position is always 0).
 int xyz_to_host(DevMesh& d, const double4* a, double* out) {
+  OnDevice on(d.device);
   double* t = nullptr;
   if (pool_alloc((void**)&t, 3 * (size_t)d.nv * sizeof(double), d.stream)) {
     cudaGetLastError();
@@ -135,6 +136,7 @@ int xyz_to_host(DevMesh& d, const double4* a, double* out) {
   return 0;
 }
 int xyz_from_host(DevMesh& d, const double* in, double4* a) {
+  OnDevice on(d.device);
   double* t = nullptr;
   if (pool_alloc((void**)&t, 3 * (size_t)d.nv * sizeof(double), d.stream)) {
     cudaGetLastError();
@@ -277,6 +279,7 @@ int subfv_mesh_create_from_topology(const subfv_topology* tp, int b2d, subfv_mes
 int subfv_mesh_destroy(subfv_mesh* m) {
   if (!m) return 0;
   {
+    OnDevice on(m->d.device);
     std::lock_guard<std::mutex> lock(m->life->mu);
     // a state still holds the mesh: it frees its buffers after this event. Without one the
     // queued work is waited for here.
@@ -580,6 +583,7 @@ int subfv_lag_get_vp(subfv_lag_state* s, double* vp) {
   DevMesh& d = s->m->d;
   if (xyz_to_host(d, d.vp, vp)) return -1;
   SUBFV_CUDA(cudaStreamSynchronize(d.stream));
+  SUBFV_CUDA(cudaGetLastError());
   return 0;
 }
 int subfv_lag_last_dt(subfv_lag_state* s, double* dt) {

@@ -167,6 +167,20 @@ void set_error(const std::string& msg);
     }                                                                             \
   } while (0)
 
+// Makes `dev` current for a scope: a kernel launch and an allocation go to the current device,
+// where a copy goes by its pointers and stream.
+struct OnDevice {
+  int before = -1;
+  explicit OnDevice(int dev) {
+    int cur = dev;
+    if (cudaGetDevice(&cur) == cudaSuccess && cur != dev && cudaSetDevice(dev) == cudaSuccess) before = cur;
+  }
+  OnDevice(const OnDevice&) = delete;
+  ~OnDevice() {
+    if (before >= 0) cudaSetDevice(before);
+  }
+};
+
 // Device-side scalars of a time loop; one struct per in-flight problem.
 struct LagScalars {
   double dtmin;               // running CFL minimum of the current step

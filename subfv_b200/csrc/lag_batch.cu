@@ -483,6 +483,7 @@ int subfv_lag_batch_get_sol(subfv_lag_batch* b, int slot, double* sol) {
     SUBFV_CUDA(cudaStreamWaitEvent(d.stream, e, 0));
     cudaEventDestroy(e);
   }
+  OnDevice on(d.device);
   double* t = nullptr;
   if (pool_alloc((void**)&t, 5 * (size_t)d.ne * sizeof(double), d.stream)) {
     cudaGetLastError();  // no room for the staging buffer: the copy takes five doubles of each record

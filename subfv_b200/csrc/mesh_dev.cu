@@ -154,6 +154,7 @@ int devmesh_create(const subfv_mesh_desc* d, DevMesh* m) {
   m->nsf = nsf;
   m->nse = nse;
   m->b2d = d->b2d;
+  SUBFV_CUDA(cudaGetDevice(&m->device));
   SUBFV_CUDA(cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking));
   cudaStream_t s = m->stream;
   size_t* B = &m->bytes;

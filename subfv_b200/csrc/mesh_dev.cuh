@@ -148,6 +148,7 @@ struct DevMesh {
   int* vel_off = nullptr;
   int* vel = nullptr;
   int* cse_sorted = nullptr;
+  int device = 0;  // the device that holds the mesh
   // status word (StatusBits) and the stream the mesh's work runs on
   unsigned* status = nullptr;
   cudaStream_t stream = nullptr;

@@ -372,6 +372,7 @@ int subfv_ns_advance(subfv_ns_state* s, int n_steps, int* steps_done, double* t)
 
 int subfv_ns_get_sol(subfv_ns_state* s, double* sol) {
   DevMesh& d = s->m->d;
+  OnDevice on(d.device);
   launch_unpack6(d, d.ne, kRec, s->U0, s->stage);
   SUBFV_CUDA(cudaMemcpyAsync(sol, s->stage, 5 * (size_t)d.ne * sizeof(double), cudaMemcpyDeviceToHost, d.stream));
   SUBFV_CUDA(cudaStreamSynchronize(d.stream));
