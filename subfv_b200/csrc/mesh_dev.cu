@@ -343,7 +343,13 @@ int devmesh_create(const subfv_mesh_desc* d, DevMesh* m) {
       upload(&m->vse_off, vse_off, B, s) || upload(&m->vse, vse, B, s) || upload(&m->csf_off, csf_off, B, s) ||
       upload(&m->csf, csf, B, s) || alloc(&m->status, 4, B, s) || upload(&m->fpos, fpos, B, s))
     return -1;
+  // whether the tile node kernel can serve the mesh, told by the creation's own wait
+  unsigned misfit = 0;
+  launch_check_node_codes(*m, m->status + 1);
+  SUBFV_CUDA(cudaGetLastError());
+  SUBFV_CUDA(cudaMemcpyAsync(&misfit, m->status + 1, sizeof(misfit), cudaMemcpyDeviceToHost, s));
   SUBFV_CUDA(cudaStreamSynchronize(s));
+  if (misfit) m->tile_end[0] = m->tile_end[1] = m->tile_end[2] = 0;
   return 0;
 }
 

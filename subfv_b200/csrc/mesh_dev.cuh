@@ -111,10 +111,10 @@ struct DevMesh {
   double* npinv = nullptr;
   unsigned long long npinv_epoch = 0;
   // The tile node kernel's codes of every (vertex, subface) and (vertex, subcell) pair
-  // (ns_node_tile.cu, k_build_node_codes), built by the first explicit Euler state on the
-  // mesh; node_codes: 1 built, -1 the mesh's vertices do not fit them, 0 not tried.
-  // tile_end: how many vertices of vorder have at most 8, 16 and 32 subfaces (0 in all when
-  // some vertex has more).
+  // (ns_node_tile.cu, k_build_node_codes), built (node_codes) by the first explicit Euler
+  // state on the mesh whose scheme reads them.
+  // tile_end: how many vertices of vorder have at most 8, 16 and 32 subfaces; 0 in all when
+  // some vertex does not fit its tile (found at creation).
   int2* vslot = nullptr;
   int4* vcorner = nullptr;
   int node_codes = 0;
@@ -184,5 +184,7 @@ void launch_vert_volume(const DevMesh& m);
 // must be allocated)
 void launch_build_geom_codes(const DevMesh& m);
 void launch_vert_is_bound(const DevMesh& m);
+// sets *fail when a vertex does not fit the tile node kernel's tiles (ns_node_tile.cu)
+void launch_check_node_codes(const DevMesh& m, unsigned* fail);
 
 }  // namespace subfv

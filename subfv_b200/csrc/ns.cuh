@@ -73,10 +73,13 @@ struct NsTable {
 constexpr int kNsCellBlock = 128;
 // The node kernel in tiles of vertices (ns_node_tile.cu): multi_point without excluded
 // boundary vertices and two_wave, on meshes whose vertices have at most 32 subfaces.
-// ensure_node_codes builds its per-mesh codes on first use, on the mesh's stream.
+// ensure_node_codes builds its per-mesh codes for the first state or batch of these schemes
+// on the mesh, on the mesh's stream, without waiting; where they find no room the other node
+// kernels serve.
 // Their bytes are charged with a state on the mesh (node_codes_bytes), not with the mesh,
 // which holds none of them until then.
-int ensure_node_codes(DevMesh* m);
+bool node_tile_scheme(const NsParams& P);
+int ensure_node_codes(DevMesh* m, const NsParams& P);
 int64_t node_codes_bytes(const DevMesh& m);
 int node_tiles(const DevMesh& m);  // blocks of the tile node kernel
 bool node_tile_serves(const DevMesh& m, const NsParams& P);

@@ -26,6 +26,7 @@ namespace {
 struct Slot {
   subfv_mesh* mesh = nullptr;
   int owns_mesh = 0;
+  int tiles = 0;           // admitted with its mesh's node codes, which the admission's event covers
   int live = 0;            // holds a problem (in the table or waiting to be removed)
   cudaEvent_t free_ev = nullptr;  // recorded on the batch stream when the slot left the table
   double *U0 = nullptr, *U1 = nullptr, *fs = nullptr, *rhs1 = nullptr, *rhs2 = nullptr;
@@ -147,7 +148,7 @@ int table_upload(subfv_ns_batch* b) {
   for (int i = 0; i < n; ++i) {
     const DevMesh& d = b->slots[b->order[i]].mesh->d;
     group = std::max(group, ns_node_lanes(d));
-    tiles = tiles && d.node_codes > 0;
+    tiles = tiles && b->slots[b->order[i]].tiles;
   }
   // the captured step loop launches one node kernel, for one group size
   if (n && (group != b->tab.group || tiles != b->tab.tiles)) {
@@ -334,7 +335,7 @@ int subfv_ns_batch_add(subfv_ns_batch* b, subfv_mesh* m, int take_mesh, const do
     set_error("subfv_ns_batch_add: null argument");
     return -2;
   }
-  if (handle_ensure_full_geometry(m->d) || ensure_node_codes(&m->d) ||
+  if (handle_ensure_full_geometry(m->d) || ensure_node_codes(&m->d, b->P) ||
       (b->P.second_order && ensure_nodal_pinv(&m->d)))
     return -1;
   const DevMesh& d = m->d;
@@ -388,6 +389,7 @@ int subfv_ns_batch_add(subfv_ns_batch* b, subfv_mesh* m, int take_mesh, const do
   q.mesh = m;
   q.owns_mesh = take_mesh ? 1 : 0;
   q.live = 1;
+  q.tiles = d.node_codes;
   q.bytes = need;
   q.first_snap = b->snap_count + 1;
   q.t0 = t0;

@@ -44,7 +44,10 @@ constexpr int kTileThreads = 256, kTileBlock = kTileThreads + 32;
 // iterations: 14.9 against 16.3 ms; 64 tubes: 133 against 145 ms); shared memory, 59 KB a
 // block, allows three as well.
 constexpr int kTileBlocksPerSm = 3;
-constexpr int kTileCorners = kTileThreads / 2;  // a vertex has at most half as many corners as positions
+// A vertex of a one-layer slab or a hexahedral box has at most half as many corners as
+// positions. Inside layers of prisms or tetrahedra it has two thirds as many corners as
+// subfaces and may have more than its tile holds; the other kernels serve such a mesh.
+constexpr int kTileCorners = kTileThreads / 2;
 // log2 of a tile's vertices by class: the vertices with up to 8, 16 and 32 subfaces
 __host__ __device__ constexpr int tile_log2(int cls) { return 5 - cls; }
 
@@ -433,8 +436,10 @@ __global__ void __launch_bounds__(kTileBlock, kTileBlocksPerSm) kb_ns_node_tile(
 // its cell (-1: no corner) and the positions whose left / right flux enters its sums. A
 // vertex's corners are its own subcells, then the other cells of its subfaces (a periodic
 // vertex's list holds its images' subfaces). Both arrays start as -1. fail: a vertex has
-// more corners than the tile's class, or a tag beyond its bits.
-__global__ void k_build_node_codes(DevMesh m, int2* __restrict__ vslot, int4* __restrict__ vcorner, int* fail) {
+// more corners than the tile's class, or a tag beyond its bits; with CHECK that is all the
+// kernel finds out.
+template <bool CHECK>
+__global__ void k_build_node_codes(DevMesh m, int2* __restrict__ vslot, int4* __restrict__ vcorner, unsigned* fail) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m.nv) return;
   const int cls = i < m.tile_end[0] ? 0 : i < m.tile_end[1] ? 1 : 2, log2 = tile_log2(cls);
@@ -480,7 +485,8 @@ __global__ void k_build_node_codes(DevMesh m, int2* __restrict__ vslot, int4* __
     const int kl = corner_of(lr.x), kr = lr.y < 0 ? 31 : corner_of(lr.y);
     const unsigned tag = lr.y < 0 ? (unsigned)(-1 - lr.y) : 0u;
     if (tag > 0xffffu) ok = false;
-    slot[j << log2] = make_int2(sf, (int)((unsigned)kl | ((unsigned)kr << 5) | (tag << 10) | ((unsigned)(ns - 1) << 26)));
+    if (!CHECK) slot[j << log2] = make_int2(sf, (int)((unsigned)kl | ((unsigned)kr << 5) | (tag << 10) | ((unsigned)(ns - 1) << 26)));
+    if (CHECK) continue;
     // the flux enters the sums of this vertex's subcells, by their positions in its list
     const int2 se = m.sf_se[sf];
     if (m.se_vert[se.x] == v && m.se_loc[se.x] < nq) {
@@ -491,8 +497,11 @@ __global__ void k_build_node_codes(DevMesh m, int2* __restrict__ vslot, int4* __
           if (sub[k] >= 0 && sub[k] == m.vse[q0 + m.se_loc[se.y]]) rm[k] |= 1u << j;
     }
   }
-  for (int k = 0; k < nc; ++k) corner[k << log2] = make_int4(sub[k], cell[k], (int)lm[k], (int)rm[k]);
-  if (!ok) *fail = 1;
+  if (CHECK) {
+    if (!ok) *fail = 1;
+  } else {
+    for (int k = 0; k < nc; ++k) corner[k << log2] = make_int4(sub[k], cell[k], (int)lm[k], (int)rm[k]);
+  }
 }
 
 template <class T, class L, int SCH>
@@ -509,10 +518,10 @@ void launch_kb_tile_t(const NsTable& t, const NsParams& P, cudaStream_t s, int w
   kb_ns_node_tile<T, L, SCH><<<t.grid_v, kTileBlock, smem, s>>>(t.items, t.wt, t.hdr, P, which, so);
 }
 
-// multi_point with excluded boundary vertices mixes two fluxes: the other kernels take it
-bool tile_scheme(const NsParams& P) { return P.scheme == 4 || (P.scheme == 1 && !P.excl); }
-
 }  // namespace
+
+// multi_point with excluded boundary vertices mixes two fluxes: the other kernels take it
+bool node_tile_scheme(const NsParams& P) { return P.scheme == 4 || (P.scheme == 1 && !P.excl); }
 
 int node_tiles(const DevMesh& m) {
   int t = 0;
@@ -520,34 +529,35 @@ int node_tiles(const DevMesh& m) {
     t += (m.tile_end[c] - begin + (1 << tile_log2(c)) - 1) >> tile_log2(c);
   return t;
 }
-bool node_tile_serves(const DevMesh& m, const NsParams& P) { return m.node_codes > 0 && tile_scheme(P); }
-bool node_tile_serves(const NsTable& t, const NsParams& P) { return t.tiles && tile_scheme(P); }
+bool node_tile_serves(const DevMesh& m, const NsParams& P) { return m.node_codes && node_tile_scheme(P); }
+bool node_tile_serves(const NsTable& t, const NsParams& P) { return t.tiles && node_tile_scheme(P); }
 
 int64_t node_codes_bytes(const DevMesh& m) {
   return (int64_t)node_tiles(m) * (int64_t)(kTileThreads * sizeof(int2) + kTileCorners * sizeof(int4));
 }
 
-int ensure_node_codes(DevMesh* m) {
-  if (m->node_codes) return 0;
-  if (m->nv == 0 || m->tile_end[2] != m->nv) {
-    m->node_codes = -1;
+void launch_check_node_codes(const DevMesh& m, unsigned* fail) {
+  if (node_tiles(m)) k_build_node_codes<true><<<grid_for(m.nv, 128), 128, 0, m.stream>>>(m, nullptr, nullptr, fail);
+}
+
+int ensure_node_codes(DevMesh* m, const NsParams& P) {
+  if (m->node_codes || !node_tile_scheme(P) || !node_tiles(*m)) return 0;
+  const size_t nt = node_tiles(*m), sb = nt * kTileThreads * sizeof(int2), cb = nt * kTileCorners * sizeof(int4);
+  int2* slots = nullptr;
+  int4* corners = nullptr;
+  if (cudaMallocAsync((void**)&slots, sb, m->stream) != cudaSuccess ||
+      cudaMallocAsync((void**)&corners, cb, m->stream) != cudaSuccess) {
+    cudaGetLastError();
+    if (slots) cudaFreeAsync(slots, m->stream);
     return 0;
   }
-  const size_t nt = node_tiles(*m), sb = nt * kTileThreads * sizeof(int2), cb = nt * kTileCorners * sizeof(int4);
-  int* fail = nullptr;
-  SUBFV_CUDA(cudaMallocAsync((void**)&m->vslot, sb, m->stream));
-  SUBFV_CUDA(cudaMallocAsync((void**)&m->vcorner, cb, m->stream));
-  SUBFV_CUDA(cudaMallocAsync((void**)&fail, sizeof(int), m->stream));
+  m->vslot = slots;
+  m->vcorner = corners;
+  m->node_codes = 1;
   SUBFV_CUDA(cudaMemsetAsync(m->vslot, 0xff, sb, m->stream));
   SUBFV_CUDA(cudaMemsetAsync(m->vcorner, 0xff, cb, m->stream));
-  SUBFV_CUDA(cudaMemsetAsync(fail, 0, sizeof(int), m->stream));
-  k_build_node_codes<<<grid_for(m->nv, 128), 128, 0, m->stream>>>(*m, m->vslot, m->vcorner, fail);
+  k_build_node_codes<false><<<grid_for(m->nv, 128), 128, 0, m->stream>>>(*m, m->vslot, m->vcorner, nullptr);
   SUBFV_CUDA(cudaGetLastError());
-  int h = 0;
-  SUBFV_CUDA(cudaMemcpyAsync(&h, fail, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
-  SUBFV_CUDA(cudaStreamSynchronize(m->stream));
-  SUBFV_CUDA(cudaFreeAsync(fail, m->stream));
-  m->node_codes = h ? -1 : 1;
   return 0;
 }
 
