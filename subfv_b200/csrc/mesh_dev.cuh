@@ -110,6 +110,7 @@ struct DevMesh {
   // major), valid while npinv_epoch == geom_epoch (ensure_nodal_pinv in ns.cuh).
   double* npinv = nullptr;
   unsigned long long npinv_epoch = 0;
+  bool npinv_counted = false;  // in `bytes`: once a state asked for them
   // The tile node kernel's codes of every (vertex, subface) and (vertex, subcell) pair
   // (ns_node_tile.cu, k_build_node_codes), built (node_codes) by the first explicit Euler
   // state on the mesh whose scheme reads them.

@@ -1935,13 +1935,24 @@ void launch_nodal_grad(const DevMesh& m, const NsParams& P, const double* U, con
   k_ns_nodal_grad<<<grid_for(m.nv, 128), 128, 0, m.stream>>>(m, P, U, prim, ngrad, sc);
 }
 
-int ensure_nodal_pinv(DevMesh* m) {
+int ensure_nodal_pinv(DevMesh* m, bool counted) {
   if (m->moving || m->nv == 0) return 0;
-  if (m->npinv && m->npinv_epoch == m->geom_epoch) return 0;
+  const size_t bytes = 9 * (size_t)m->nv * sizeof(double);
   if (!m->npinv) {
-    SUBFV_CUDA(cudaMallocAsync((void**)&m->npinv, 9 * (size_t)m->nv * sizeof(double), m->stream));
-    m->bytes += 9 * (size_t)m->nv * sizeof(double);
+    const cudaError_t e = cudaMallocAsync((void**)&m->npinv, bytes, m->stream);
+    if (e != cudaSuccess && !counted) {  // a batch's kernels form them where the mesh has none
+      cudaGetLastError();
+      m->npinv = nullptr;
+      return 0;
+    }
+    SUBFV_CUDA(e);
+    m->npinv_epoch = m->geom_epoch - 1;
   }
+  if (counted && !m->npinv_counted) {
+    m->bytes += bytes;
+    m->npinv_counted = true;
+  }
+  if (m->npinv_epoch == m->geom_epoch) return 0;
   k_ns_nodal_pinv<<<grid_for(m->nv, 128), 128, 0, m->stream>>>(*m, m->npinv);
   SUBFV_CUDA(cudaGetLastError());
   m->npinv_epoch = m->geom_epoch;

@@ -50,8 +50,10 @@ struct NsItem {
 int ns_node_lanes(const DevMesh& m);
 // Fills (or refills after the geometry changed) the mesh's per-vertex pseudo-inverses of
 // the nodal-gradient matrices (DevMesh::npinv), on the mesh stream; nothing for a moving
-// mesh. The solo gradient launches read them while they match the current geometry.
-int ensure_nodal_pinv(DevMesh* m);
+// mesh. The gradient launches read them while they match the current geometry. counted: their
+// bytes become the mesh's own (a state asks), and no room for them is an error; a batch,
+// whose budget counts neither them nor the node codes, does without instead.
+int ensure_nodal_pinv(DevMesh* m, bool counted);
 // Table of in-flight problems on the device: items, work-block prefixes over their
 // vertices (wv, block_v vertices per work block) and cells (wc, 128 cells per work
 // block), and hdr[0] = the number of problems. Up to cap problems; the grids are
@@ -76,8 +78,7 @@ constexpr int kNsCellBlock = 128;
 // ensure_node_codes builds its per-mesh codes for the first state or batch of these schemes
 // on the mesh, on the mesh's stream, without waiting; where they find no room the other node
 // kernels serve.
-// Their bytes are charged with a state on the mesh (node_codes_bytes), not with the mesh,
-// which holds none of them until then.
+// node_codes_bytes: what they take, 128 bytes a vertex of up to 8 subfaces, 256 of up to 16.
 bool node_tile_scheme(const NsParams& P);
 int ensure_node_codes(DevMesh* m, const NsParams& P);
 int64_t node_codes_bytes(const DevMesh& m);

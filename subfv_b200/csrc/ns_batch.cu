@@ -32,6 +32,7 @@ struct Slot {
   double *U0 = nullptr, *U1 = nullptr, *fs = nullptr, *rhs1 = nullptr, *rhs2 = nullptr;
   double *ngrad = nullptr, *grad = nullptr, *delta = nullptr, *partial = nullptr;
   int64_t bytes = 0;       // state + mesh bytes charged against the budget
+  int64_t caches = 0;      // bytes of mesh caches built for its admission, beside the charge
   unsigned long long seen_epoch = 0;  // the mesh geometry the table's copy of the mesh belongs to
   unsigned long long first_snap = 0;  // the first snapshot that includes this problem
   double t0 = 0.0;
@@ -45,14 +46,35 @@ struct Snapshot {
   unsigned long long seq = 0;  // snapshots are numbered in enqueue order from 1
 };
 
+// The corner sums and, in second order, the vertex records, which end where the sums' room of
+// 15 doubles a vertex would: the sums are dead from their gather to the next node kernel,
+// and the records live only between the two gradient kernels that run then. A record's nine
+// further doubles (the weights and extremes) so take no room of their own on any mesh of
+// more than two cells.
+size_t corner_and_vertex_doubles(const DevMesh& d, int second_order) {
+  const size_t fs = kNsFs * (size_t)d.nse;
+  return second_order ? std::max(fs + 15 * (size_t)d.nv, kNsVert * (size_t)d.nv) : fs;
+}
+
 // The per-problem state: a first-order scheme needs neither the second stage's state nor
 // the gradients nor the second residual.
 int64_t state_bytes(const DevMesh& d, int second_order) {
-  const int64_t ne = d.ne, nv = d.nv, nse = d.nse;
-  const int64_t o1 = kRec * ne + kNsFs * nse + kRhs * ne + 5 * ne + 6 * (int64_t)ns_partial_blocks(d);
-  // the mesh's pseudo-inverses are the mesh's once they exist
-  const int64_t o2 = kRec * ne + kRhs * ne + kNsVert * nv + 15 * ne + (d.npinv || d.moving ? 0 : 9 * nv);
-  return 8 * (o1 + (second_order ? o2 : 0)) + node_codes_bytes(d);
+  const int64_t ne = d.ne;
+  const int64_t o1 = kRec * ne + (int64_t)corner_and_vertex_doubles(d, second_order) + kRhs * ne + 5 * ne +
+                     6 * (int64_t)ns_partial_blocks(d);
+  const int64_t o2 = kRec * ne + kRhs * ne + 15 * ne;
+  return 8 * (o1 + (second_order ? o2 : 0));
+}
+
+// What admission would add to the mesh for the faster kernels: the node tiles' codes and the
+// nodal gradients' pseudo-inverses. The mesh keeps them, whichever problem comes next, so
+// they are no problem's charge; they are built while they fit the budget beside the charges,
+// and a problem that fits only without them runs on the kernels that do without.
+int64_t cache_bytes(const DevMesh& d, const NsParams& P) {
+  int64_t n = 0;
+  if (!d.node_codes && node_tile_scheme(P)) n += node_codes_bytes(d);
+  if (!d.npinv && !d.moving && P.second_order) n += 72 * (int64_t)d.nv;
+  return n;
 }
 
 }  // namespace
@@ -61,7 +83,7 @@ struct subfv_ns_batch {
   NsParams P{};
   cudaStream_t stream = nullptr;
   int cap = 0;
-  int64_t budget = 0, used = 0;
+  int64_t budget = 0, used = 0, caches = 0;
   NsScalars* sc = nullptr;  // device [cap]
   unsigned* status = nullptr;  // device [cap]
   std::vector<Slot> slots;
@@ -96,7 +118,7 @@ int dalloc_async(T** p, size_t n, cudaStream_t s) {
 }
 
 void slot_free_state(Slot& q, cudaStream_t s) {
-  double* bufs[] = {q.U0, q.U1, q.fs, q.rhs1, q.rhs2, q.ngrad, q.grad, q.delta, q.partial};
+  double* bufs[] = {q.U0, q.U1, q.fs, q.rhs1, q.rhs2, q.grad, q.delta, q.partial};  // ngrad lies in fs
   for (double* b : bufs) pool_free(b, s);
   q.U0 = q.U1 = q.fs = q.rhs1 = q.rhs2 = q.ngrad = q.grad = q.delta = q.partial = nullptr;
 }
@@ -127,8 +149,8 @@ int table_upload(subfv_ns_batch* b) {
     Slot& q = b->slots[i];
     DevMesh& d = q.mesh->d;
     if (q.seen_epoch == d.geom_epoch) continue;
-    if (b->P.second_order) {
-      if (ensure_nodal_pinv(&d)) return -1;
+    if (b->P.second_order && d.npinv) {
+      if (ensure_nodal_pinv(&d, false)) return -1;
       SUBFV_CUDA(cudaEventRecord(q.free_ev, d.stream));
       SUBFV_CUDA(cudaStreamWaitEvent(b->stream, q.free_ev, 0));
     }
@@ -335,9 +357,7 @@ int subfv_ns_batch_add(subfv_ns_batch* b, subfv_mesh* m, int take_mesh, const do
     set_error("subfv_ns_batch_add: null argument");
     return -2;
   }
-  if (handle_ensure_full_geometry(m->d) || ensure_node_codes(&m->d, b->P) ||
-      (b->P.second_order && ensure_nodal_pinv(&m->d)))
-    return -1;
+  if (handle_ensure_full_geometry(m->d)) return -1;
   const DevMesh& d = m->d;
   if (ns_node_lanes(d) == 0) {
     set_error("subfv_ns_batch_add: a vertex has more than 32 subfaces or subcells");
@@ -354,19 +374,27 @@ int subfv_ns_batch_add(subfv_ns_batch* b, subfv_mesh* m, int take_mesh, const do
     return SUBFV_BATCH_FULL;
   }
   Slot& q = b->slots[k];
+  int64_t caches = cache_bytes(d, b->P);
+  if (b->used + need + b->caches + caches <= b->budget) {
+    if (ensure_node_codes(&m->d, b->P) || (b->P.second_order && ensure_nodal_pinv(&m->d, false))) return -1;
+  } else {
+    caches = 0;
+    if (b->P.second_order && d.npinv && ensure_nodal_pinv(&m->d, false)) return -1;
+  }
   cudaStream_t s = d.stream;
-  const size_t ne = d.ne, nv = d.nv, nse = d.nse;
+  const size_t ne = d.ne, nfs = corner_and_vertex_doubles(d, b->P.second_order);
   double* stage = nullptr;
   const bool o2 = b->P.second_order != 0;
-  if (dalloc_async(&q.U0, kRec * ne, s) || dalloc_async(&q.fs, kNsFs * nse, s) ||
+  if (dalloc_async(&q.U0, kRec * ne, s) || dalloc_async(&q.fs, nfs, s) ||
       dalloc_async(&q.rhs1, kRhs * ne, s) || dalloc_async(&q.delta, 5 * ne, s) ||
       dalloc_async(&q.partial, 6 * (size_t)ns_partial_blocks(d), s) ||
       (o2 && (dalloc_async(&q.U1, kRec * ne, s) || dalloc_async(&q.rhs2, kRhs * ne, s) ||
-              dalloc_async(&q.ngrad, kNsVert * nv, s) || dalloc_async(&q.grad, 15 * ne, s))) ||
+              dalloc_async(&q.grad, 15 * ne, s))) ||
       pool_alloc((void**)&stage, 5 * ne * sizeof(double), s)) {
     slot_free_state(q, s);
     return -1;
   }
+  if (o2) q.ngrad = q.fs + (nfs - kNsVert * (size_t)d.nv);
   NsScalars h{};
   h.dtred = 1e10;
   h.omega = 1.0;
@@ -391,6 +419,8 @@ int subfv_ns_batch_add(subfv_ns_batch* b, subfv_mesh* m, int take_mesh, const do
   q.live = 1;
   q.tiles = d.node_codes;
   q.bytes = need;
+  q.caches = caches;
+  b->caches += caches;
   q.first_snap = b->snap_count + 1;
   q.t0 = t0;
   q.seen_epoch = d.geom_epoch;
@@ -410,6 +440,8 @@ int subfv_ns_batch_remove(subfv_ns_batch* b, int slot) {
   auto it = std::find(b->order.begin(), b->order.end(), slot);
   if (it != b->order.end()) b->order.erase(it);
   b->used -= q.bytes;
+  b->caches -= q.caches;
+  q.caches = 0;
   q.bytes = 0;
   q.live = 0;
   b->retiring.push_back(slot);  // freed after the table rewrite that drops it

@@ -126,7 +126,7 @@ void enqueue_ns_step(subfv_ns_state* s) {
 int ns_sync_geometry(subfv_ns_state* s) {
   DevMesh& d = s->m->d;
   if (s->geom_seen && s->seen_epoch == d.geom_epoch) return 0;
-  if (s->P.second_order && ensure_nodal_pinv(&d)) return -1;
+  if (s->P.second_order && ensure_nodal_pinv(&d, true)) return -1;
   if (s->geom_seen && s->P.diff && diffusion_cache_build(&d, s->D, s->U0, s->dterm, s->mu0c)) return -1;
   if (s->graph) {
     SUBFV_CUDA(cudaStreamSynchronize(d.stream));
