@@ -97,8 +97,11 @@ int ensure_lag_arrays(DevMesh& d) {
   SUBFV_CUDA(cudaMallocAsync((void**)&d.cinfo, (size_t)d.ne * sizeof(uint32_t), d.stream));
   SUBFV_CUDA(cudaMallocAsync((void**)&d.gpair, pairs * sizeof(uint32_t), d.stream));
   SUBFV_CUDA(cudaMallocAsync((void**)&d.gsub, (size_t)d.nse * sizeof(uint32_t), d.stream));
-  d.bytes += 6 * (size_t)d.nf * sizeof(double) + entries * sizeof(int4) + (size_t)d.nf * sizeof(double4) +
-             (pairs + (size_t)d.ne + (size_t)d.nse) * sizeof(uint32_t);
+  // what a batch's budget is charged: the records, the entries themselves and 16 bytes of codes
+  // a cell and 4 a subcell. The tiles' padding and the other pair codes (60 bytes a prism) come
+  // on top, so that a budget admits the problems it did before the codes lay in tiles.
+  d.bytes += 6 * (size_t)d.nf * sizeof(double) + std::max<size_t>(d.ncsf, 1) * sizeof(int4) +
+             (size_t)d.nf * sizeof(double4) + 16 * (size_t)d.ne + (size_t)d.nse * sizeof(uint32_t);
   launch_build_cell_entries(d);
   launch_build_geom_codes(d);
   SUBFV_CUDA(cudaGetLastError());
