@@ -403,6 +403,8 @@ int subfv_ns_batch_slot_info(const subfv_ns_batch* b, int slot, double* t, int64
 /* Copy a problem's state to the host (waits for the queued steps unless the latest
  * snapshot shows the problem finished). */
 int subfv_ns_batch_get_sol(subfv_ns_batch* b, int slot, double* sol);
+/* For checks: how often the batch has captured its step loop. */
+int subfv_probe_ns_captures(const subfv_ns_batch* b);
 /* Launch shape: block_v threads (one per vertex) per block of the vertex kernels (64,
  * 128 or 256), and the persistent grid sizes of the vertex and cell kernels. Results do
  * not depend on it. */
@@ -434,6 +436,8 @@ int subfv_lag_batch_sync(subfv_lag_batch* b);
 int subfv_lag_batch_slot_info(const subfv_lag_batch* b, int slot, double* t, int64_t* steps, int* done,
                               unsigned* status);
 int subfv_lag_batch_get_sol(subfv_lag_batch* b, int slot, double* sol);
+/* as subfv_probe_ns_captures */
+int subfv_probe_lag_captures(const subfv_lag_batch* b);
 /* persistent grid size of every batched kernel; results do not depend on it */
 int subfv_lag_batch_set_grid(subfv_lag_batch* b, int grid);
 

@@ -117,6 +117,8 @@ SIGNATURES = {
     "subfv_lag_batch_sync": (c_int, [P]),
     "subfv_lag_batch_slot_info": (c_int, [P, c_int, PD, C.POINTER(c_i64), C.POINTER(c_int), C.POINTER(C.c_uint)]),
     "subfv_lag_batch_get_sol": (c_int, [P, c_int, PD]),
+    "subfv_probe_lag_captures": (c_int, [P]),
+    "subfv_probe_ns_captures": (c_int, [P]),
     "subfv_lag_batch_set_grid": (c_int, [P, c_int]),
     "subfv_bcsr_create": (c_int, [c_int, c_int, PI32, PI32, PD, C.POINTER(P)]),
     "subfv_bcsr_destroy": (c_int, [P]),

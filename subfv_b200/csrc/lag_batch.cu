@@ -66,8 +66,9 @@ struct subfv_lag_batch {
   cudaEvent_t stage_ev[2] = {nullptr, nullptr};
   int stage_cur = 0;
   bool dirty = true;
-  cudaGraphExec_t graph = nullptr;
-  int graph_steps = 0;
+  // the captured step loop, with the thread-per-cell kernels and with the tiles
+  cudaGraphExec_t graph[2] = {nullptr, nullptr};
+  int captures = 0;
   Snapshot snap[2];
   std::deque<int> outstanding;  // snapshot indices in enqueue order
   int snap_next = 0;
@@ -87,23 +88,32 @@ void slot_free_state(Slot& q, cudaStream_t s) {
   q.sol6 = q.rhs6 = nullptr;
 }
 
-int graph_for(subfv_lag_batch* b, int steps) {
-  if (b->graph && b->graph_steps == steps) return 0;
-  if (b->graph) {
-    cudaGraphExecDestroy(b->graph);
-    b->graph = nullptr;
-  }
+constexpr int kGraphSteps = 8;
+
+// destroys a captured loop once no launch of it runs any more
+int graph_drop(subfv_lag_batch* b, int which) {
+  if (!b->graph[which]) return 0;
+  SUBFV_CUDA(cudaStreamSynchronize(b->stream));
+  cudaGraphExecDestroy(b->graph[which]);
+  b->graph[which] = nullptr;
+  return 0;
+}
+
+int graph_for(subfv_lag_batch* b) {
+  cudaGraphExec_t& exec = b->graph[b->tab.small];
+  if (exec) return 0;
   cudaGraph_t g;
   SUBFV_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-  for (int i = 0; i < steps; ++i) launch_lag_batch_step(b->tab, b->precision, b->stream);
+  for (int i = 0; i < kGraphSteps; ++i) launch_lag_batch_step(b->tab, b->precision, b->stream);
   SUBFV_CUDA(cudaStreamEndCapture(b->stream, &g));
-  cudaError_t e = cudaGraphInstantiate(&b->graph, g, 0);
+  cudaError_t e = cudaGraphInstantiate(&exec, g, 0);
   cudaGraphDestroy(g);
   if (e != cudaSuccess) {
+    exec = nullptr;
     set_error(std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
     return -1;
   }
-  b->graph_steps = steps;
+  ++b->captures;
   return 0;
 }
 
@@ -119,24 +129,23 @@ int table_upload(subfv_lag_batch* b) {
   int* hdr = wc + (b->cap + 1);
   const int n = (int)b->order.size();
   wf[0] = wv[0] = wc[0] = 0;
-  int max_csf = 0, max_pairs = 0;
+  // The tiles' warps follow the largest cell the batch has held: they never shrink, so the
+  // loop captured with them is made anew only for a larger one. The loop of the other side of
+  // the line stays for when the table crosses it again, as a served table near it does with
+  // every problem that joins or leaves.
+  int max_csf = b->tab.max_csf, max_pairs = b->tab.max_pairs;
   int64_t cells = 0;
   for (int i = 0; i < n; ++i) {
     cells += b->slots[b->order[i]].mesh->d.ne;
     max_csf = std::max(max_csf, b->slots[b->order[i]].mesh->d.max_csf);
     max_pairs = std::max(max_pairs, b->slots[b->order[i]].mesh->d.max_pairs);
   }
-  const int small = cells <= geo::kTileCells;
-  if (n && (max_csf != b->tab.max_csf || max_pairs != b->tab.max_pairs || small != b->tab.small)) {
-    if (b->graph) {  // the captured step loop launches the cell kernels chosen for the old sizes
-      SUBFV_CUDA(cudaStreamSynchronize(b->stream));
-      cudaGraphExecDestroy(b->graph);
-      b->graph = nullptr;
-    }
+  if (max_csf != b->tab.max_csf || max_pairs != b->tab.max_pairs) {
+    if (graph_drop(b, 1)) return -1;
     b->tab.max_csf = max_csf;
     b->tab.max_pairs = max_pairs;
-    b->tab.small = small;
   }
+  if (n) b->tab.small = cells <= geo::kTileCells ? 1 : 0;
   for (int i = 0; i < n; ++i) {
     Slot& q = b->slots[b->order[i]];
     LagItem& I = it[i];
@@ -261,7 +270,8 @@ int subfv_lag_batch_destroy(subfv_lag_batch* b) {
     if (q.free_ev) cudaEventDestroy(q.free_ev);
   }
   if (b->stream) cudaStreamSynchronize(b->stream);
-  if (b->graph) cudaGraphExecDestroy(b->graph);
+  for (cudaGraphExec_t g : b->graph)
+    if (g) cudaGraphExecDestroy(g);
   cudaFree(b->sc);
   cudaFree(b->status);
   cudaFree(b->tab.items);
@@ -368,6 +378,8 @@ int subfv_lag_batch_remove(subfv_lag_batch* b, int slot) {
   return 0;
 }
 
+int subfv_probe_lag_captures(const subfv_lag_batch* b) { return b ? b->captures : -2; }
+
 int subfv_lag_batch_set_grid(subfv_lag_batch* b, int grid) {
   if (!b || grid < 1) {
     set_error("subfv_lag_batch_set_grid: the grid must be positive");
@@ -375,11 +387,7 @@ int subfv_lag_batch_set_grid(subfv_lag_batch* b, int grid) {
   }
   if (grid != b->tab.grid) {
     b->tab.grid = grid;
-    if (b->graph) {
-      SUBFV_CUDA(cudaStreamSynchronize(b->stream));
-      cudaGraphExecDestroy(b->graph);
-      b->graph = nullptr;
-    }
+    if (graph_drop(b, 0) || graph_drop(b, 1)) return -1;
   }
   return 0;
 }
@@ -390,10 +398,10 @@ int subfv_lag_batch_advance(subfv_lag_batch* b, int n_steps) {
     return -2;
   }
   if (table_upload(b)) return -1;
-  const int chunk = 8;
+  const int chunk = kGraphSteps;
   if (n_steps >= chunk) {
-    if (graph_for(b, chunk)) return -1;
-    for (int i = 0; i + chunk <= n_steps; i += chunk) SUBFV_CUDA(cudaGraphLaunch(b->graph, b->stream));
+    if (graph_for(b)) return -1;
+    for (int i = 0; i + chunk <= n_steps; i += chunk) SUBFV_CUDA(cudaGraphLaunch(b->graph[b->tab.small], b->stream));
   }
   for (int i = 0; i < n_steps % chunk; ++i) launch_lag_batch_step(b->tab, b->precision, b->stream);
   SUBFV_CUDA(cudaGetLastError());

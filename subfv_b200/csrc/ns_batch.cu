@@ -95,8 +95,9 @@ struct subfv_ns_batch {
   cudaEvent_t stage_ev[2] = {nullptr, nullptr};
   int stage_cur = 0;
   bool dirty = true;
-  cudaGraphExec_t graph = nullptr;
-  int graph_steps = 0;
+  // the captured step loop, with the other node kernels and with the tiles
+  cudaGraphExec_t graph[2] = {nullptr, nullptr};
+  int captures = 0;
   Snapshot snap[2];
   std::deque<int> outstanding;  // snapshot indices in enqueue order
   int snap_next = 0;
@@ -123,23 +124,32 @@ void slot_free_state(Slot& q, cudaStream_t s) {
   q.U0 = q.U1 = q.fs = q.rhs1 = q.rhs2 = q.ngrad = q.grad = q.delta = q.partial = nullptr;
 }
 
-int graph_for(subfv_ns_batch* b, int steps) {
-  if (b->graph && b->graph_steps == steps) return 0;
-  if (b->graph) {
-    cudaGraphExecDestroy(b->graph);
-    b->graph = nullptr;
-  }
+constexpr int kGraphSteps = 8;
+
+// destroys a captured loop once no launch of it runs any more
+int graph_drop(subfv_ns_batch* b, int which) {
+  if (!b->graph[which]) return 0;
+  SUBFV_CUDA(cudaStreamSynchronize(b->stream));
+  cudaGraphExecDestroy(b->graph[which]);
+  b->graph[which] = nullptr;
+  return 0;
+}
+
+int graph_for(subfv_ns_batch* b) {
+  cudaGraphExec_t& exec = b->graph[b->tab.tiles];
+  if (exec) return 0;
   cudaGraph_t g;
   SUBFV_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-  for (int i = 0; i < steps; ++i) launch_ns_batch_step(b->tab, b->P, b->stream);
+  for (int i = 0; i < kGraphSteps; ++i) launch_ns_batch_step(b->tab, b->P, b->stream);
   SUBFV_CUDA(cudaStreamEndCapture(b->stream, &g));
-  cudaError_t e = cudaGraphInstantiate(&b->graph, g, 0);
+  cudaError_t e = cudaGraphInstantiate(&exec, g, 0);
   cudaGraphDestroy(g);
   if (e != cudaSuccess) {
+    exec = nullptr;
     set_error(std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
     return -1;
   }
-  b->graph_steps = steps;
+  ++b->captures;
   return 0;
 }
 
@@ -172,13 +182,10 @@ int table_upload(subfv_ns_batch* b) {
     group = std::max(group, ns_node_lanes(d));
     tiles = tiles && b->slots[b->order[i]].tiles;
   }
-  // the captured step loop launches one node kernel, for one group size
-  if (n && (group != b->tab.group || tiles != b->tab.tiles)) {
-    if (b->graph) {
-      SUBFV_CUDA(cudaStreamSynchronize(b->stream));
-      cudaGraphExecDestroy(b->graph);
-      b->graph = nullptr;
-    }
+  // The loop without tiles is captured for one group size; the one with them has none, and
+  // each stays for when a mesh beyond the tiles joins or leaves.
+  if (n) {
+    if (group != b->tab.group && graph_drop(b, 0)) return -1;
     b->tab.group = group;
     b->tab.tiles = tiles;
   }
@@ -327,7 +334,8 @@ int subfv_ns_batch_destroy(subfv_ns_batch* b) {
     if (q.free_ev) cudaEventDestroy(q.free_ev);
   }
   if (b->stream) cudaStreamSynchronize(b->stream);
-  if (b->graph) cudaGraphExecDestroy(b->graph);
+  for (cudaGraphExec_t g : b->graph)
+    if (g) cudaGraphExecDestroy(g);
   cudaFree(b->sc);
   cudaFree(b->status);
   cudaFree(b->tab.items);
@@ -417,7 +425,7 @@ int subfv_ns_batch_add(subfv_ns_batch* b, subfv_mesh* m, int take_mesh, const do
   q.mesh = m;
   q.owns_mesh = take_mesh ? 1 : 0;
   q.live = 1;
-  q.tiles = d.node_codes;
+  q.tiles = d.node_codes && node_tile_scheme(b->P);
   q.bytes = need;
   q.caches = caches;
   b->caches += caches;
@@ -449,6 +457,8 @@ int subfv_ns_batch_remove(subfv_ns_batch* b, int slot) {
   return 0;
 }
 
+int subfv_probe_ns_captures(const subfv_ns_batch* b) { return b ? b->captures : -2; }
+
 int subfv_ns_batch_set_launch(subfv_ns_batch* b, int block_v, int grid_v, int grid_c) {
   if (!b || (block_v != 64 && block_v != 128 && block_v != 256) || grid_v < 1 || grid_c < 1) {
     set_error("subfv_ns_batch_set_launch: block_v must be 64, 128 or 256 and the grids positive");
@@ -459,11 +469,7 @@ int subfv_ns_batch_set_launch(subfv_ns_batch* b, int block_v, int grid_v, int gr
     b->tab.block_v = block_v;
     b->tab.grid_v = grid_v;
     b->tab.grid_c = grid_c;
-    if (b->graph) {
-      SUBFV_CUDA(cudaStreamSynchronize(b->stream));
-      cudaGraphExecDestroy(b->graph);
-      b->graph = nullptr;
-    }
+    if (graph_drop(b, 0) || graph_drop(b, 1)) return -1;
   }
   return 0;
 }
@@ -475,11 +481,7 @@ int subfv_ns_batch_set_node_kernel(subfv_ns_batch* b, int lanes) {
   }
   if (b->P.node_group != lanes) {
     b->P.node_group = lanes;
-    if (b->graph) {
-      SUBFV_CUDA(cudaStreamSynchronize(b->stream));
-      cudaGraphExecDestroy(b->graph);
-      b->graph = nullptr;
-    }
+    if (graph_drop(b, 0) || graph_drop(b, 1)) return -1;
   }
   return 0;
 }
@@ -490,10 +492,10 @@ int subfv_ns_batch_advance(subfv_ns_batch* b, int n_steps) {
     return -2;
   }
   if (table_upload(b)) return -1;
-  const int chunk = 8;
+  const int chunk = kGraphSteps;
   if (n_steps >= chunk) {
-    if (graph_for(b, chunk)) return -1;
-    for (int i = 0; i + chunk <= n_steps; i += chunk) SUBFV_CUDA(cudaGraphLaunch(b->graph, b->stream));
+    if (graph_for(b)) return -1;
+    for (int i = 0; i + chunk <= n_steps; i += chunk) SUBFV_CUDA(cudaGraphLaunch(b->graph[b->tab.tiles], b->stream));
   }
   for (int i = 0; i < n_steps % chunk; ++i) launch_ns_batch_step(b->tab, b->P, b->stream);
   SUBFV_CUDA(cudaGetLastError());

@@ -131,3 +131,23 @@ def test_batch_of_both_kinds(native, cuda_ok, cfg):
         s = NsState(meshes[i], replace(c, tmax=1e30), sols[i])
         assert (st, n, t) == s.advance(steps[i])
         np.testing.assert_array_equal(sol, s.sol())
+
+
+def test_step_loop_captured_once_for_either_kind(native, cuda_ok):
+    """A mesh beyond the tiles joins and leaves, several times: the loop with the tiles and the
+    one without are each captured once."""
+    from subfv_b200 import _lib, meshgen
+    from subfv_b200.mesh import Mesh
+    from subfv_b200.ns import NsBatch, NsConfig
+    c = NsConfig(**CFGS["mp_o2"], method=4, boundary_2d=False, cfl=0.4)
+    m, beyond = (Mesh.from_raw(r) for r in (two_layers(8), two_layers(9)))
+    b = NsBatch(c, capacity=4, budget_bytes=1 << 32)
+    assert b.add(m, _perturbed_gresho(m, 7), 1e30) is not None
+    for _ in range(3):
+        b.advance(8)
+        k = b.add(beyond, _perturbed_gresho(beyond, 7), 1e30)
+        b.advance(8)
+        b.remove(k)
+    b.sync()
+    assert _lib.load().subfv_probe_ns_captures(b._h) == 2
+    b.close()
