@@ -1950,7 +1950,7 @@ int ensure_nodal_pinv(DevMesh* m, bool counted) {
   }
   if (counted && !m->npinv_counted) {
     m->bytes += bytes;
-    m->npinv_counted = true;
+    m->npinv_counted = 1;
   }
   if (m->npinv_epoch == m->geom_epoch) return 0;
   k_ns_nodal_pinv<<<grid_for(m->nv, 128), 128, 0, m->stream>>>(*m, m->npinv);
