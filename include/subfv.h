@@ -325,9 +325,11 @@ int subfv_ns_get_sol(subfv_ns_state* s, double* sol);
  * a group of at least that many lanes. With a group layout the second-order cell
  * gradient also runs a group of 8 lanes per cell (one per vertex) when no cell has more
  * than 8 vertices. The multi_point and two_wave schemes run in tiles of vertices whatever
- * the layout (unless boundary vertices are excluded or a vertex has more than 32
- * subfaces): there it is the layout of the gradients alone. Results are bit-identical in
- * every layout. */
+ * the layout, unless multi_point excludes boundary vertices or some vertex does not fit: a
+ * vertex of up to 8, 16 or 32 subfaces may have 4, 8 or 16 cells around it (slabs of one
+ * layer and hexahedral boxes always fit; inside layers of prisms a vertex of 5 or of 9 and
+ * more prisms a layer does not, nor do most tetrahedral meshes). There it is the layout of
+ * the gradients alone. Results are bit-identical in every layout. */
 int subfv_ns_state_set_node_kernel(subfv_ns_state* s, int lanes);
 /* res = sum of |delta|_2 and res_vect(5) of the last add_timedisc_and_solve call */
 int subfv_ns_residuals(subfv_ns_state* s, double* res, double* res_vect, double* dt);
@@ -371,7 +373,9 @@ int subfv_ns_init_gresho(subfv_mesh* m, double mach, double* sol);
 #define SUBFV_BATCH_FULL (-3) /* no free slot or the HBM budget is exhausted: retry later */
 typedef struct subfv_ns_batch subfv_ns_batch;
 /* capacity: the most problems in flight; budget_bytes: the device bytes that admitted
- * problems (their meshes plus their state) may hold. */
+ * problems (their meshes plus their state) may hold. Beside them a mesh keeps caches for the
+ * faster kernels (node codes, 128 to 512 bytes a vertex; pseudo-inverses, 72), built while
+ * they fit the budget too; a problem that fits only without them runs without. */
 int subfv_ns_batch_create(const subfv_ns_cfg* cfg, int capacity, int64_t budget_bytes, subfv_ns_batch** out);
 int subfv_ns_batch_destroy(subfv_ns_batch* b);
 /* Device bytes of the per-problem state batch b allocates for a problem on mesh m. */

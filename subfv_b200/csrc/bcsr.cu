@@ -16,7 +16,8 @@
 //   reference's left-to-right order.
 // * Gram-Schmidt (modified, as the reference's): one launch per Arnoldi column keeps the
 //   new vector in registers and shared memory over all its projections (k_mgs_column);
-//   beyond its capacity, the axpy of step i is fused with the dot product of step i+1.
+//   where that cannot run (mgs_plan), the axpy of step i is fused with the dot product of
+//   step i+1.
 // * One restart cycle's Arnoldi process (m columns) has no host decision in it: it is
 //   captured once per matrix and workspace as a CUDA graph and replayed.
 // * Givens rotations and the back substitution run on the host in the reference's order.

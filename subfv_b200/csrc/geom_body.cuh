@@ -224,8 +224,9 @@ __device__ inline void state_update(const DevMesh& m, double* sol6, const double
 //   the centroid's tetrahedra, one per pair, summed by a warp per component;
 //   the subcells' tetrahedra, two per (vertex, subface) pair, summed per subcell;
 //   the cell's volume and tests, and the state's update.
-// What bounds it: FP64 issue. One thread per cell ran the 5,500 instructions of a prism as
-// one chain, at 16 warps an SM (180,000 prisms 85 us, 3,000 prisms 20 us).
+// What bounds it: latency, of the loads (43% of a warp's cycles at 3,034 prisms) and of the
+// barriers between the phases (21%); issue is at 11%, the FP64 pipe at 7%. One thread per cell
+// ran the 5,500 instructions of a prism as one chain (3,000 prisms 20 us, here 12.5).
 // Above kTileCells cells (of a mesh, or of a batch's table) one thread per cell is as fast
 // or faster (both cell kernels together: tiles 38.7 us at 16,200 prisms, 43.4 at 21,632,
 // 45.3 at 27,848; a thread per cell 44.6 at 28,322, 46.6 at 33,800, and its time hardly

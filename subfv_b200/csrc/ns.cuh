@@ -74,7 +74,8 @@ struct NsTable {
 };
 constexpr int kNsCellBlock = 128;
 // The node kernel in tiles of vertices (ns_node_tile.cu): multi_point without excluded
-// boundary vertices and two_wave, on meshes whose vertices have at most 32 subfaces.
+// boundary vertices and two_wave, on meshes whose vertices of up to 8, 16 and 32 subfaces have
+// at most 4, 8 and 16 cells.
 // ensure_node_codes builds its per-mesh codes for the first state or batch of these schemes
 // on the mesh, on the mesh's stream, without waiting; where they find no room the other node
 // kernels serve.

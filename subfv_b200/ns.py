@@ -309,9 +309,9 @@ class NsState:
         """0: one thread per vertex; 1: a group of lanes per vertex (8/16/32 as the mesh
         needs); 8, 16, 32: a group of at least that many lanes. A group layout also runs
         the cell gradient with 8 lanes per cell (cells of up to 8 vertices). multi_point
-        and two_wave run in tiles of vertices in every layout (meshes of up to 32
-        subfaces a vertex), which then is that of the gradients alone. Same results in
-        all."""
+        and two_wave run in tiles of vertices in every layout (meshes whose vertices of up
+        to 8, 16 and 32 subfaces have at most 4, 8 and 16 cells), which then is that of
+        the gradients alone. Same results in all."""
         check(_lib.load().subfv_ns_state_set_node_kernel(self._h, int(lanes)), "subfv_ns_state_set_node_kernel")
 
     def residuals(self):

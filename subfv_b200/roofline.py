@@ -36,10 +36,11 @@ def lag_kernel_bytes(s: MeshSizes) -> dict:
     # k_face_geom<0>: vertex records, face vertex and subface ids, the subfaces' vertex
     # slots; writes: face centroids, normal records and subface sums, subface areas
     b["face_geom"] = 32 * nv + 16 * nf + 16 * nf + nf + 32 * nf + 32 * nf + 32 * nf + 8 * nsf
-    # k_geom_step: cell vertex lists, vertex records, cell faces and their static codes,
-    # the face centroids, normal records and subface sums, the subcells' codes; writes:
-    # subcell and cell volumes; update: cell records read + write, rhs read
-    b["cell_geom"] = (4 * (ne + 1) + 4 * nse + 32 * nv + 32 * ne + 16 * ne + 96 * nf + 4 * nse
+    # k_geom_step: cell vertex lists, vertex records, cell faces, the cells' code and that of
+    # each (face, vertex) pair (as many as gather entries), the face centroids, normal records
+    # and subface sums; writes: subcell and cell volumes; update: cell records read + write,
+    # rhs read
+    b["cell_geom"] = (4 * (ne + 1) + 4 * nse + 32 * nv + 32 * ne + 4 * ne + 4 * ncsf + 96 * nf
                       + 8 * nse + 8 * ne + 64 * ne * 2 + 48 * ne)
     return b
 
