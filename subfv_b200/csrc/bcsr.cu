@@ -420,10 +420,11 @@ __device__ inline double mgs_sum(double s, unsigned long long* slots, const int 
     const double v = warp_tree(part[threadIdx.x]);
     if (blockIdx.x == 0) {
       // all of a lane's slots in flight at once, until each holds a value
-      unsigned long long bits[kMgsLaneSlots] = {};
+      unsigned long long bits[kMgsLaneSlots];
       const unsigned long long own = __shfl_sync(0xffffffffu, mgs_word(v), 0);
-      bool late = true;
-      for (int spin = 0; spin < polls && late; ++spin) {
+      bool late;
+      int spin = 0;
+      do {
 #pragma unroll
         for (int u = 0; u < kMgsLaneSlots; ++u) {
           const int q = threadIdx.x + 32 * u;
@@ -432,7 +433,7 @@ __device__ inline double mgs_sum(double s, unsigned long long* slots, const int 
         late = false;
 #pragma unroll
         for (int u = 0; u < kMgsLaneSlots; ++u) late = late || bits[u] == kNoPartial;
-      }
+      } while (late && ++spin < polls);
       double t = 0.0;
 #pragma unroll
       for (int u = 0; u < kMgsLaneSlots; ++u) t = t + __longlong_as_double((long long)bits[u]);
@@ -444,8 +445,10 @@ __device__ inline double mgs_sum(double s, unsigned long long* slots, const int 
       }
     } else if (threadIdx.x == 0) {
       all[blockIdx.x] = mgs_word(v);
-      unsigned long long t = kNoPartial;
-      for (int spin = 0; spin < polls && t == kNoPartial; ++spin) t = *sum;
+      unsigned long long t;
+      int spin = 0;
+      do t = *sum;
+      while (t == kNoPartial && ++spin < polls);
       total = t;
     }
     if (threadIdx.x == 0 && total == kNoPartial) *fail = 1u;
